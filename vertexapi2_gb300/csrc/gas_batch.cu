@@ -660,9 +660,7 @@ gas_status gas_batch_set_graph(gas_batch *b, int32_t nVertices, int32_t nEdges,
   if (st) return st;
   CoreGraph g;
   gas::internal::core_graph(b->core, &g);
-  b->maxOutDeg = 0;
-  for (int32_t v = 0; v < nVertices; ++v)
-    b->maxOutDeg = std::max(b->maxOutDeg, (*g.hOutOff)[(size_t)v + 1] - (*g.hOutOff)[v]);
+  b->maxOutDeg = g.maxOutDeg;
   st = build_units(b, g, b->chunk);
   if (st == GAS_OK && weights && nEdges > 0)  // weights in CSR order for push rounds
     st = gas::internal::core_permute_csr(b->core, weights, &b->weightsOut);

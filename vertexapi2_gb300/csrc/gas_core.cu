@@ -21,7 +21,7 @@
 #include <cstring>
 #include <new>
 #include <string>
-#include <thread>
+#include <type_traits>
 #include <vector>
 
 #include "gas_gb300_core.h"
@@ -173,6 +173,11 @@ struct gas_core_s {
   bool fusedRounds = true;      // one-phase rounds when every degree is <= 8
   bool edgeScatterOn = false;   // keep csr2csc and run scatter-capable rounds
   bool edgeScatterReady = false;  // a scatter list awaits the Program's scatter
+  // One allocation holds the arrays whose sizes follow from V and E (the
+  // next set_graph reuses it when it fits): a cudaMalloc / cudaFree pair
+  // costs about 100 us, and there are some fifty arrays.
+  unsigned char *arena = nullptr;
+  size_t arenaBytes = 0;
   int32_t *inOff = nullptr, *inSrc = nullptr, *outOff = nullptr, *outDst = nullptr;
   void *ed = nullptr;
   void *vd = nullptr, *vnew = nullptr, *vsaved = nullptr, *valt = nullptr;
@@ -180,6 +185,7 @@ struct gas_core_s {
   uint32_t *frontBits = nullptr;  // three active-set bitmaps of the fused rounds
   int32_t bitWords = 0;
   // degree bins of the dense pass (see dense.cuh)
+  int32_t *bins = nullptr;  // hubs | binMid | binSmall | binTiny
   int32_t *binMid = nullptr, *binSmall = nullptr, *binTiny = nullptr;
   int32_t nMid = 0, nSmall = 0, nTiny = 0;
   int32_t *chunkVertex = nullptr, *chunkBegin = nullptr, *chunkFirst = nullptr;
@@ -240,18 +246,16 @@ static uint32_t *round_bits(gas_core_s *c, int32_t stamp) {
 
 namespace {
 
-void free_graph(gas_core *c) {
-  void *ptrs[] = {c->inOff, c->inSrc, c->outOff, c->outDst, c->ed, c->vd, c->vnew, c->vsaved,
-                  c->valt, c->retBits, c->frontBits, c->binMid, c->binSmall,
-                  c->binTiny, c->chunkVertex, c->chunkBegin, c->chunkFirst, c->chunkCount,
-                  c->chunkSlot, c->chunkArrive, c->chunkFlags, c->chunkVal,
-                  c->fvid[0], c->fvid[1], c->fpre[0], c->fpre[1], c->fsplit[0], c->fsplit[1],
-                  c->fbeg[0], c->fbeg[1], c->sbeg[0], c->sbeg[1],
-                  c->rsplit, c->svid[0], c->svid[1], c->spre[0], c->spre[1], c->ssplit[0],
-                  c->ssplit[1], c->mark, c->carryVal, c->carryFlag, c->ctl, c->stats,
-                  c->cscPerm, c->csrPerm, c->csr2csc, c->fcell, c->ellIn, c->ellOut, c->ellEd};
+// Drops the graph; the arena stays for the next one unless `all`.
+void free_graph(gas_core *c, bool all = true) {
+  void *ptrs[] = {c->vsaved, c->frontBits, c->csrPerm, c->fcell, c->ellIn, c->ellOut, c->ellEd};
   for (void *p : ptrs)
     if (p) cudaFree(p);
+  if (all && c->arena) {
+    cudaFree(c->arena);
+    c->arena = nullptr;
+    c->arenaBytes = 0;
+  }
   c->cscPerm = c->csrPerm = nullptr;
   c->csr2csc = nullptr;
   c->fcell = nullptr;
@@ -262,7 +266,7 @@ void free_graph(gas_core *c) {
   c->ed = c->vd = c->vnew = c->vsaved = c->valt = nullptr;
   c->retBits = nullptr;
   c->frontBits = nullptr;
-  c->binMid = c->binSmall = c->binTiny = nullptr;
+  c->bins = c->binMid = c->binSmall = c->binTiny = nullptr;
   c->chunkVertex = c->chunkBegin = c->chunkFirst = c->chunkCount = c->chunkSlot = nullptr;
   c->chunkArrive = c->chunkFlags = nullptr;
   c->chunkVal = nullptr;
@@ -278,6 +282,60 @@ void free_graph(gas_core *c) {
   c->ctl = nullptr;
   c->stats = nullptr;
   c->haveGraph = false;
+}
+
+// Lays the V- and E-sized arrays out in the arena at `base` (null: only the
+// size is wanted), each on a 256-byte boundary.
+size_t carve_arena(gas_core *c, unsigned char *base, bool edgeMap, int32_t maxHubs, int32_t maxChunks) {
+  size_t used = 0;
+  auto take = [&](auto **p, size_t bytes) {
+    *p = reinterpret_cast<std::remove_reference_t<decltype(**p)> *>(base + used);
+    used += (std::max<size_t>(bytes, 1) + 255) & ~(size_t)255;
+  };
+  auto bytes = [&](void **p, size_t n) {
+    *p = base + used;
+    used += (std::max<size_t>(n, 1) + 255) & ~(size_t)255;
+  };
+  const size_t V = (size_t)c->nV, E = (size_t)c->nE, gb = (size_t)((c->gatherBytes + 15) / 16 * 16);
+  take(&c->inOff, 4 * (V + 1));
+  // whole 16-byte quads: the dense pass reads source ids (and 4-byte edge
+  // data) four at a time, up to the quad that holds a vertex's last edge
+  take(&c->inSrc, 4 * (E + 4));
+  take(&c->outOff, 4 * (V + 1));
+  take(&c->outDst, 4 * E);
+  if (c->edgeBytes > 0) bytes(&c->ed, (size_t)c->edgeBytes * (E + 4));
+  if (c->edgeBytes > 0) take(&c->cscPerm, 4 * E);
+  if (edgeMap) take(&c->csr2csc, 4 * E);
+  bytes(&c->vd, (size_t)c->vertexBytes * V);
+  bytes(&c->vnew, (size_t)c->vertexBytes * V);
+  bytes(&c->valt, (size_t)c->vertexBytes * V);
+  take(&c->retBits, 4 * 3 * (size_t)c->bitWords);
+  take(&c->bins, 4 * V);
+  take(&c->chunkVertex, 4 * (size_t)maxChunks);
+  take(&c->chunkBegin, 4 * (size_t)maxChunks);
+  take(&c->chunkFirst, 4 * (size_t)maxChunks);
+  take(&c->chunkCount, 4 * (size_t)maxChunks);
+  take(&c->chunkSlot, 4 * (size_t)maxChunks);
+  take(&c->chunkFlags, 4 * (size_t)maxChunks);
+  take(&c->chunkArrive, 4 * (size_t)maxHubs);
+  bytes(&c->chunkVal, gb * maxChunks);
+  for (int k = 0; k < 2; ++k) {
+    take(&c->fvid[k], 4 * V);
+    take(&c->fpre[k], 4 * V);
+    take(&c->fbeg[k], 4 * V);
+    take(&c->fsplit[k], 4 * (size_t)c->maxGatherTiles);
+    take(&c->svid[k], 4 * V);
+    take(&c->spre[k], 4 * V);
+    take(&c->sbeg[k], 4 * V);
+    take(&c->ssplit[k], 4 * (size_t)c->maxScatTiles);
+  }
+  take(&c->rsplit, 4 * (size_t)c->maxGatherTiles);
+  take(&c->mark, 4 * V);
+  bytes(&c->carryVal, gb * c->maxGatherTiles);
+  take(&c->carryFlag, 4 * (size_t)c->maxGatherTiles);
+  take(&c->ctl, sizeof(Ctl));
+  take(&c->stats, 16 * (size_t)kMaxRounds);
+  return used;
 }
 
 gas_status set_device(gas_core *c) {
@@ -444,6 +502,7 @@ bool core_graph(gas_core_s *c, CoreGraph *out) {
   out->edgeBytes = c->edgeBytes;
   out->hInOff = &c->hInOff;
   out->hOutOff = &c->hOutOff;
+  out->maxOutDeg = c->maxOutDeg;
   return true;
 }
 }  // namespace internal
@@ -521,34 +580,49 @@ gas_status gas_core_set_graph(gas_core *c, int32_t nV, int32_t nE, const int32_t
   gas_status st = set_device(c);
   if (st) return st;
   if (c->stream) cudaStreamSynchronize(c->stream);
-  free_graph(c);
+  free_graph(c, false);
+  auto give_up = [c](gas_status s) {  // no graph, and no memory kept for one
+    free_graph(c);
+    return s;
+  };
+
+  // working memory of the build, given back at its end: the edge list, the
+  // edge data in edge-list order, the sorts, the bins' counts
+  const size_t listBytes = ((size_t)std::max(nE, 1) * 4 + 255) & ~(size_t)255;
+  const size_t edBytes = ((size_t)edgeBytes * std::max(nE, 1) + 255) & ~(size_t)255;
+  const size_t sortBytes = sort_scratch_bytes(nV, nE, nullptr, nullptr);
+  unsigned char *work = nullptr;
+  cudaError_t e = cudaMalloc((void **)&work, 256 + 2 * listBytes + edBytes + sortBytes);
+  if (e != cudaSuccess) return give_up(cuda_fail(e, "setGraph edge list upload"));
+  struct Release {
+    unsigned char *p;
+    ~Release() { cudaFree(p); }
+  } release{work};
+  DegreeBins *dCounts = reinterpret_cast<DegreeBins *>(work);
+  int32_t *dS = reinterpret_cast<int32_t *>(work + 256);
+  int32_t *dD = reinterpret_cast<int32_t *>(work + 256 + listBytes);
+  unsigned char *dEd = work + 256 + 2 * listBytes;
+  SortScratch sx;
+  sort_scratch_bytes(nV, nE, &sx, dEd + edBytes);
+  auto A = [&](cudaError_t r) {
+    if (e == cudaSuccess) e = r;
+  };
 
   // the edge list on the device: id check, then CSC (gather) and CSR
   // (scatter) by stable radix sorts (gas_graph_build.cu)
-  int32_t *dS = nullptr, *dD = nullptr;
-  cudaError_t e0 = dalloc(&dS, (size_t)nE);
-  if (e0 == cudaSuccess) e0 = dalloc(&dD, (size_t)nE);
-  if (e0 == cudaSuccess && nE > 0)
-    e0 = cudaMemcpyAsync(dS, srcs, sizeof(int32_t) * nE, cudaMemcpyHostToDevice, c->stream);
-  if (e0 == cudaSuccess && nE > 0)
-    e0 = cudaMemcpyAsync(dD, dsts, sizeof(int32_t) * nE, cudaMemcpyHostToDevice, c->stream);
-  auto drop_list = [&] {
-    if (dS) cudaFree(dS);
-    if (dD) cudaFree(dD);
-  };
-  if (e0 != cudaSuccess) {
-    drop_list();
-    return cuda_fail(e0, "setGraph edge list upload");
+  if (nE > 0) {
+    A(cudaMemcpyAsync(dS, srcs, sizeof(int32_t) * nE, cudaMemcpyHostToDevice, c->stream));
+    A(cudaMemcpyAsync(dD, dsts, sizeof(int32_t) * nE, cudaMemcpyHostToDevice, c->stream));
+    if (edgeBytes > 0)
+      A(cudaMemcpyAsync(dEd, edgeData, (size_t)edgeBytes * nE, cudaMemcpyHostToDevice, c->stream));
+    if (e != cudaSuccess) return give_up(cuda_fail(e, "setGraph edge list upload"));
   }
-  long long bad = -1;
-  st = device_first_bad_edge(c->stream, nV, nE, dS, dD, &bad);
-  if (st == GAS_OK && bad >= 0)
-    st = fail(GAS_ERR_INVALID, "edge %lld (%d -> %d) has a vertex id outside [0, %d)", bad,
-              srcs[bad], dsts[bad], nV);
-  if (st) {
-    drop_list();
-    return st;
-  }
+  EdgeCheck check;
+  st = device_check_edges(c->stream, nV, nE, dS, dD, work, &check);
+  if (st == GAS_OK && check.firstBad >= 0)
+    st = fail(GAS_ERR_INVALID, "edge %lld (%d -> %d) has a vertex id outside [0, %d)", check.firstBad,
+              srcs[check.firstBad], dsts[check.firstBad], nV);
+  if (st) return give_up(st);
 
   c->nV = nV;
   c->nE = nE;
@@ -557,64 +631,70 @@ gas_status gas_core_set_graph(gas_core *c, int32_t nV, int32_t nE, const int32_t
   c->gatherBytes = gatherBytes;
   c->maxGatherTiles = (int32_t)(((long long)nV + nE) / GAS_GATHER_TILE + 2);
   c->maxScatTiles = (int32_t)(((long long)nV + nE) / GAS_SCATTER_TILE + 2);
-
-  cudaError_t e = cudaSuccess;
-  auto A = [&](cudaError_t r) {
-    if (e == cudaSuccess) e = r;
-  };
-  A(dalloc(&c->inOff, (size_t)nV + 1));
-  // whole 16-byte quads: the dense pass reads source ids (and 4-byte edge
-  // data) four at a time, up to the quad that holds a vertex's last edge
-  A(dalloc(&c->inSrc, (size_t)nE + 4));
-  A(dalloc(&c->outOff, (size_t)nV + 1));
-  A(dalloc(&c->outDst, (size_t)nE));
-  if (edgeBytes > 0) A(cudaMalloc(&c->ed, (size_t)edgeBytes * ((size_t)nE + 4)));
-  if (edgeBytes > 0) A(dalloc(&c->cscPerm, (size_t)nE));
+  c->bitWords = (nV + 31) / 32;
   const bool edgeMap = c->edgeScatterOn && edgeBytes > 0;
+  // bounds on the vertices of more than kChunkEdges in-edges and their chunks
+  const int32_t maxHubs = nE / (gas::detail::kChunkEdges + 1);
+  const int32_t maxChunks = nE / gas::detail::kChunkEdges + maxHubs;
+
+  const size_t need = carve_arena(c, nullptr, edgeMap, maxHubs, maxChunks);
+  if (c->arenaBytes < need || c->arenaBytes / 4 > need) {  // too small, or mostly idle
+    if (c->arena) cudaFree(c->arena);
+    c->arena = nullptr;
+    c->arenaBytes = 0;
+    A(cudaMalloc((void **)&c->arena, need));
+    if (e != cudaSuccess) return give_up(cuda_fail(e, "setGraph device allocation"));
+    c->arenaBytes = need;
+  }
+  carve_arena(c, c->arena, edgeMap, maxHubs, maxChunks);
   if (c->keepCsrPerm || edgeMap) A(dalloc(&c->csrPerm, (size_t)nE));
-  if (edgeMap) A(dalloc(&c->csr2csc, (size_t)nE));
-  if (e == cudaSuccess) {
-    st = device_build_adjacency(c->stream, nV, nE, dD, dS, c->inOff, c->inSrc, c->cscPerm);
-    if (st == GAS_OK)
-      st = device_build_adjacency(c->stream, nV, nE, dS, dD, c->outOff, c->outDst, c->csrPerm);
-    if (st == GAS_OK && edgeMap)
-      st = device_csr_to_csc(c->stream, nE, c->cscPerm, c->csrPerm, c->csr2csc);
-    if (st == GAS_OK && edgeBytes > 0 && nE > 0) {
-      void *dEd = nullptr;
-      A(cudaMalloc(&dEd, (size_t)edgeBytes * nE));
-      A(cudaMemcpyAsync(dEd, edgeData, (size_t)edgeBytes * nE, cudaMemcpyHostToDevice, c->stream));
-      if (e == cudaSuccess) st = device_gather_bytes(c->stream, dEd, c->cscPerm, nE, edgeBytes, c->ed);
-      A(cudaStreamSynchronize(c->stream));
-      if (dEd) cudaFree(dEd);
-    }
-    c->hInOff.resize((size_t)nV + 1);
-    c->hOutOff.resize((size_t)nV + 1);
-    A(cudaMemcpyAsync(c->hInOff.data(), c->inOff, sizeof(int32_t) * ((size_t)nV + 1),
-                      cudaMemcpyDeviceToHost, c->stream));
-    A(cudaMemcpyAsync(c->hOutOff.data(), c->outOff, sizeof(int32_t) * ((size_t)nV + 1),
-                      cudaMemcpyDeviceToHost, c->stream));
-    A(cudaStreamSynchronize(c->stream));
-  }
-  drop_list();
-  if (st != GAS_OK || e != cudaSuccess) {
-    free_graph(c);
-    return st != GAS_OK ? st : cuda_fail(e, "setGraph build");
-  }
+  if (e != cudaSuccess) return give_up(cuda_fail(e, "setGraph device allocation"));
+
+  st = device_build_adjacency(c->stream, nV, nE, dD, dS, check.dstSorted, c->inOff, c->inSrc, c->cscPerm, sx);
+  if (st == GAS_OK)
+    st = device_build_adjacency(c->stream, nV, nE, dS, dD, check.srcSorted, c->outOff, c->outDst,
+                                c->csrPerm, sx);
+  if (st == GAS_OK && edgeMap)
+    st = device_csr_to_csc(c->stream, nE, c->cscPerm, c->csrPerm, c->csr2csc);
+  if (st == GAS_OK && edgeBytes > 0 && nE > 0)
+    st = device_gather_bytes(c->stream, dEd, c->cscPerm, nE, edgeBytes, c->ed);
+  // in-degree bins of the dense pass, heaviest first: the order in which it
+  // hands out work units
+  A(cudaMemsetAsync(dCounts, 0, sizeof(DegreeBins), c->stream));
+  const HubChunks hubs = {c->chunkVertex, c->chunkBegin, c->chunkFirst, c->chunkCount, c->chunkSlot};
+  if (st == GAS_OK && e == cudaSuccess)
+    st = device_degree_bins(c->stream, nV, c->inOff, c->outOff, maxHubs, c->bins, hubs, dCounts, sx);
+  if (st) return give_up(st);
+  A(cudaMemsetAsync(c->mark, 0, sizeof(int32_t) * std::max(nV, 1), c->stream));
+  A(cudaMemsetAsync(c->retBits, 0, sizeof(uint32_t) * 3 * std::max(c->bitWords, 1), c->stream));
+  A(cudaMemsetAsync(c->chunkArrive, 0, sizeof(unsigned) * std::max(maxHubs, 1), c->stream));
+  A(cudaMemsetAsync(c->carryFlag, 0, sizeof(unsigned) * c->maxGatherTiles, c->stream));
+  A(cudaMemsetAsync(c->ctl, 0, sizeof(Ctl), c->stream));
+  A(cudaMemsetAsync(c->vd, 0, (size_t)vertexBytes * std::max(nV, 1), c->stream));
+  c->hInOff.resize((size_t)nV + 1);
+  c->hOutOff.resize((size_t)nV + 1);
+  DegreeBins bins;
+  A(cudaMemcpyAsync(c->hInOff.data(), c->inOff, sizeof(int32_t) * ((size_t)nV + 1),
+                    cudaMemcpyDeviceToHost, c->stream));
+  A(cudaMemcpyAsync(c->hOutOff.data(), c->outOff, sizeof(int32_t) * ((size_t)nV + 1),
+                    cudaMemcpyDeviceToHost, c->stream));
+  A(cudaMemcpyAsync(&bins, dCounts, sizeof(bins), cudaMemcpyDeviceToHost, c->stream));
+  A(cudaStreamSynchronize(c->stream));
+  if (e != cudaSuccess) return give_up(cuda_fail(e, "setGraph build"));
   if (edgeMap && !c->keepCsrPerm) {  // only the composed map is needed
     cudaFree(c->csrPerm);
     c->csrPerm = nullptr;
   }
-  A(cudaMalloc(&c->vd, (size_t)vertexBytes * std::max(nV, 1)));
-  A(cudaMalloc(&c->vnew, (size_t)vertexBytes * std::max(nV, 1)));
-  A(cudaMalloc(&c->valt, (size_t)vertexBytes * std::max(nV, 1)));
-  c->bitWords = (nV + 31) / 32;
-  A(dalloc(&c->retBits, 3 * (size_t)c->bitWords));
-  c->maxInDeg = 0;
-  c->maxOutDeg = 0;
-  for (int32_t v = 0; v < nV; ++v) {
-    c->maxInDeg = std::max(c->maxInDeg, c->hInOff[(size_t)v + 1] - c->hInOff[v]);
-    c->maxOutDeg = std::max(c->maxOutDeg, c->hOutOff[(size_t)v + 1] - c->hOutOff[v]);
-  }
+  c->maxInDeg = bins.maxIn;
+  c->maxOutDeg = bins.maxOut;
+  c->nMid = bins.nMid;
+  c->nSmall = bins.nSmall;
+  c->nTiny = bins.nTiny + bins.nZero;
+  c->binMid = c->bins + bins.nHub;
+  c->binSmall = c->binMid + bins.nMid;
+  c->binTiny = c->binSmall + bins.nSmall;
+  c->nChunks = bins.nChunks;
+  c->nChunkVertices = bins.nHub;
   if (c->maxInDeg <= GAS_TPV_MAX_DEGREE && c->maxOutDeg <= GAS_TPV_MAX_DEGREE) {  // fused rounds
     A(cudaMalloc(&c->fcell, (size_t)GAS_FUSED_CELL_BYTES(vertexBytes) * std::max(nV, 1)));
     // fixed-width adjacency rows: a vertex's neighbours in one or two 16-byte
@@ -624,6 +704,7 @@ gas_status gas_core_set_graph(gas_core *c, int32_t nV, int32_t nE, const int32_t
     A(dalloc(&c->ellIn, cells));
     A(dalloc(&c->ellOut, cells));
     if (edgeBytes > 0) A(cudaMalloc(&c->ellEd, cells * edgeBytes));
+    A(dalloc(&c->frontBits, 3 * (size_t)c->bitWords));
     if (e == cudaSuccess && nV > 0) {
       const int blocks = (int)std::min<int64_t>(((int64_t)nV + 255) / 256, 65535LL * 32);
       ell_rows_kernel<<<blocks, 256, 0, c->stream>>>(nV, c->inOff, c->inSrc, c->ed, edgeBytes,
@@ -632,98 +713,10 @@ gas_status gas_core_set_graph(gas_core *c, int32_t nV, int32_t nE, const int32_t
                                                      c->ellWidth, c->ellOut, nullptr);
       A(cudaGetLastError());
     }
-    A(dalloc(&c->frontBits, 3 * (size_t)c->bitWords));
-  }
-  // in-degree bins of the dense pass
-  std::vector<int32_t> bMid, bSmall, bTiny, chV, chB, chF, chC, chS;
-  for (int32_t v = 0; v < nV; ++v) {
-    const int32_t deg = c->hInOff[(size_t)v + 1] - c->hInOff[v];
-    if (deg <= GAS_TPV_MAX_DEGREE) {
-      bTiny.push_back(v);
-    } else if (deg <= 64) {
-      bSmall.push_back(v);
-    } else if (deg <= gas::detail::kChunkEdges) {
-      bMid.push_back(v);
-    } else {
-      const int32_t nch = (deg + gas::detail::kChunkEdges - 1) / gas::detail::kChunkEdges;
-      const int32_t first = (int32_t)chV.size(), slot = (int32_t)(chS.empty() ? 0 : chS.back() + 1);
-      for (int32_t k = 0; k < nch; ++k) {
-        chV.push_back(v);
-        chB.push_back(c->hInOff[v] + k * gas::detail::kChunkEdges);
-        chF.push_back(first);
-        chC.push_back(nch);
-        chS.push_back(slot);
-      }
-    }
-  }
-  // heaviest first: the dense pass hands out work units in this order
-  const auto byInDegDesc = [c](int32_t x, int32_t y) {
-    return c->hInOff[(size_t)x + 1] - c->hInOff[x] > c->hInOff[(size_t)y + 1] - c->hInOff[y];
-  };
-  std::stable_sort(bMid.begin(), bMid.end(), byInDegDesc);
-  std::stable_sort(bSmall.begin(), bSmall.end(), byInDegDesc);
-  c->nMid = (int32_t)bMid.size();
-  c->nSmall = (int32_t)bSmall.size();
-  c->nTiny = (int32_t)bTiny.size();
-  c->nChunks = (int32_t)chV.size();
-  c->nChunkVertices = chS.empty() ? 0 : chS.back() + 1;
-  A(dalloc(&c->binMid, bMid.size()));
-  A(dalloc(&c->binSmall, bSmall.size()));
-  A(dalloc(&c->binTiny, bTiny.size()));
-  A(dalloc(&c->chunkVertex, chV.size()));
-  A(dalloc(&c->chunkBegin, chB.size()));
-  A(dalloc(&c->chunkFirst, chF.size()));
-  A(dalloc(&c->chunkCount, chC.size()));
-  A(dalloc(&c->chunkSlot, chS.size()));
-  A(dalloc(&c->chunkArrive, (size_t)c->nChunkVertices));
-  A(dalloc(&c->chunkFlags, chV.size()));
-  A(cudaMalloc(&c->chunkVal, (size_t)((gatherBytes + 15) / 16 * 16) * std::max<size_t>(chV.size(), 1)));
-  for (int k = 0; k < 2; ++k) {
-    A(dalloc(&c->fvid[k], (size_t)nV));
-    A(dalloc(&c->fpre[k], (size_t)nV));
-    A(dalloc(&c->fbeg[k], (size_t)nV));
-    A(dalloc(&c->sbeg[k], (size_t)nV));
-    A(dalloc(&c->fsplit[k], (size_t)c->maxGatherTiles));
-    A(dalloc(&c->svid[k], (size_t)nV));
-    A(dalloc(&c->spre[k], (size_t)nV));
-    A(dalloc(&c->ssplit[k], (size_t)c->maxScatTiles));
-  }
-  A(dalloc(&c->rsplit, (size_t)c->maxGatherTiles));
-  A(dalloc(&c->mark, (size_t)nV));
-  const size_t gb = (size_t)((gatherBytes + 15) / 16 * 16);
-  A(cudaMalloc(&c->carryVal, gb * c->maxGatherTiles));
-  A(dalloc(&c->carryFlag, (size_t)c->maxGatherTiles));
-  A(dalloc(&c->ctl, 1));
-  A(dalloc(&c->stats, (size_t)kMaxRounds * 2));
-  if (e != cudaSuccess) {
-    free_graph(c);
-    return cuda_fail(e, "setGraph device allocation");
-  }
-  A(cudaMemsetAsync(c->mark, 0, sizeof(int32_t) * std::max(nV, 1), c->stream));
-  A(cudaMemsetAsync(c->retBits, 0, sizeof(uint32_t) * 3 * std::max(c->bitWords, 1), c->stream));
-  if (c->frontBits)
-    A(cudaMemsetAsync(c->frontBits, 0, sizeof(uint32_t) * 3 * std::max(c->bitWords, 1), c->stream));
-  auto up = [&](int32_t *dst, const std::vector<int32_t> &src) {
-    if (!src.empty())
-      A(cudaMemcpyAsync(dst, src.data(), sizeof(int32_t) * src.size(), cudaMemcpyHostToDevice,
-                        c->stream));
-  };
-  up(c->binMid, bMid);
-  up(c->binSmall, bSmall);
-  up(c->binTiny, bTiny);
-  up(c->chunkVertex, chV);
-  up(c->chunkBegin, chB);
-  up(c->chunkFirst, chF);
-  up(c->chunkCount, chC);
-  up(c->chunkSlot, chS);
-  A(cudaMemsetAsync(c->chunkArrive, 0, sizeof(unsigned) * std::max(c->nChunkVertices, 1), c->stream));
-  A(cudaMemsetAsync(c->carryFlag, 0, sizeof(unsigned) * c->maxGatherTiles, c->stream));
-  A(cudaMemsetAsync(c->ctl, 0, sizeof(Ctl), c->stream));
-  A(cudaMemsetAsync(c->vd, 0, (size_t)vertexBytes * std::max(nV, 1), c->stream));
-  A(cudaStreamSynchronize(c->stream));  // host staging buffers die here
-  if (e != cudaSuccess) {
-    free_graph(c);
-    return cuda_fail(e, "setGraph upload");
+    if (e == cudaSuccess)
+      A(cudaMemsetAsync(c->frontBits, 0, sizeof(uint32_t) * 3 * std::max(c->bitWords, 1), c->stream));
+    A(cudaStreamSynchronize(c->stream));
+    if (e != cudaSuccess) return give_up(cuda_fail(e, "setGraph device allocation"));
   }
   c->haveGraph = true;
   c->dirty = 0;

@@ -1,27 +1,41 @@
-// Device graph builder: CSR / CSC from an edge list on the GPU.
+// Device graph builder: CSR / CSC from an edge list on the GPU, and the
+// degree bins of the pull passes.
 //
 // The reference builds both adjacencies on the host (util.h:44-121,
 // edgeListToCSR/CSC; gpugas.h:212-322 copies them up).  Here the edge list
 // is copied to the device once and each adjacency is a stable LSD radix
-// sort of (key, edge index) pairs, 8-bit digits:
+// sort of (key, payload) pairs with digits of at most 8 bits (the key bits
+// divided evenly over the passes: fewer digits, longer runs):
 //
 //   per pass:  block histograms of the digit (4096 edges per block)
 //              -> exclusive scan in digit-major order (a digit's blocks in
 //                 order after every smaller digit)
-//              -> scatter: each block ranks its edges per digit in edge
-//                 order (warp match + per-warp counts), so equal keys keep
-//                 edge-list order
+//              -> scatter: each warp ranks 512 consecutive edges per digit
+//                 in edge order (warp match + per-warp counts), the block
+//                 stages its edges in shared memory in digit order and
+//                 writes each digit's run with consecutive threads
 //
 // which gives the same order as build_adjacency's stable counting sort
-// (in-edges of a vertex in edge-list order).  Offsets come from per-key
-// counts and an exclusive scan; adjacency and edge data are gathered by the
-// sorted edge indices (the permutation).
+// (in-edges of a vertex in edge-list order).  The payload is the adjacency
+// itself, or the edge index where the permutation is wanted (edge data).
+// Offsets are binary searches in the sorted keys (counters per key are
+// contended by every SM at a power-law graph's hubs).  An edge list already in key order -- files list edges by
+// source -- needs no sort on that side.
+//
+// A scatter moves 8 bytes in and 8 out an edge and pass.  On 128 M edges
+// (R-MAT-22, three passes) it takes 1.36 / 1.37 / 1.13 ms, about 1.5 TB/s,
+// bound by the ranking (match, shared-memory counts) rather than by HBM; a
+// block that wrote its edges unstaged, one 256-edge step at a time with
+// four block barriers a step, took 2.81 / 2.80 / 1.60 ms.  The offsets'
+// searches take 0.12 ms a side there (per-key counters 1.46 and 2.15 ms).
+// Degree bins: 0.14 ms (a host loop with std::stable_sort took about 12 ms
+// on R-MAT-20).
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <vector>
 
-#include "gas_gb300/detail/primitives.cuh"
+#include "gas_gb300/detail/dense.cuh"
 #include "gas_internal.h"
 
 using gas::internal::cuda_fail;
@@ -29,16 +43,17 @@ using gas::internal::fail;
 
 namespace {
 
-constexpr int kBins = 256;
+constexpr int kBins = 256;  // at most 8 bits a digit
 constexpr int kRThreads = 256;
 constexpr int kRItems = 16;
 constexpr int kRTile = kRThreads * kRItems;  // edges per sort block
+constexpr int kRWarps = kRThreads / 32;
 constexpr int kSThreads = 1024;
 constexpr int kSItems = 8;
 constexpr int kSTile = kSThreads * kSItems;  // elements per scan block
 
-__global__ void radix_hist_kernel(const uint32_t *keys, long long n, int shift, int nBlocks,
-                                  uint32_t *hist) {
+__global__ void radix_hist_kernel(const uint32_t *keys, long long n, int shift, uint32_t digitMask,
+                                  int nBlocks, uint32_t *hist) {
   __shared__ uint32_t h[kBins];
   h[threadIdx.x] = 0u;
   __syncthreads();
@@ -46,52 +61,99 @@ __global__ void radix_hist_kernel(const uint32_t *keys, long long n, int shift, 
 #pragma unroll 4
   for (int i = 0; i < kRItems; ++i) {
     const long long idx = base + (long long)i * kRThreads + threadIdx.x;
-    if (idx < n) atomicAdd(&h[(keys[idx] >> shift) & (kBins - 1)], 1u);
+    if (idx < n) atomicAdd(&h[(keys[idx] >> shift) & digitMask], 1u);
   }
   __syncthreads();
-  hist[(size_t)threadIdx.x * nBlocks + blockIdx.x] = h[threadIdx.x];
+  if (threadIdx.x <= digitMask) hist[(size_t)threadIdx.x * nBlocks + blockIdx.x] = h[threadIdx.x];
 }
 
 // Stable scatter of one pass.  vals == null stands for the identity
-// (edge index), the first pass's payload.
-__global__ void radix_scatter_kernel(const uint32_t *keysIn, const uint32_t *valsIn,
-                                     uint32_t *keysOut, uint32_t *valsOut, long long n, int shift,
-                                     int nBlocks, const uint32_t *histScan) {
-  __shared__ uint32_t run[kBins];
-  __shared__ uint32_t warpOff[kRThreads / 32][kBins];
+// (edge index), the first pass's payload; keysOut == null drops the keys.
+__global__ void __launch_bounds__(kRThreads)
+    radix_scatter_kernel(const uint32_t *keysIn, const uint32_t *valsIn, uint32_t *keysOut,
+                         uint32_t *valsOut, long long n, int shift, uint32_t digitMask, int nBlocks,
+                         const uint32_t *histScan) {
+  __shared__ uint32_t cnt[kRWarps][kBins];  // per warp and digit: edges so far, then first slot
+  __shared__ uint32_t start[kBins];         // the digit's first slot in the tile
+  __shared__ uint32_t gbase[kBins];         // its global position minus that slot
+  __shared__ uint32_t buf[kRTile];
+  __shared__ uint32_t warpTot[kRWarps];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned ltMask = (1u << lane) - 1u;
-  run[tid] = histScan[(size_t)tid * nBlocks + blockIdx.x];
+#pragma unroll
+  for (int w = 0; w < kRWarps; ++w) cnt[w][tid] = 0u;
   const long long base = (long long)blockIdx.x * kRTile;
-  for (int i = 0; i < kRItems; ++i) {
-    const long long idx = base + (long long)i * kRThreads + tid;
-    const bool valid = idx < n;
-    const uint32_t key = valid ? keysIn[idx] : 0u;
-    const uint32_t d = (key >> shift) & (kBins - 1);
+  const int count = (int)min((long long)kRTile, n - base);
+  const int first = warp * (32 * kRItems) + lane;  // this thread's edges: first + 32 j
+  uint32_t key[kRItems], pos[kRItems];
+#pragma unroll
+  for (int j = 0; j < kRItems; ++j)
+    key[j] = first + 32 * j < count ? keysIn[base + first + 32 * j] : 0u;
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < kRItems; ++j) {
+    const bool valid = first + 32 * j < count;
+    const uint32_t d = (key[j] >> shift) & digitMask;
     const unsigned peers = __match_any_sync(gas::detail::kFullMask, valid ? d : 0xffffffffu);
-    const int rank = __popc(peers & ltMask);
+    const uint32_t before = cnt[warp][d];
+    __syncwarp();
+    if (valid && (peers & ltMask) == 0u) cnt[warp][d] = before + (uint32_t)__popc(peers);
+    __syncwarp();
+    pos[j] = before + (uint32_t)__popc(peers & ltMask);
+  }
+  __syncthreads();
+  {  // digit tid: the warps' first slots, then the digit's own
+    uint32_t run = 0u;
 #pragma unroll
-    for (int w = 0; w < kRThreads / 32; ++w) warpOff[w][tid] = 0u;
-    __syncthreads();
-    if (valid && rank == 0) warpOff[warp][d] = (uint32_t)__popc(peers);
-    __syncthreads();
-    {  // per digit: offsets of the warps of this step, after the earlier steps
-      uint32_t r = run[tid];
+    for (int w = 0; w < kRWarps; ++w) {
+      const uint32_t c = cnt[w][tid];
+      cnt[w][tid] = run;
+      run += c;
+    }
+    uint32_t incl = run;
 #pragma unroll
-      for (int w = 0; w < kRThreads / 32; ++w) {
-        const uint32_t c = warpOff[w][tid];
-        warpOff[w][tid] = r;
-        r += c;
-      }
-      run[tid] = r;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(gas::detail::kFullMask, incl, o);
+      if (lane >= o) incl += y;
     }
+    if (lane == 31) warpTot[warp] = incl;
     __syncthreads();
-    if (valid) {
-      const uint32_t pos = warpOff[warp][d] + (uint32_t)rank;
-      keysOut[pos] = key;
-      valsOut[pos] = valsIn ? valsIn[idx] : (uint32_t)idx;
+    uint32_t excl = incl - run;
+#pragma unroll
+    for (int w = 0; w < kRWarps; ++w)
+      if (w < warp) excl += warpTot[w];
+    start[tid] = excl;
+    gbase[tid] = (tid <= (int)digitMask ? histScan[(size_t)tid * nBlocks + blockIdx.x] : 0u) - excl;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < kRItems; ++j)
+    if (first + 32 * j < count) {
+      const uint32_t d = (key[j] >> shift) & digitMask;
+      pos[j] += start[d] + cnt[warp][d];
+      buf[pos[j]] = key[j];
     }
-    __syncthreads();
+  __syncthreads();
+  uint32_t dst[kRItems];
+#pragma unroll
+  for (int j = 0; j < kRItems; ++j) {
+    const int i = tid + kRThreads * j;
+    if (i < count) {
+      const uint32_t k = buf[i];
+      dst[j] = gbase[(k >> shift) & digitMask] + (uint32_t)i;
+      if (keysOut) keysOut[dst[j]] = k;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < kRItems; ++j)
+    if (first + 32 * j < count)
+      buf[pos[j]] = valsIn ? valsIn[base + first + 32 * j] : (uint32_t)(base + first + 32 * j);
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < kRItems; ++j) {
+    const int i = tid + kRThreads * j;
+    if (i < count) valsOut[dst[j]] = buf[i];
   }
 }
 
@@ -141,32 +203,48 @@ __global__ void scan_add_kernel(uint32_t *data, long long n, const uint32_t *off
   if (i < n) data[i] += offs[i / kSTile];
 }
 
-gas_status exclusive_scan(uint32_t *data, long long n, cudaStream_t s) {
-  if (n <= 0) return GAS_OK;
-  const long long blocks = (n + kSTile - 1) / kSTile;
-  if (blocks == 1) {
-    scan_block_kernel<<<1, kSThreads, 0, s>>>(data, n, nullptr);
-    cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? GAS_OK : cuda_fail(e, "graph build scan");
-  }
-  uint32_t *sums = nullptr;
-  cudaError_t e = cudaMallocAsync(&sums, sizeof(uint32_t) * blocks, s);
-  if (e != cudaSuccess) return cuda_fail(e, "graph build scan");
-  scan_block_kernel<<<(unsigned)blocks, kSThreads, 0, s>>>(data, n, sums);
-  gas_status st = exclusive_scan(sums, blocks, s);
-  if (st == GAS_OK) {
-    scan_add_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(data, n, sums);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) st = cuda_fail(e, "graph build scan");
-  }
-  cudaFreeAsync(sums, s);
-  return st;
+// Words exclusive_scan needs for n elements (its block sums, level by level).
+size_t scan_words(long long n) {
+  size_t w = 0;
+  for (long long b = (n + kSTile - 1) / kSTile; b > 1; b = (b + kSTile - 1) / kSTile) w += (size_t)b;
+  return w + 1;
 }
 
-__global__ void count_keys_kernel(const int32_t *keys, long long n, uint32_t *cnt) {
+// In place; `sums` holds scan_words(n) words.
+gas_status exclusive_scan(uint32_t *data, long long n, uint32_t *sums, cudaStream_t s) {
+  if (n <= 0) return GAS_OK;
+  const long long blocks = (n + kSTile - 1) / kSTile;
+  scan_block_kernel<<<(unsigned)blocks, kSThreads, 0, s>>>(data, n, blocks > 1 ? sums : nullptr);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_fail(e, "graph build scan");
+  if (blocks == 1) return GAS_OK;
+  gas_status st = exclusive_scan(sums, blocks, sums + blocks, s);
+  if (st) return st;
+  scan_add_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(data, n, sums);
+  e = cudaGetLastError();
+  return e == cudaSuccess ? GAS_OK : cuda_fail(e, "graph build scan");
+}
+
+// off[v] = first position of a key >= v in the sorted keys, v = 0..nV.
+__global__ void offsets_kernel(const uint32_t *keys, long long n, int32_t nV, int32_t *off) {
+  for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v <= nV;
+       v += (long long)gridDim.x * blockDim.x) {
+    long long lo = 0, hi = n;
+    while (lo < hi) {
+      const long long mid = (lo + hi) >> 1;
+      if (keys[mid] < (uint32_t)v)
+        lo = mid + 1;
+      else
+        hi = mid;
+    }
+    off[v] = (int32_t)lo;
+  }
+}
+
+__global__ void iota_kernel(uint32_t *out, long long n) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
-    atomicAdd(cnt + keys[i], 1u);
+    out[i] = (uint32_t)i;
 }
 
 __global__ void gather_kernel(const int32_t *src, const uint32_t *perm, long long n, int32_t *dst) {
@@ -201,12 +279,116 @@ __global__ void scatter_bytes_kernel(const unsigned char *in, const uint32_t *pe
   }
 }
 
+// Ids in [0, nV)?  *firstBad = the first edge with one outside; also
+// whether each end's ids come in ascending order (unsorted[0]: a,
+// unsorted[1]: b).
 __global__ void check_ids_kernel(const int32_t *a, const int32_t *b, long long n, int32_t nV,
-                                 unsigned long long *firstBad) {
+                                 unsigned long long *firstBad, unsigned *unsorted) {
+  bool ua = false, ub = false;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    if ((unsigned)a[i] >= (unsigned)nV || (unsigned)b[i] >= (unsigned)nV)
+       i += (long long)gridDim.x * blockDim.x) {
+    const int32_t x = a[i], y = b[i];
+    if ((unsigned)x >= (unsigned)nV || (unsigned)y >= (unsigned)nV)
       atomicMin(firstBad, (unsigned long long)i);
+    if (i > 0) {
+      ua |= a[i - 1] > x;
+      ub |= b[i - 1] > y;
+    }
+  }
+  // one store per warp that saw a descent (every writer stores the same)
+  if (__any_sync(gas::detail::kFullMask, ua) && (threadIdx.x & 31) == 0) unsorted[0] = 1u;
+  if (__any_sync(gas::detail::kFullMask, ub) && (threadIdx.x & 31) == 0) unsorted[1] = 1u;
+}
+
+// Sort key of each vertex's degree class, in the order the pull pass hands
+// its work out: hubs (in-degree > kChunkEdges) first, then in-degree 65..
+// kChunkEdges and 9..64 by falling degree, then 1..8, then no in-edges.
+// Adds the class counts, the hubs' chunks and the largest degrees to *c.
+__global__ void degree_class_kernel(const int32_t *inOff, const int32_t *outOff, int32_t nV,
+                                    uint32_t *key, gas::internal::DegreeBins *c) {
+  using gas::detail::kChunkEdges;
+  __shared__ int sums[8];
+  if (threadIdx.x < 8) sums[threadIdx.x] = 0;
+  __syncthreads();
+  int n[5] = {0, 0, 0, 0, 0}, chunks = 0, maxIn = 0, maxOut = 0;
+  for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < nV;
+       v += (long long)gridDim.x * blockDim.x) {
+    const int d = inOff[v + 1] - inOff[v];
+    maxIn = max(maxIn, d);
+    maxOut = max(maxOut, outOff[v + 1] - outOff[v]);
+    uint32_t k;
+    if (d > kChunkEdges) {
+      k = 0u;
+      ++n[0];
+      chunks += (d + kChunkEdges - 1) / kChunkEdges;
+    } else if (d > 64) {
+      k = 1u + (uint32_t)(kChunkEdges - d);
+      ++n[1];
+    } else if (d > GAS_TPV_MAX_DEGREE) {
+      k = 1u + kChunkEdges + (uint32_t)(64 - d);
+      ++n[2];
+    } else {
+      k = 65u + kChunkEdges + (d == 0 ? 1u : 0u);
+      ++n[d == 0 ? 4 : 3];
+    }
+    key[v] = k;
+  }
+#pragma unroll
+  for (int i = 0; i < 5; ++i) {
+    const int w = __reduce_add_sync(gas::detail::kFullMask, n[i]);
+    if ((threadIdx.x & 31) == 0 && w) atomicAdd(&sums[i], w);
+  }
+  const int wc = __reduce_add_sync(gas::detail::kFullMask, chunks);
+  const int wi = __reduce_max_sync(gas::detail::kFullMask, maxIn);
+  const int wo = __reduce_max_sync(gas::detail::kFullMask, maxOut);
+  if ((threadIdx.x & 31) == 0) {
+    if (wc) atomicAdd(&sums[5], wc);
+    atomicMax(&sums[6], wi);
+    atomicMax(&sums[7], wo);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (sums[0]) atomicAdd(&c->nHub, sums[0]);
+    if (sums[1]) atomicAdd(&c->nMid, sums[1]);
+    if (sums[2]) atomicAdd(&c->nSmall, sums[2]);
+    if (sums[3]) atomicAdd(&c->nTiny, sums[3]);
+    if (sums[4]) atomicAdd(&c->nZero, sums[4]);
+    if (sums[5]) atomicAdd(&c->nChunks, sums[5]);
+    atomicMax(&c->maxIn, sums[6]);
+    atomicMax(&c->maxOut, sums[7]);
+  }
+}
+
+// Chunks of each hub (hubs: the first c->nHub entries of `bins`), 0 past them.
+__global__ void hub_count_kernel(const int32_t *bins, const int32_t *inOff,
+                                 const gas::internal::DegreeBins *c, int32_t maxHubs, uint32_t *count) {
+  const int n = c->nHub;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < maxHubs; i += gridDim.x * blockDim.x) {
+    const int v = i < n ? bins[i] : 0;
+    count[i] = i < n ? (uint32_t)((inOff[v + 1] - inOff[v] + gas::detail::kChunkEdges - 1) /
+                                  gas::detail::kChunkEdges)
+                     : 0u;
+  }
+}
+
+// The hubs' chunk entries (a warp per hub); first[i] = hub i's first chunk.
+__global__ void hub_chunks_kernel(const int32_t *bins, const int32_t *inOff,
+                                  const gas::internal::DegreeBins *c, const uint32_t *first,
+                                  gas::internal::HubChunks out) {
+  const int n = c->nHub, lane = threadIdx.x & 31;
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n;
+       i += (gridDim.x * blockDim.x) >> 5) {
+    const int v = bins[i], b = inOff[v];
+    const int nch = (inOff[v + 1] - b + gas::detail::kChunkEdges - 1) / gas::detail::kChunkEdges;
+    const int f = (int)first[i];
+    for (int k = lane; k < nch; k += 32) {
+      out.vertex[f + k] = v;
+      out.begin[f + k] = b + k * gas::detail::kChunkEdges;
+      out.first[f + k] = f;
+      out.count[f + k] = nch;
+      out.slot[f + k] = i;
+    }
+  }
 }
 
 __global__ void invert_kernel(const uint32_t *perm, long long n, uint32_t *inv) {
@@ -228,77 +410,145 @@ int grid_for(long long n) { return (int)std::max<long long>(1, std::min<long lon
 namespace gas {
 namespace internal {
 
-gas_status device_first_bad_edge(cudaStream_t s, int32_t nV, int32_t nE, const int32_t *dSrcs,
-                                 const int32_t *dDsts, long long *firstBad) {
-  *firstBad = -1;
+gas_status device_check_edges(cudaStream_t s, int32_t nV, int32_t nE, const int32_t *dSrcs,
+                              const int32_t *dDsts, void *scratch, EdgeCheck *out) {
+  *out = EdgeCheck();
   if (nE <= 0) return GAS_OK;
-  unsigned long long *d = nullptr, h = ~0ull;
-  cudaError_t e = cudaMallocAsync(&d, sizeof(h), s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(d, &h, sizeof(h), cudaMemcpyHostToDevice, s);
+  struct {
+    unsigned long long bad;
+    unsigned unsorted[2];
+  } h = {~0ull, {0u, 0u}};
+  cudaError_t e = cudaMemcpyAsync(scratch, &h, sizeof(h), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) {
-    check_ids_kernel<<<grid_for(nE), 256, 0, s>>>(dSrcs, dDsts, nE, nV, d);
+    unsigned long long *d = static_cast<unsigned long long *>(scratch);
+    check_ids_kernel<<<grid_for(nE), 256, 0, s>>>(dSrcs, dDsts, nE, nV, d,
+                                                  reinterpret_cast<unsigned *>(d + 1));
     e = cudaGetLastError();
   }
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&h, d, sizeof(h), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&h, scratch, sizeof(h), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (d) cudaFreeAsync(d, s);
   if (e != cudaSuccess) return cuda_fail(e, "edge id check");
-  if (h != ~0ull) *firstBad = (long long)h;
+  if (h.bad != ~0ull) out->firstBad = (long long)h.bad;
+  out->srcSorted = h.unsorted[0] == 0u;
+  out->dstSorted = h.unsorted[1] == 0u;
   return GAS_OK;
 }
 
-gas_status device_build_adjacency(cudaStream_t s, int32_t nV, int32_t nE, const int32_t *dKey,
-                                  const int32_t *dOther, int32_t *dOff, int32_t *dAdj,
-                                  uint32_t *dPermOut) {
-  cudaError_t e = cudaSuccess;
-  const long long n = nE;
-  // offsets: per-key counts, exclusive scan over V + 1 entries
-  e = cudaMemsetAsync(dOff, 0, sizeof(int32_t) * ((size_t)nV + 1), s);
-  if (e != cudaSuccess) return cuda_fail(e, "graph build");
-  if (n > 0) count_keys_kernel<<<grid_for(n), 256, 0, s>>>(dKey, n, reinterpret_cast<uint32_t *>(dOff));
-  gas_status st = exclusive_scan(reinterpret_cast<uint32_t *>(dOff), (long long)nV + 1, s);
-  if (st || n == 0) return st;
-  // stable radix sort of (key, edge index)
-  int bits = 1;
-  while (bits < 31 && (1ll << bits) < nV) ++bits;
-  const int passes = (bits + 7) / 8;
+namespace {
+
+// Passes of a sort of `bits`-bit keys and the digit width of each.
+struct Digits {
+  int passes, bits;
+};
+Digits digits_for(int bits) {
+  Digits d;
+  d.passes = (bits + 7) / 8;
+  d.bits = (bits + d.passes - 1) / d.passes;
+  return d;
+}
+
+// Stable sort of n (key, payload) pairs by `bits`-bit keys; payload null:
+// the index.  The sorted payload goes to valsOut, the sorted keys to
+// *sortedKeys (inside the scratch) unless sortedKeys is null.
+gas_status radix_sort(cudaStream_t s, long long n, const uint32_t *keys, const uint32_t *vals, int bits,
+                      uint32_t *valsOut, const uint32_t **sortedKeys, const SortScratch &x) {
+  const Digits dg = digits_for(bits);
+  const uint32_t mask = (1u << dg.bits) - 1u;
   const int nBlocks = (int)((n + kRTile - 1) / kRTile);
-  uint32_t *k0 = nullptr, *k1 = nullptr, *v0 = nullptr, *v1 = nullptr, *hist = nullptr;
-  e = cudaMallocAsync(&k0, sizeof(uint32_t) * n, s);
-  if (e == cudaSuccess) e = cudaMallocAsync(&k1, sizeof(uint32_t) * n, s);
-  if (e == cudaSuccess) e = cudaMallocAsync(&v0, sizeof(uint32_t) * n, s);
-  if (e == cudaSuccess) e = cudaMallocAsync(&v1, sizeof(uint32_t) * n, s);
-  if (e == cudaSuccess) e = cudaMallocAsync(&hist, sizeof(uint32_t) * (size_t)kBins * nBlocks, s);
-  const uint32_t *kin = reinterpret_cast<const uint32_t *>(dKey);
-  const uint32_t *vin = nullptr;
-  uint32_t *kout = k0, *vout = v0;
-  for (int p = 0; p < passes && e == cudaSuccess; ++p) {
-    radix_hist_kernel<<<nBlocks, kRThreads, 0, s>>>(kin, n, 8 * p, nBlocks, hist);
+  const uint32_t *kin = keys, *vin = vals;
+  for (int p = 0; p < dg.passes; ++p) {
+    const bool lastPass = p + 1 == dg.passes;
+    uint32_t *kout = x.keys[p & 1];
+    // the last pass writes valsOut; before it the payload alternates
+    // between valsOut and the spare so that it never reads what it writes
+    uint32_t *vout = ((dg.passes - 1 - p) & 1) ? x.spare : valsOut;
+    radix_hist_kernel<<<nBlocks, kRThreads, 0, s>>>(kin, n, p * dg.bits, mask, nBlocks, x.hist);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return cuda_fail(e, "graph build sort");
+    gas_status st = exclusive_scan(x.hist, (long long)(mask + 1) * nBlocks, x.sums, s);
+    if (st) return st;
+    radix_scatter_kernel<<<nBlocks, kRThreads, 0, s>>>(
+        kin, vin, lastPass && !sortedKeys ? nullptr : kout, vout, n, p * dg.bits, mask, nBlocks, x.hist);
     e = cudaGetLastError();
-    if (e != cudaSuccess) break;
-    st = exclusive_scan(hist, (long long)kBins * nBlocks, s);
-    if (st) break;
-    radix_scatter_kernel<<<nBlocks, kRThreads, 0, s>>>(kin, vin, kout, vout, n, 8 * p, nBlocks,
-                                                       hist);
-    e = cudaGetLastError();
+    if (e != cudaSuccess) return cuda_fail(e, "graph build sort");
     kin = kout;
     vin = vout;
-    kout = kout == k0 ? k1 : k0;
-    vout = vout == v0 ? v1 : v0;
   }
-  if (e == cudaSuccess && st == GAS_OK) {
-    gather_kernel<<<grid_for(n), 256, 0, s>>>(dOther, vin, n, dAdj);
-    e = cudaGetLastError();
-    if (e == cudaSuccess && dPermOut)
-      e = cudaMemcpyAsync(dPermOut, vin, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s);
+  if (sortedKeys) *sortedKeys = kin;
+  return GAS_OK;
+}
+
+}  // namespace
+
+size_t sort_scratch_bytes(int32_t nV, int32_t nE, SortScratch *x, void *base) {
+  const long long n = std::max<long long>(std::max(nE, nV), 1);
+  const long long hist = (long long)kBins * ((n + kRTile - 1) / kRTile);
+  unsigned char *p = static_cast<unsigned char *>(base);
+  size_t used = 0;
+  auto take = [&](size_t words) {
+    uint32_t *r = reinterpret_cast<uint32_t *>(p + used);
+    used += (words * 4 + 255) & ~(size_t)255;
+    return r;
+  };
+  uint32_t *k0 = take(n), *k1 = take(n), *sp = take(n), *h = take(hist);
+  uint32_t *su = take(scan_words(std::max<long long>(hist, n)));
+  if (x) *x = SortScratch{{k0, k1}, sp, h, su};
+  return used;
+}
+
+gas_status device_build_adjacency(cudaStream_t s, int32_t nV, int32_t nE, const int32_t *dKey,
+                                  const int32_t *dOther, bool sorted, int32_t *dOff, int32_t *dAdj,
+                                  uint32_t *dPermOut, const SortScratch &x) {
+  const long long n = nE;
+  const uint32_t *keys = reinterpret_cast<const uint32_t *>(dKey);
+  cudaError_t e = cudaSuccess;
+  if (n > 0 && sorted) {
+    e = cudaMemcpyAsync(dAdj, dOther, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, s);
+    if (e == cudaSuccess && dPermOut) {
+      iota_kernel<<<grid_for(n), 256, 0, s>>>(dPermOut, n);
+      e = cudaGetLastError();
+    }
+    if (e != cudaSuccess) return cuda_fail(e, "graph build");
+  } else if (n > 0) {
+    int bits = 1;
+    while (bits < 31 && (1ll << bits) < nV) ++bits;
+    gas_status st = radix_sort(s, n, keys, dPermOut ? nullptr : reinterpret_cast<const uint32_t *>(dOther),
+                               bits, dPermOut ? dPermOut : reinterpret_cast<uint32_t *>(dAdj), &keys, x);
+    if (st) return st;
+    if (dPermOut) {
+      gather_kernel<<<grid_for(n), 256, 0, s>>>(dOther, dPermOut, n, dAdj);
+      e = cudaGetLastError();
+      if (e != cudaSuccess) return cuda_fail(e, "graph build");
+    }
   }
-  cudaFreeAsync(k0, s);
-  cudaFreeAsync(k1, s);
-  cudaFreeAsync(v0, s);
-  cudaFreeAsync(v1, s);
-  cudaFreeAsync(hist, s);
-  if (st) return st;
+  offsets_kernel<<<grid_for((long long)nV + 1), 256, 0, s>>>(keys, n, nV, dOff);
+  e = cudaGetLastError();
   return e == cudaSuccess ? GAS_OK : cuda_fail(e, "graph build");
+}
+
+gas_status device_degree_bins(cudaStream_t s, int32_t nV, const int32_t *inOff, const int32_t *outOff,
+                              int32_t maxHubs, int32_t *bins, const HubChunks &hubs, DegreeBins *dCounts,
+                              const SortScratch &x) {
+  if (nV <= 0) return GAS_OK;
+  int32_t *first = reinterpret_cast<int32_t *>(x.spare);
+  degree_class_kernel<<<std::min(grid_for(nV), 152 * 8), 256, 0, s>>>(inOff, outOff, nV, x.keys[1], dCounts);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_fail(e, "degree bins");
+  // keys below 2^11 (66 + kChunkEdges): two passes; keys[1] is free again
+  // when the second pass, whose keys are dropped, would write it
+  static_assert(gas::detail::kChunkEdges + 66 < (1 << 11), "degree class keys");
+  gas_status st = radix_sort(s, nV, x.keys[1], nullptr, 11, reinterpret_cast<uint32_t *>(bins), nullptr, x);
+  if (st) return st;
+  if (maxHubs > 0) {
+    uint32_t *cnt = reinterpret_cast<uint32_t *>(first);
+    hub_count_kernel<<<grid_for(maxHubs), 256, 0, s>>>(bins, inOff, dCounts, maxHubs, cnt);
+    st = exclusive_scan(cnt, maxHubs, x.sums, s);
+    if (st) return st;
+    hub_chunks_kernel<<<grid_for(32ll * maxHubs), 256, 0, s>>>(bins, inOff, dCounts, cnt, hubs);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return cuda_fail(e, "degree bins");
+  }
+  return GAS_OK;
 }
 
 gas_status device_csr_to_csc(cudaStream_t s, int32_t n, const uint32_t *cscPerm,

@@ -22,15 +22,43 @@ void build_adjacency(int32_t nV, int32_t nE, const int32_t *key, const int32_t *
                      std::vector<int32_t> &off, std::vector<int32_t> &adj,
                      std::vector<int32_t> *perm);
 
-// The same on the device (gas_graph_build.cu): stable radix sort of
-// (key, edge index); dOff[V+1], dAdj[E], optional dPerm[E].  Device arrays,
-// stream-ordered on `s`.
+// The same on the device (gas_graph_build.cu).  Working memory of its
+// sorts, for max(nV, nE) elements: sort_scratch_bytes sizes it, and with a
+// base address lays it out in *x.
+struct SortScratch {
+  uint32_t *keys[2];
+  uint32_t *spare;
+  uint32_t *hist;
+  uint32_t *sums;
+};
+size_t sort_scratch_bytes(int32_t nV, int32_t nE, SortScratch *x, void *base);
+// dOff[V+1], dAdj[E], optional dPerm[E] of a stable sort of the edges by
+// dKey.  `sorted`: the keys already ascend.  Device arrays, stream-ordered
+// on `s`.
 gas_status device_build_adjacency(cudaStream_t s, int32_t nV, int32_t nE, const int32_t *dKey,
-                                  const int32_t *dOther, int32_t *dOff, int32_t *dAdj,
-                                  uint32_t *dPerm);
-// Index of the first edge with an id outside [0, nV), or -1 (waits).
-gas_status device_first_bad_edge(cudaStream_t s, int32_t nV, int32_t nE, const int32_t *dSrcs,
-                                 const int32_t *dDsts, long long *firstBad);
+                                  const int32_t *dOther, bool sorted, int32_t *dOff, int32_t *dAdj,
+                                  uint32_t *dPerm, const SortScratch &x);
+// The first edge with an id outside [0, nV), or -1, and whether the edges
+// come by ascending source / destination (waits; 16 bytes of scratch).
+struct EdgeCheck {
+  long long firstBad = -1;
+  bool srcSorted = true, dstSorted = true;
+};
+gas_status device_check_edges(cudaStream_t s, int32_t nV, int32_t nE, const int32_t *dSrcs,
+                              const int32_t *dDsts, void *scratch, EdgeCheck *out);
+// In-degree classes of the pull passes (dense.cuh): bins[V] = hubs (more
+// than kChunkEdges in-edges) | 65..kChunkEdges | 9..64 | 1..8 | 0, the
+// second and third by falling degree, ties and the others by vertex id; the
+// hubs' chunks; counts (zero before the call) and the largest degrees.
+struct DegreeBins {
+  int32_t nHub, nMid, nSmall, nTiny, nZero, nChunks, maxIn, maxOut;
+};
+struct HubChunks {
+  int32_t *vertex, *begin, *first, *count, *slot;
+};
+gas_status device_degree_bins(cudaStream_t s, int32_t nV, const int32_t *inOff, const int32_t *outOff,
+                              int32_t maxHubs, int32_t *bins, const HubChunks &hubs, DegreeBins *dCounts,
+                              const SortScratch &x);
 // out[q] = CSC position of the edge at CSR position q.
 gas_status device_csr_to_csc(cudaStream_t s, int32_t n, const uint32_t *cscPerm,
                              const uint32_t *csrPerm, int32_t *out);
@@ -51,6 +79,7 @@ struct CoreGraph {
   int32_t edgeBytes;
   const std::vector<int32_t> *hInOff;
   const std::vector<int32_t> *hOutOff;
+  int32_t maxOutDeg;
 };
 bool core_graph(struct gas_core_s *c, CoreGraph *out);
 // Keep the CSR permutation at the next set_graph (false also frees a kept

@@ -902,8 +902,7 @@ gas_status gas_server_add_graph(gas_server *h, int32_t nVertices, int32_t nEdges
   g->weighted = weights != nullptr;
   g->bytes = need;
   {
-    const std::vector<int32_t> &off = *g->bg.g.hOutOff;
-    for (int32_t v = 0; v < nVertices; ++v) g->maxOutDeg = std::max(g->maxOutDeg, off[v + 1] - off[v]);
+    g->maxOutDeg = g->bg.g.maxOutDeg;
     for (int32_t i = 0; weights && i < nEdges; ++i) g->maxWeight = std::max(g->maxWeight, weights[i]);
   }
   std::lock_guard<std::mutex> lk(s.mu);
