@@ -31,6 +31,7 @@
 #include "edge_scatter.cuh"
 #include "fused.cuh"
 #include "gather.cuh"
+#include "pull.cuh"
 #include "scatter.cuh"
 
 namespace gas {
@@ -107,6 +108,31 @@ __device__ __forceinline__ bool fused_barrier(unsigned *bar, unsigned *errWord, 
     if (x) atomicAdd(cnt, x);
     if (y) atomicAdd(cnt + 1, y);
     s_ok = barrier_thread0(bar, errWord) ? 1u : 0u;
+  }
+  __syncthreads();
+  return s_ok != 0u;
+}
+
+// The same for a block of up to 32 warps: one warp adds the warps' sums (a
+// thread that added 32 of them would take about as long as the barrier).
+__device__ __forceinline__ bool counts_barrier(unsigned *bar, unsigned *errWord, const DenseCounts &c,
+                                               unsigned long long *cnt) {
+  __shared__ uint4 sums[32];
+  __shared__ unsigned s_ok;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint4 w = make_uint4(__reduce_add_sync(kFullMask, c.active), __reduce_add_sync(kFullMask, c.inEdges),
+                             __reduce_add_sync(kFullMask, c.ret), __reduce_add_sync(kFullMask, c.outEdges));
+  if (lane == 0) sums[warp] = w;
+  __syncthreads();
+  if (warp == 0) {
+    const uint4 v = lane < (int)(blockDim.x >> 5) ? sums[lane] : make_uint4(0u, 0u, 0u, 0u);
+    const unsigned na = __reduce_add_sync(kFullMask, v.x), ni = __reduce_add_sync(kFullMask, v.y);
+    const unsigned nr = __reduce_add_sync(kFullMask, v.z), no = __reduce_add_sync(kFullMask, v.w);
+    if (lane == 0) {
+      if (na) atomicAdd(cnt, ((unsigned long long)na << 32) | ni);
+      if (nr) atomicAdd(cnt + 1, ((unsigned long long)nr << 32) | no);
+      s_ok = barrier_thread0(bar, errWord) ? 1u : 0u;
+    }
   }
   __syncthreads();
   return s_ok != 0u;
@@ -236,37 +262,91 @@ __device__ __forceinline__ bool dense_to_list(const gas_run_args &ra, const gas_
 // runs as a pull pass over the marked frontier.
 constexpr long long kMarkPullFactor = 4;
 
-// The leading dense rounds of a run that starts with every vertex active,
-// in a kernel that holds nothing else: 40 registers a thread, 6 CTAs per SM
-// (the main kernel's list-round code needs 64 or more).  It stops before
-// the first list round and leaves ra.resume for the main kernel (resume[3]:
-// 0 go on, 1 the run is over, 2 stopped at maxRounds before a dense round);
-// the rounds, stamps, resets and statistics are the main kernel's own.
-template <class P, int MinBlocks>
-__global__ void __launch_bounds__(kGNT, MinBlocks) run_dense_kernel(const gas_run_args ra) {
-  DenseCtx dc = dense_ctx(ra);
-  void *const vdBuf[2] = {ra.g.vertexData, ra.vertexAlt};
+// The leading dense rounds of a run that starts with every vertex active
+// (pull.cuh), one CTA per SM.  It stops before the first
+// list round and leaves ra.resume for the main kernel (resume[3]: 0 go on,
+// 1 the run is over, 2 stopped at maxRounds before a dense round); the
+// rounds, stamps, resets and statistics are the main kernel's own.
+template <class P, bool WIDE>
+__global__ void __launch_bounds__(PullThreads<P>::value, 1) run_dense_kernel(const gas_run_args ra) {
+  typedef typename P::VertexData VD;
+  typedef typename PullSource<P>::type Src;
+  constexpr bool kMessage = PullSource<P>::kMessage;
+  extern __shared__ __align__(16) unsigned char pullSmem[];
+  Src *hot = reinterpret_cast<Src *>(pullSmem);
+  uint32_t *hotPrev = reinterpret_cast<uint32_t *>(pullSmem + kHotBytes);
+  VD *vd = reinterpret_cast<VD *>(ra.g.vertexData);
+  // messages alternate between the two spare vertex buffers, vertex data
+  // between its own and the first of them
+  Src *const buf[2] = {reinterpret_cast<Src *>(kMessage ? ra.g.vertexNew : ra.g.vertexData),
+                       reinterpret_cast<Src *>(ra.vertexAlt)};
+  __shared__ PullRound<P> round;
+  __shared__ PullUnits units;
+  PullCtx<P> a;
+  a.hot = hot;
+  a.hotPrev = hotPrev;
+  a.round = &round;
+  const int hotWords = (ra.nHot + 31) >> 5;
+  const int stride = gridDim.x * blockDim.x, gtid = blockIdx.x * blockDim.x + threadIdx.x;
   const long long E = ra.g.nEdges;
-  int vcur = 0, r = 0, pending = 0, ended = 0;
-  for (;;) {
+  int r = 0, pending = 0, ended = 0;
+  PullFirst first;
+  if constexpr (kMessage) {  // the round-0 messages
+    for (int v = gtid; v < ra.g.nVertices; v += stride) buf[0][v] = P::gatherMap(vd + v, vd + v, nullptr);
+    if (!grid_barrier(ra.barrier, ra.g.errWord)) ended = 1;
+  }
+  for (; !ended;) {
     if (ra.maxRounds > 0 && r >= ra.maxRounds) {
-      ended = 2;  // stopped before a dense round: its frontier is round r-1's stamps
+      ended = 2;  // stopped before a dense round: its frontier is round r-1's bits
       break;
     }
+    const int32_t stamp = ra.stampBase + r;
     if (blockIdx.x == 0 && threadIdx.x == 0) round_resets(ra, r, ra.cur ^ (r & 1), ra.sidx ^ (r & 1));
-    clear_ahead(ra, ra.stampBase + r);
-    dense_round(dc, ra, vdBuf, vcur, r, r == 0);
-    dense_pass<P>(dc);
-    if (!grid_barrier(ra.barrier, ra.g.errWord)) {
+    clear_ahead(ra, stamp);
+    for (int i = gtid; i < hotWords; i += stride) ra.hotBits[(unsigned)(stamp + 1) % 3u][i] = 0u;
+    // the hot sources' values and bits as of the previous round's end
+    if (r == 0) {
+      if (threadIdx.x < (unsigned)hotWords) hotPrev[threadIdx.x] = 0u;
+      // (from buf[0]: message Programs already update vertex data in place
+      // where other blocks have started the round)
+#pragma unroll 8
+      for (int k = threadIdx.x + 1; k < ra.nHot; k += blockDim.x) hot[k] = load_cg(buf[0] + ra.hotVertex[k]);
+    } else if (ra.nHot > 1) {
+      const int4 *from = reinterpret_cast<const int4 *>(ra.hotVal[r & 1]);
+      const int quads = (int)(((size_t)ra.nHot * sizeof(Src) + 15) / 16);
+#pragma unroll 8
+      for (int k = threadIdx.x; k < quads; k += blockDim.x) reinterpret_cast<int4 *>(hot)[k] = __ldcg(from + k);
+      const uint32_t *bits = ra.hotBits[(unsigned)(stamp - 1) % 3u];
+      for (int k = threadIdx.x; k < hotWords; k += blockDim.x) hotPrev[k] = __ldcg(bits + k);
+    }
+    unsigned long long *cnt = ra.denseCnt + kDenseCntStride * (r % 3);
+    if (threadIdx.x == 0) {
+      round.cur = buf[r & 1];
+      round.next = buf[(r & 1) ^ 1];
+      round.hotNext = reinterpret_cast<Src *>(ra.hotVal[(r + 1) & 1]);
+      round.prevBits = round_bits(ra, stamp - 1);
+      round.curBits = round_bits(ra, stamp);
+      round.hotBits = ra.hotBits[(unsigned)stamp % 3u];
+      round.cnt = cnt;
+      round.iteration = ra.g.iteration + r;
+      // vertices without in-edges are active in round 0 alone: rounds 0 and
+      // 1 leave their final value in both buffers
+      units = pull_units<WIDE>(ra, r >= 2 ? ra.nTiny - ra.nZero : ra.nTiny);
+    }
+    __syncthreads();
+    a.cur = round.cur;
+    a.allActive = r == 0;
+    if (WIDE && r == 0) first = pull_first<WIDE>(ra, units, pull_first_unit());
+    const DenseCounts counts = pull_pass<P, WIDE>(a, ra, units, first);
+    if (!counts_barrier(ra.barrier, ra.g.errWord, counts, cnt)) {
       ended = 1;
       break;
     }
-    const unsigned long long statA = dc.cnt[0], statR = dc.cnt[1];
+    const unsigned long long statA = cnt[0], statR = cnt[1];
     if ((statA >> 32) == 0) {  // no vertex was active: the run ended before this round
       ended = 1;
       break;
     }
-    vcur ^= 1;
     if (blockIdx.x == 0 && threadIdx.x == 0 && r < ra.maxStatRounds) {
       ra.stats[2 * (size_t)r] = statA;
       ra.stats[2 * (size_t)r + 1] = statR;
@@ -291,7 +371,7 @@ __global__ void __launch_bounds__(kGNT, MinBlocks) run_dense_kernel(const gas_ru
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     ra.resume[0] = r;
-    ra.resume[1] = vcur;
+    ra.resume[1] = kMessage ? 0 : r & 1;
     ra.resume[2] = pending;
     ra.resume[3] = ended;
   }

@@ -21,6 +21,11 @@
 //     third argument; a Program may declare `static constexpr bool
 //     haveGather = false` to make run() skip the gather (as bfs.cu does by
 //     calling gatherApply(false));
+//   * a Program whose gatherMap depends on the source's VertexData alone may
+//     declare `static constexpr bool gatherFromSource = true`: run() then
+//     evaluates it once per source and round, with null edge data, where
+//     every vertex is active (pull.cuh); one whose gatherReduce gives the
+//     same bits in any order may declare `reduceAnyOrder = true` likewise;
 //   * getResults() returns edge data in the caller's original order (the
 //     reference copies CSC-sorted data back, gpugas.h:333-336);
 //   * a Program declaring `static constexpr bool scatterEdges = true` (and
@@ -78,6 +83,7 @@ class EngineGPU {
     edHost_ = edgeData;
     const int32_t eb = kEdgeBytes;
     if (kScatterEdges && !note(gas_core_enable_edge_scatter(core_, 1))) return;
+    if (!note(gas_core_set_pull_entry(core_, kPullEntry, kPullFlags))) return;
     if (!note(gas_core_set_graph(core_, nVertices, nEdges, edgeListSrcs, edgeListDsts,
                                  eb ? (const void *)edgeData : nullptr, eb,
                                  (int32_t)sizeof(VertexData), (int32_t)sizeof(GatherResult))))
@@ -184,6 +190,12 @@ class EngineGPU {
       std::is_empty<EdgeData>::value ? 0 : (int32_t)sizeof(EdgeData);
   static constexpr bool kScatterEdges =
       detail::ProgramScatterEdges<Program>::value && kEdgeBytes > 0;
+  // Programs with a scatter run list rounds only
+  static constexpr int32_t kPullEntry =
+      kScatterEdges ? 0 : (int32_t)sizeof(typename detail::PullSource<Program>::type);
+  static constexpr int32_t kPullFlags =
+      (detail::PullQuadEd<Program>::value ? GAS_PULL_QUAD_EDGES : 0) |
+      (detail::ProgramReduceAnyOrder<Program>::value ? GAS_PULL_ANY_ORDER : 0);
 
   bool note(gas_status s) {
     status_ = s;
@@ -220,26 +232,29 @@ class EngineGPU {
   // Fused rounds of an apply-only run (BFS: no gather) also use 1 CTA per SM.
   static constexpr int kFusedApplyBlocksPerSM = 1;
   // A run that starts with every vertex active runs its leading dense rounds
-  // in run_dense_kernel (40 registers, 6 CTAs per SM), then resumes here.
-  static constexpr int kDenseBlocksPerSM = 6;
+  // in run_dense_kernel (one CTA and about 132 KB of shared memory per SM), then resumes here.
 
   static gas_status launchRun(void *user, const gas_run_args *ra, void *stream) {
     EngineGPU *self = static_cast<EngineGPU *>(user);
-    if (ra->allActive && ra->resume && !ra->denseFirst && self->runBlocksPerSM_ == 0) {
-      const void *dk = (const void *)detail::run_dense_kernel<Program, kDenseBlocksPerSM>;
-      if (self->denseGrid_ == 0) {
+    if (ra->allActive && ra->resume && ra->pullIds && !ra->denseFirst && self->runBlocksPerSM_ == 0) {
+      const void *dk = ra->pullWide ? (const void *)detail::run_dense_kernel<Program, true>
+                                    : (const void *)detail::run_dense_kernel<Program, false>;
+      const size_t smem = detail::pull_smem_bytes<Program>();
+      if (self->denseGrid_ == 0 || self->denseWide_ != ra->pullWide) {
+        self->denseWide_ = ra->pullWide;
         int dev = 0, sms = 0, per = 0, coop = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, dk, detail::kGNT, 0);
-        if (per > kDenseBlocksPerSM) per = kDenseBlocksPerSM;
-        self->denseGrid_ = (coop && per > 0 && sms > 0) ? per * sms : -1;
+        cudaFuncSetAttribute(dk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, dk, detail::PullThreads<Program>::value, smem);
+        cudaGetLastError();
+        self->denseGrid_ = (coop && per > 0 && sms > 0) ? sms : -1;
       }
       if (self->denseGrid_ > 0) {
         void *dargs[] = {const_cast<gas_run_args *>(ra)};
-        cudaError_t e = cudaLaunchCooperativeKernel(dk, dim3(self->denseGrid_), dim3(detail::kGNT), dargs, 0,
-                                                    (cudaStream_t)stream);
+        cudaError_t e = cudaLaunchCooperativeKernel(dk, dim3(self->denseGrid_), dim3(detail::PullThreads<Program>::value),
+                                                    dargs, smem, (cudaStream_t)stream);
         if (e == cudaSuccess) {
           gas_run_args rest = *ra;
           rest.denseFirst = 1;
@@ -300,6 +315,7 @@ class EngineGPU {
   int runGridFused_ = 0;
   int runGridFusedApply_ = 0;
   int denseGrid_ = 0;
+  int denseWide_ = 0;  // the form denseGrid_ was found for
   int runBlocksPerSM_ = 0;
   VertexData *vdHost_ = nullptr;
   EdgeData *edHost_ = nullptr;

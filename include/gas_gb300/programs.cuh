@@ -10,6 +10,8 @@
 //   * BFS takes the iteration number as a third apply() argument instead of
 //     reading the driver's __constant__ g_iterationCountGPU (bfs.cu:28,63);
 //     the engine passes the round number (or gas_engine_set_iteration's);
+//   * CC, PageRank and PPR declare gatherFromSource, SSSP and CC
+//     reduceAnyOrder (pull.cuh);
 //   * BFS declares haveGather = false, which is how the reference driver
 //     runs it (gatherApply(false), bfs.cu:104).
 #pragma once
@@ -50,6 +52,7 @@ struct SSSP {
   typedef int GatherResult;
   static constexpr int maxLength = 100000;
   static constexpr int gatherZero = INT_MAX - maxLength;
+  static constexpr bool reduceAnyOrder = true;
 
   __host__ __device__ static int gatherReduce(const int &left, const int &right) {
     return left < right ? left : right;
@@ -71,6 +74,8 @@ struct CC {
   struct EdgeData {};
   typedef int GatherResult;
   static constexpr int gatherZero = INT_MAX;
+  static constexpr bool gatherFromSource = true;
+  static constexpr bool reduceAnyOrder = true;
 
   __host__ __device__ static int gatherReduce(const int &left, const int &right) {
     return left < right ? left : right;
@@ -97,6 +102,7 @@ struct PageRank {
   struct EdgeData {};
   typedef float GatherResult;
   static constexpr float gatherZero = 0.0f;
+  static constexpr bool gatherFromSource = true;
 
   __host__ __device__ static float gatherMap(const VertexData *, const VertexData *src,
                                              const EdgeData *) {
@@ -126,6 +132,7 @@ struct PPR {
   struct EdgeData {};
   typedef float GatherResult;
   static constexpr float gatherZero = 0.0f;
+  static constexpr bool gatherFromSource = true;
 
   __host__ __device__ static float gatherMap(const VertexData *, const VertexData *src,
                                              const EdgeData *) {

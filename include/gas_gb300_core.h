@@ -45,6 +45,10 @@ extern "C" {
  * word, rounded up to 16 (one aligned vector load reads a whole cell). */
 #define GAS_FUSED_CELL_BYTES(vertexBytes) ((((vertexBytes) * 2 + 4) + 15) / 16 * 16)
 
+/* Shared memory of the leading dense rounds' kernel for the values of the
+ * graph's hot sources, the vertices of highest out-degree (pull.cuh). */
+#define GAS_PULL_HOT_BYTES (128 * 1024)
+
 /* A vertex list on the device: ids, exclusive prefix of the degree that the
  * consumer walks (in-degree for the gather, out-degree for the scatter),
  * CSC/CSR begin offset of each vertex, merge-path tile splits, and a
@@ -183,6 +187,29 @@ typedef struct {
    * next frontier is then the vertices whose bits its last round set
    * (retBits) instead of a list */
   int32_t *denseEndOut;
+  /* layout of the leading dense rounds' kernel (pull.cuh; null pullIds: none,
+   * see gas_core_set_pull_entry): the work units (slices of 32-lane steps)
+   * as {first int4, quads of the longest vertex or steps} and one past the last, their
+   * source ids -- a hot vertex as 0x80000000 | table slot -- and 4-byte edge
+   * data (null: other sizes), four a lane and step; per vertex of the degree
+   * bins, in their order (hubs first), and per chunk, one record {vertex, CSC
+   * begin, edges, out-degree}; the slot of each vertex (-1: not hot); the hot
+   * vertices, those of out-degree >= hotMinOut, by slot (slot 0 is nobody's);
+   * compact copies of their source values (by round parity) and frontier bits
+   * (by stamp % 3) */
+  const void *pullIds;        /* int4 */
+  const void *pullEds;        /* int4 */
+  const void *pullSlices;     /* int2 */
+  int32_t pullWide;           /* more lanes a vertex (pull_mid_lanes) */
+  const void *pullRec;        /* [nVertices] int4 */
+  const void *chunkRec;       /* [nChunks] int4 */
+  const int32_t *slotOf;      /* [nVertices] */
+  const int32_t *hotVertex;   /* [nHot] */
+  int32_t nHot;               /* slots, the unused one included */
+  int32_t hotMinOut;
+  void *hotVal[2];            /* GAS_PULL_HOT_BYTES each */
+  uint32_t *hotBits[3];       /* [ceil(nHot / 32)], clear at launch */
+  int32_t nZero;              /* vertices without in-edges, the last of binTiny */
 } gas_run_args;
 
 /* The vertices whose apply returned true in the round just scattered, for
@@ -221,6 +248,15 @@ GAS_API gas_status gas_core_set_graph(gas_core *c, int32_t nVertices, int32_t nE
                                       const int32_t *srcs, const int32_t *dsts,
                                       const void *edgeData, int32_t edgeBytes,
                                       int32_t vertexBytes, int32_t gatherBytes);
+
+/* Bytes of a source value in the leading dense rounds (the message of a
+ * Program that declares gatherFromSource, else its VertexData), before
+ * gas_core_set_graph: the graph then keeps the layout of that kernel
+ * (gas_run_args::pullIds, about 5 bytes an edge, 10 with 4-byte edge
+ * data, and 20 a vertex).  0 (the default): none. */
+#define GAS_PULL_QUAD_EDGES 1 /* flags: gatherMap reads 4-byte edge data */
+#define GAS_PULL_ANY_ORDER 2  /* flags: reductions in any order (reduceAnyOrder) */
+GAS_API gas_status gas_core_set_pull_entry(gas_core *c, int32_t bytes, int32_t flags);
 
 GAS_API gas_status gas_core_upload_vertex_data(gas_core *c, const void *host);
 GAS_API gas_status gas_core_download_vertex_data(gas_core *c, void *host);

@@ -127,6 +127,7 @@ SIGNATURES = {
     "gas_core_destroy": (_I32, [_P]),
     "gas_core_stream": (_I32, [_P, C.POINTER(_P)]),
     "gas_core_set_graph": (_I32, [_P, _I32, _I32, _PI32, _PI32, _P, _I32, _I32, _I32]),
+    "gas_core_set_pull_entry": (_I32, [_P, _I32, _I32]),
     "gas_core_upload_vertex_data": (_I32, [_P, _P]),
     "gas_core_download_vertex_data": (_I32, [_P, _P]),
     "gas_core_download_edge_data": (_I32, [_P, _P]),

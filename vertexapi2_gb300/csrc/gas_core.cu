@@ -25,7 +25,7 @@
 #include <vector>
 
 #include "gas_gb300_core.h"
-#include "gas_gb300/detail/dense.cuh"
+#include "gas_gb300/detail/pull.cuh"
 #include "gas_gb300/detail/scatter.cuh"
 #include "gas_internal.h"
 
@@ -104,6 +104,9 @@ struct Ctl {
 enum DirtyBit : unsigned {
   kF0 = 1u, kF1 = 2u, kS0 = 4u, kS1 = 8u, kT0 = 16u, kT1 = 32u,
 };
+
+// Words of the hot vertices' bitmap (at least 4 bytes a value).
+constexpr int kHotWords = GAS_PULL_HOT_BYTES / 4 / 32;
 
 constexpr int kRing = 8;
 constexpr int kLag = 3;
@@ -193,6 +196,21 @@ struct gas_core_s {
   int32_t nChunks = 0, nChunkVertices = 0;
   unsigned *chunkArrive = nullptr, *chunkFlags = nullptr;
   void *chunkVal = nullptr;
+  // layout of the leading dense rounds' kernel (pull.cuh), kept when the
+  // Program's source values have pullEntry > 0 bytes
+  int32_t pullEntry = 0;
+  bool pullQuadEd = false;      // its gathers read 4-byte edge data
+  bool pullAnyOrder = false;    // its reductions may take any order
+  bool pullWide = false;        // this graph's layout has more lanes a vertex
+  unsigned char *pullMem = nullptr;  // slices | ids | edge data, reused as the arena is
+  size_t pullBytes = 0;
+  int2 *pullSlices = nullptr;
+  int4 *pullIds = nullptr, *pullEds = nullptr;
+  int32_t *slotOf = nullptr, *hotVertex = nullptr;
+  int4 *pullRec = nullptr, *chunkRec = nullptr;
+  void *hotVal[2] = {nullptr, nullptr};
+  uint32_t *hotBits = nullptr;  // three bitmaps of kHotWords words
+  int32_t nHot = 0, hotMinOut = 0, nZero = 0;
   int32_t denseAlpha = 10;  // dense (pull) round when out-edges * alpha > E
   int32_t *fvid[2] = {nullptr, nullptr}, *fpre[2] = {nullptr, nullptr};
   int32_t *fbeg[2] = {nullptr, nullptr};
@@ -256,6 +274,11 @@ void free_graph(gas_core *c, bool all = true) {
     c->arena = nullptr;
     c->arenaBytes = 0;
   }
+  if (all && c->pullMem) {
+    cudaFree(c->pullMem);
+    c->pullMem = nullptr;
+    c->pullBytes = 0;
+  }
   c->cscPerm = c->csrPerm = nullptr;
   c->csr2csc = nullptr;
   c->fcell = nullptr;
@@ -270,6 +293,12 @@ void free_graph(gas_core *c, bool all = true) {
   c->chunkVertex = c->chunkBegin = c->chunkFirst = c->chunkCount = c->chunkSlot = nullptr;
   c->chunkArrive = c->chunkFlags = nullptr;
   c->chunkVal = nullptr;
+  c->pullSlices = nullptr;
+  c->pullIds = c->pullEds = c->pullRec = c->chunkRec = nullptr;
+  c->slotOf = c->hotVertex = nullptr;
+  c->hotVal[0] = c->hotVal[1] = nullptr;
+  c->hotBits = nullptr;
+  c->nHot = c->hotMinOut = c->nZero = 0;
   c->nMid = c->nSmall = c->nTiny = c->nChunks = c->nChunkVertices = 0;
   for (int k = 0; k < 2; ++k) {
     c->fvid[k] = c->fpre[k] = c->fbeg[k] = c->fsplit[k] = nullptr;
@@ -311,6 +340,15 @@ size_t carve_arena(gas_core *c, unsigned char *base, bool edgeMap, int32_t maxHu
   bytes(&c->valt, (size_t)c->vertexBytes * V);
   take(&c->retBits, 4 * 3 * (size_t)c->bitWords);
   take(&c->bins, 4 * V);
+  if (c->pullEntry > 0) {
+    take(&c->slotOf, 4 * V);
+    take(&c->hotVertex, GAS_PULL_HOT_BYTES);
+    take(&c->pullRec, 16 * V);
+    take(&c->chunkRec, 16 * (size_t)maxChunks);
+    bytes(&c->hotVal[0], GAS_PULL_HOT_BYTES);
+    bytes(&c->hotVal[1], GAS_PULL_HOT_BYTES);
+    take(&c->hotBits, 4 * 3 * (size_t)kHotWords);
+  }
   take(&c->chunkVertex, 4 * (size_t)maxChunks);
   take(&c->chunkBegin, 4 * (size_t)maxChunks);
   take(&c->chunkFirst, 4 * (size_t)maxChunks);
@@ -664,6 +702,12 @@ gas_status gas_core_set_graph(gas_core *c, int32_t nV, int32_t nE, const int32_t
   const HubChunks hubs = {c->chunkVertex, c->chunkBegin, c->chunkFirst, c->chunkCount, c->chunkSlot};
   if (st == GAS_OK && e == cudaSuccess)
     st = device_degree_bins(c->stream, nV, c->inOff, c->outOff, maxHubs, c->bins, hubs, dCounts, sx);
+  HotInfo *dHot = reinterpret_cast<HotInfo *>(dCounts + 1);
+  A(cudaMemsetAsync(dHot, 0, sizeof(HotInfo), c->stream));
+  PullLayout pl = {c->slotOf, c->hotVertex, c->pullRec, c->chunkRec, c->pullAnyOrder, false};
+  if (st == GAS_OK && e == cudaSuccess && c->pullEntry > 0)
+    st = device_pull_records(c->stream, nV, c->inOff, c->outOff, c->bins, hubs, dCounts, maxChunks,
+                             gas::detail::pull_hot_capacity(c->pullEntry), pl, dHot, sx);
   if (st) return give_up(st);
   A(cudaMemsetAsync(c->mark, 0, sizeof(int32_t) * std::max(nV, 1), c->stream));
   A(cudaMemsetAsync(c->retBits, 0, sizeof(uint32_t) * 3 * std::max(c->bitWords, 1), c->stream));
@@ -674,6 +718,8 @@ gas_status gas_core_set_graph(gas_core *c, int32_t nV, int32_t nE, const int32_t
   c->hInOff.resize((size_t)nV + 1);
   c->hOutOff.resize((size_t)nV + 1);
   DegreeBins bins;
+  HotInfo hot;
+  A(cudaMemcpyAsync(&hot, dHot, sizeof(hot), cudaMemcpyDeviceToHost, c->stream));
   A(cudaMemcpyAsync(c->hInOff.data(), c->inOff, sizeof(int32_t) * ((size_t)nV + 1),
                     cudaMemcpyDeviceToHost, c->stream));
   A(cudaMemcpyAsync(c->hOutOff.data(), c->outOff, sizeof(int32_t) * ((size_t)nV + 1),
@@ -690,11 +736,46 @@ gas_status gas_core_set_graph(gas_core *c, int32_t nV, int32_t nE, const int32_t
   c->nMid = bins.nMid;
   c->nSmall = bins.nSmall;
   c->nTiny = bins.nTiny + bins.nZero;
+  c->nZero = bins.nZero;
+  c->nHot = hot.nHot;
+  c->hotMinOut = hot.nHot > 1 ? hot.minOut : 0x7fffffff;
   c->binMid = c->bins + bins.nHub;
   c->binSmall = c->binMid + bins.nMid;
   c->binTiny = c->binSmall + bins.nSmall;
   c->nChunks = bins.nChunks;
   c->nChunkVertices = bins.nHub;
+  if (c->pullEntry > 0) {
+    // the slices of the leading dense rounds' kernel; their extents are
+    // wanted before the rest of the memory can be sized
+    c->pullWide = pl.wide = bins.nChunks + bins.nMid / (32 / gas::detail::pull_mid_lanes(false)) + bins.nSmall / 32 <
+                            gas::detail::kPullNarrowUnits;
+    const size_t listed = ((size_t)pull_slice_count(bins, pl.wide) + 1) * sizeof(int2);
+    const size_t sliceBytes = (listed + 255) & ~(size_t)255;
+    int2 *dSlices = reinterpret_cast<int2 *>(sx.keys[0]);
+    long long quads = 0;
+    st = device_pull_slices(c->stream, bins, pl, dSlices, &quads, sx);
+    if (st) return give_up(st);
+    const bool eds = c->pullQuadEd && edgeBytes == 4;
+    const size_t idBytes = ((size_t)quads * 16 + 256) & ~(size_t)255;
+    const size_t want = sliceBytes + idBytes * (eds ? 2 : 1);
+    if (c->pullBytes < want || c->pullBytes / 4 > want) {
+      if (c->pullMem) cudaFree(c->pullMem);
+      c->pullMem = nullptr;
+      c->pullBytes = 0;
+      A(cudaMalloc((void **)&c->pullMem, want));
+      if (e != cudaSuccess) return give_up(cuda_fail(e, "setGraph device allocation"));
+      c->pullBytes = want;
+    }
+    c->pullSlices = reinterpret_cast<int2 *>(c->pullMem);
+    c->pullIds = reinterpret_cast<int4 *>(c->pullMem + sliceBytes);
+    c->pullEds = eds ? reinterpret_cast<int4 *>(c->pullMem + sliceBytes + idBytes) : nullptr;
+    if (nV > 0) A(cudaMemcpyAsync(c->pullSlices, dSlices, listed, cudaMemcpyDeviceToDevice, c->stream));
+    st = device_pull_fill(c->stream, bins, pl, c->pullSlices, c->inSrc, static_cast<const int32_t *>(c->ed),
+                          c->pullIds, c->pullEds);
+    if (st) return give_up(st);
+    A(cudaStreamSynchronize(c->stream));
+    if (e != cudaSuccess) return give_up(cuda_fail(e, "setGraph build"));
+  }
   if (c->maxInDeg <= GAS_TPV_MAX_DEGREE && c->maxOutDeg <= GAS_TPV_MAX_DEGREE) {  // fused rounds
     A(cudaMalloc(&c->fcell, (size_t)GAS_FUSED_CELL_BYTES(vertexBytes) * std::max(nV, 1)));
     // fixed-width adjacency rows: a vertex's neighbours in one or two 16-byte
@@ -731,6 +812,16 @@ gas_status gas_core_set_graph(gas_core *c, int32_t nV, int32_t nE, const int32_t
   c->cur = c->sidx = 0;
   c->pendingCommit = false;
   c->haveScatList = false;
+  return GAS_OK;
+}
+
+gas_status gas_core_set_pull_entry(gas_core *c, int32_t bytes, int32_t flags) {
+  if (!c) return fail(GAS_ERR_INVALID, "gas_core_set_pull_entry: engine is NULL");
+  if (bytes < 0) return fail(GAS_ERR_INVALID, "negative source value size");
+  // too large for a table worth its upkeep: no layout
+  c->pullEntry = bytes > 0 && gas::detail::pull_hot_capacity(bytes) > 0 ? std::max(bytes, 4) : 0;
+  c->pullQuadEd = (flags & GAS_PULL_QUAD_EDGES) != 0;
+  c->pullAnyOrder = (flags & GAS_PULL_ANY_ORDER) != 0;
   return GAS_OK;
 }
 
@@ -1143,12 +1234,26 @@ gas_status gas_core_run_persistent(gas_core *c, int32_t maxIters, int32_t haveGa
     if (c->frontBits)
       seg(c->frontBits + (size_t)((unsigned)(ra.stampBase + 1) % 3u) * c->bitWords,
           sizeof(uint32_t) * std::max(c->bitWords, 1));
+    if (c->hotBits) seg(c->hotBits, sizeof(uint32_t) * 3 * kHotWords);
     const int32_t most = std::max(c->bitWords, std::max(c->nChunkVertices, 64));
     const int blocks = std::min(c->numSMs > 0 ? c->numSMs : 1, (most + 255) / 256);
     zero_segments_kernel<<<blocks, 256, 0, c->stream>>>(z);
     A(cudaGetLastError());
     if (e != cudaSuccess) return cuda_fail(e, "run setup");
   }
+  ra.pullIds = c->pullIds;
+  ra.pullEds = c->pullEds;
+  ra.pullSlices = c->pullSlices;
+  ra.pullWide = c->pullWide ? 1 : 0;
+  ra.pullRec = c->pullRec;
+  ra.chunkRec = c->chunkRec;
+  ra.slotOf = c->slotOf;
+  ra.hotVertex = c->hotVertex;
+  ra.nHot = c->nHot;
+  ra.hotMinOut = c->hotMinOut;
+  ra.nZero = c->nZero;
+  for (int k = 0; k < 2; ++k) ra.hotVal[k] = c->hotVal[k];
+  for (int k = 0; k < 3; ++k) ra.hotBits[k] = c->hotBits ? c->hotBits + k * kHotWords : nullptr;
   ra.binMid = c->binMid;
   ra.binSmall = c->binSmall;
   ra.binTiny = c->binTiny;

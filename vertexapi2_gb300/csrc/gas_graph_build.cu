@@ -35,7 +35,7 @@
 #include <algorithm>
 #include <vector>
 
-#include "gas_gb300/detail/dense.cuh"
+#include "gas_gb300/detail/pull.cuh"
 #include "gas_internal.h"
 
 using gas::internal::cuda_fail;
@@ -391,6 +391,176 @@ __global__ void hub_chunks_kernel(const int32_t *bins, const int32_t *inOff,
   }
 }
 
+// Sort key of the out-degrees, the largest first.
+__global__ void out_degree_key_kernel(const int32_t *outOff, int32_t nV, uint32_t *key) {
+  for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < nV;
+       v += (long long)gridDim.x * blockDim.x)
+    key[v] = 65535u - (uint32_t)min(outOff[v + 1] - outOff[v], 65535);
+}
+
+// order: the vertices by falling out-degree.  The hot ones: as many whole
+// degree classes as fit `capacity` slots, of which the first stays unused
+// (one block).
+__global__ void hot_pick_kernel(const uint32_t *order, const int32_t *outOff, int32_t nV, int32_t capacity,
+                                gas::internal::HotInfo *info, int32_t *hotVertex) {
+  __shared__ int sHot;
+  const int most = capacity - 1;
+  auto deg = [&](int k) { return outOff[order[k] + 1] - outOff[order[k]]; };
+  if (threadIdx.x == 0) {
+    const int minOut = nV > most ? max(1, deg(most) + 1) : 1;
+    int lo = 0, hi = min(nV, most);  // the first k of a smaller degree
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (deg(mid) >= minOut)
+        lo = mid + 1;
+      else
+        hi = mid;
+    }
+    sHot = lo;
+    info->nHot = lo + 1;
+    info->minOut = minOut;
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < sHot; k += blockDim.x) hotVertex[k + 1] = (int32_t)order[k];
+}
+
+__global__ void hot_slots_kernel(const gas::internal::HotInfo *info, const int32_t *hotVertex, int32_t *slotOf) {
+  const int n = info->nHot;
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x + 1; k < n; k += gridDim.x * blockDim.x)
+    slotOf[hotVertex[k]] = k;
+}
+
+__global__ void pull_records_kernel(const int32_t *bins, const int32_t *inOff, const int32_t *outOff, int32_t nV,
+                                    int4 *rec) {
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nV;
+       i += (long long)gridDim.x * blockDim.x) {
+    const int v = bins[i], b = inOff[v];
+    rec[i] = make_int4(v, b, inOff[v + 1] - b, outOff[v + 1] - outOff[v]);
+  }
+}
+
+__global__ void chunk_records_kernel(const gas::internal::DegreeBins *c, gas::internal::HubChunks hubs,
+                                     const int32_t *inOff, const int32_t *outOff, int4 *rec) {
+  const int n = c->nChunks;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const int v = hubs.vertex[i], b = hubs.begin[i];
+    rec[i] = make_int4(v, b, min(gas::detail::kChunkEdges, inOff[v + 1] - b), outOff[v + 1] - outOff[v]);
+  }
+}
+
+// A slice's class and first record (pull.cuh: chunks, mid, small, tiny).
+struct SliceAt {
+  const int4 *rec;
+  int count;  // vertices
+  int lanes;  // of each
+  int virt;   // of dense.cuh's lanes in each (0: quads dealt round-robin)
+};
+__device__ __forceinline__ SliceAt slice_at(const gas::internal::DegreeBins &n, const gas::internal::PullLayout &l,
+                                            int u) {
+  const int ml = gas::detail::pull_mid_lanes(l.wide), sl = gas::detail::pull_small_lanes(l.wide);
+  const int M = 32 / ml, S = 32 / sl;
+  if (u < n.nChunks) return {l.chunkRec + u, 1, 32, l.anyOrder ? 0 : 1};
+  u -= n.nChunks;
+  const int4 *rec = l.rec + n.nHub;
+  const int mid = (n.nMid + M - 1) / M, small = (n.nSmall + S - 1) / S;
+  if (u < mid) return {rec + u * M, min(M, n.nMid - u * M), ml, l.anyOrder ? 0 : 32 / ml};
+  u -= mid;
+  rec += n.nMid;
+  if (u < small) return {rec + u * S, min(S, n.nSmall - u * S), sl, l.anyOrder ? 0 : gas::detail::kSmallLanes / sl};
+  u -= small;
+  rec += n.nSmall;
+  return {rec + u * 32, min(32, n.nTiny + n.nZero - u * 32), 1, 0};
+}
+
+__device__ __forceinline__ int slice_layers(const SliceAt &s, int quads, int k) {
+  return s.lanes * s.virt == 8 ? gas::detail::pull_layers<8>(quads, k) : gas::detail::pull_layers<32>(quads, k);
+}
+
+// Per slice its longest vertex's quads, or its steps where quads are dealt
+// round-robin, and the int4 it takes: 32 a step.
+__global__ void slice_steps_kernel(const gas::internal::DegreeBins n, const gas::internal::PullLayout l, int nSlices,
+                                   uint32_t *size, int2 *slices) {
+  const int u = blockIdx.x * blockDim.x + threadIdx.x;
+  if (u > nSlices) return;
+  if (u == nSlices) {
+    size[u] = 0u;
+    slices[u] = make_int2(0, 0);
+    return;
+  }
+  const SliceAt s = slice_at(n, l, u);
+  int quads = 0;
+  for (int k = 0; k < s.count; ++k)
+    quads = max(quads, s.virt == 0 ? ((s.rec[k].z + 3) / 4 + s.lanes - 1) / s.lanes
+                                   : gas::detail::pull_range(s.rec[k].y, s.rec[k].z).quads);
+  int steps = s.virt == 0 ? quads : s.virt == 8 ? 2 : 1;
+  for (int k = 0; k < s.virt; ++k) steps += slice_layers(s, quads, k);
+  size[u] = 32u * (uint32_t)steps;
+  slices[u].y = quads;
+}
+
+__global__ void slice_extents_kernel(const uint32_t *base, int nSlices, int2 *slices) {
+  const int u = blockIdx.x * blockDim.x + threadIdx.x;
+  if (u <= nSlices) slices[u].x = (int)base[u];
+}
+
+// A warp per slice writes its steps in the order pull.cuh walks them.
+__global__ void slice_fill_kernel(const gas::internal::DegreeBins n, const gas::internal::PullLayout l,
+                                  const int2 *slices, int nSlices, const int32_t *inSrc, const int32_t *ed, int4 *ids,
+                                  int4 *eds) {
+  const int lane = threadIdx.x & 31;
+  for (int u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < nSlices; u += (gridDim.x * blockDim.x) >> 5) {
+    const SliceAt s = slice_at(n, l, u);
+    const int2 at = slices[u];
+    const int g = lane / s.lanes, sl = lane % s.lanes;
+    const int4 rec = g < s.count ? s.rec[g] : make_int4(-1, 0, 0, 0);
+    size_t pos = (size_t)at.x + lane;
+    // one step: edges [e, e + count) of the CSC, count <= 4
+    auto put = [&](int e, int count) {
+      int id[4], w[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        id[j] = gas::detail::kNoEdge;
+        w[j] = 0;
+        if (j < count) {
+          const int32_t src = inSrc[e + j], slot = l.slotOf[src];
+          id[j] = slot >= 0 ? (int32_t)(0x80000000u | (uint32_t)slot) : src;
+          if (eds) w[j] = ed[e + j];
+        }
+      }
+      ids[pos] = make_int4(id[0], id[1], id[2], id[3]);
+      if (eds) eds[pos] = make_int4(w[0], w[1], w[2], w[3]);
+      pos += 32;
+    };
+    if (s.virt == 0) {
+      for (int t = 0; t < at.y; ++t) {
+        const int e = 4 * (t * s.lanes + sl);
+        put(rec.y + e, min(4, rec.z - e));
+      }
+      continue;
+    }
+    const gas::detail::PullRange r = gas::detail::pull_range(rec.y, rec.z);
+    const int tail = (rec.y + rec.z) & ~3;
+    if (s.virt == 8) {
+      put(rec.y, r.head);
+      put(tail, r.tail);
+    } else if (s.virt == 1) {
+      if (sl < 4)
+        put(rec.y + sl, sl < r.head ? 1 : 0);
+      else
+        put(tail + sl - 4, sl - 4 < r.tail ? 1 : 0);
+    } else {
+      put(sl == 0 ? rec.y : tail, sl == 0 ? r.head : sl == 1 ? r.tail : 0);
+    }
+    for (int k = 0; k < s.virt; ++k) {
+      const int layers = slice_layers(s, at.y, k);
+      for (int j = 0; j < layers; ++j) {
+        const int q = sl * s.virt + k + s.lanes * s.virt * j;
+        put(4 * (r.first + q), q < r.quads ? 4 : 0);
+      }
+    }
+  }
+}
+
 __global__ void invert_kernel(const uint32_t *perm, long long n, uint32_t *inv) {
   for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < n;
        p += (long long)gridDim.x * blockDim.x)
@@ -549,6 +719,60 @@ gas_status device_degree_bins(cudaStream_t s, int32_t nV, const int32_t *inOff, 
     if (e != cudaSuccess) return cuda_fail(e, "degree bins");
   }
   return GAS_OK;
+}
+
+gas_status device_pull_records(cudaStream_t s, int32_t nV, const int32_t *inOff, const int32_t *outOff,
+                               const int32_t *bins, const HubChunks &hubs, const DegreeBins *dCounts,
+                               int32_t maxChunks, int32_t capacity, const PullLayout &out, HotInfo *info,
+                               const SortScratch &x) {
+  if (nV <= 0) return GAS_OK;
+  out_degree_key_kernel<<<grid_for(nV), 256, 0, s>>>(outOff, nV, x.keys[1]);
+  // the order is needed only until the hot vertices are listed: it stands
+  // where their slots go
+  uint32_t *order = reinterpret_cast<uint32_t *>(out.slotOf);
+  gas_status st = radix_sort(s, nV, x.keys[1], nullptr, 16, order, nullptr, x);
+  if (st) return st;
+  hot_pick_kernel<<<1, 1024, 0, s>>>(order, outOff, nV, capacity, info, out.hotVertex);
+  cudaError_t e = cudaMemsetAsync(out.slotOf, 0xff, 4 * (size_t)nV, s);
+  if (e != cudaSuccess) return cuda_fail(e, "pull layout");
+  hot_slots_kernel<<<grid_for(capacity), 256, 0, s>>>(info, out.hotVertex, out.slotOf);
+  pull_records_kernel<<<grid_for(nV), 256, 0, s>>>(bins, inOff, outOff, nV, out.rec);
+  if (maxChunks > 0)
+    chunk_records_kernel<<<grid_for(maxChunks), 256, 0, s>>>(dCounts, hubs, inOff, outOff, out.chunkRec);
+  e = cudaGetLastError();
+  return e == cudaSuccess ? GAS_OK : cuda_fail(e, "pull layout");
+}
+
+int32_t pull_slice_count(const DegreeBins &n, bool wide) {
+  const int M = 32 / gas::detail::pull_mid_lanes(wide), S = 32 / gas::detail::pull_small_lanes(wide);
+  return n.nChunks + (n.nMid + M - 1) / M + (n.nSmall + S - 1) / S + (n.nTiny + n.nZero + 31) / 32;
+}
+
+gas_status device_pull_slices(cudaStream_t s, const DegreeBins &n, const PullLayout &l, int2 *slices,
+                              long long *quads, const SortScratch &x) {
+  const int32_t k = pull_slice_count(n, l.wide);
+  *quads = 0;
+  if (k == 0) return GAS_OK;
+  uint32_t *base = x.spare;
+  slice_steps_kernel<<<(k + 256) / 256, 256, 0, s>>>(n, l, k, base, slices);
+  gas_status st = exclusive_scan(base, (long long)k + 1, x.sums, s);
+  if (st) return st;
+  slice_extents_kernel<<<(k + 256) / 256, 256, 0, s>>>(base, k, slices);
+  uint32_t total = 0;
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&total, base + k, 4, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  *quads = total;
+  return e == cudaSuccess ? GAS_OK : cuda_fail(e, "pull layout");
+}
+
+gas_status device_pull_fill(cudaStream_t s, const DegreeBins &n, const PullLayout &l, const int2 *slices,
+                            const int32_t *inSrc, const int32_t *ed, int4 *ids, int4 *eds) {
+  const int32_t k = pull_slice_count(n, l.wide);
+  if (k == 0) return GAS_OK;
+  slice_fill_kernel<<<grid_for(32ll * k), 256, 0, s>>>(n, l, slices, k, inSrc, ed, ids, eds);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? GAS_OK : cuda_fail(e, "pull layout");
 }
 
 gas_status device_csr_to_csc(cudaStream_t s, int32_t n, const uint32_t *cscPerm,

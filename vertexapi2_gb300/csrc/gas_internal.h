@@ -59,6 +59,31 @@ struct HubChunks {
 gas_status device_degree_bins(cudaStream_t s, int32_t nV, const int32_t *inOff, const int32_t *outOff,
                               int32_t maxHubs, int32_t *bins, const HubChunks &hubs, DegreeBins *dCounts,
                               const SortScratch &x);
+// The layout of the leading dense rounds' kernel (gas_run_args::pullIds and
+// the fields after it).  First, from the CSC, the out-degrees and the bins:
+// the vertices' and chunks' records and the hot vertices, `capacity` at most;
+// *info (device) receives their number and their smallest out-degree.
+struct HotInfo {
+  int32_t nHot, minOut;
+};
+struct PullLayout {
+  int32_t *slotOf, *hotVertex;
+  int4 *rec, *chunkRec;
+  bool anyOrder;  // steps as pull_any walks them, else as pull_ordered does
+  bool wide;      // more lanes a vertex (pull_mid_lanes)
+};
+gas_status device_pull_records(cudaStream_t s, int32_t nV, const int32_t *inOff, const int32_t *outOff,
+                               const int32_t *bins, const HubChunks &hubs, const DegreeBins *dCounts,
+                               int32_t maxChunks, int32_t capacity, const PullLayout &out, HotInfo *info,
+                               const SortScratch &x);
+// Then, with the counts on the host: the number n of slices, their first int4
+// and quads (slices[n + 1]) and *quads, the int4 they take together (waits);
+// and their ids and 4-byte edge data (eds null: none).
+int32_t pull_slice_count(const DegreeBins &n, bool wide);
+gas_status device_pull_slices(cudaStream_t s, const DegreeBins &n, const PullLayout &l, int2 *slices,
+                              long long *quads, const SortScratch &x);
+gas_status device_pull_fill(cudaStream_t s, const DegreeBins &n, const PullLayout &l, const int2 *slices,
+                            const int32_t *inSrc, const int32_t *ed, int4 *ids, int4 *eds);
 // out[q] = CSC position of the edge at CSR position q.
 gas_status device_csr_to_csc(cudaStream_t s, int32_t n, const uint32_t *cscPerm,
                              const uint32_t *csrPerm, int32_t *out);
