@@ -141,45 +141,73 @@ constexpr int kPprChunk = 4096;
 
 struct PprArgs {
   int32_t nVertices;
-  int32_t nQueries;           // queries in the batch (<= the row width QP)
+  int32_t nQueries;           // queries in the batch (<= row)
+  int32_t row;                // floats of a vertex row (ppr_row_width)
   const int32_t *inSources;   // CSC
   const int32_t *outDegree;   // [V]
-  const uint8_t *lastActive;  // [V] last round in which the vertex is active
-  int32_t nUnits;             // work units, longest first
-  const int32_t *unitV;
-  const int32_t *unitBeg;
-  const int32_t *unitLen;
-  const int32_t *unitSlot;    // -1, or the unit's partial-sum slot (hubs)
+  int32_t nUnits;             // work units: hub chunks, then longest first
+  int32_t nLong;              // of them hub chunks or longer than kPprLong
+  const int4 *unit;           // {vertex, CSC begin, edges | last active round << 16,
+                              //  partial-sum slot of a hub chunk or -1}
   const int32_t *slotFirst;   // [slots] first slot of the slot's vertex
   const int32_t *slotCount;   // [slots] chunks of that vertex
   const int32_t *slotHub;     // [slots] hub index (arrival counter)
-  float *partial;             // [slots][QP] (per batch)
-  unsigned *arrive;           // [hubs] arrivals, never reset within a batch
-  const int32_t *sources;     // [nQueries]
-  float *rank[2];             // [V][QP]
-  float *contrib[2];          // [V][QP] rank / outdeg (0 where outdeg is 0)
+  float *partial;             // [slots][row] (per batch)
+  unsigned *arrive;           // [hubs][ppr_slices(row)] arrivals, never reset within a batch
+  const int32_t *sources;     // [nQueries], readable to a multiple of 4
+  float *rank[2];             // [V][row]
+  float *contrib[2];          // [V][row] rank / outdeg (0 where outdeg is 0)
   float damp;                 // 1 - alpha, as the program computes it in float
   float teleport;             // alpha
 };
 
-// The graph part of PprArgs, from a graph's PPR arrays (the work-unit block
-// `mem` holds unitV | unitBeg | unitLen | unitSlot | slotFirst | slotCount |
-// slotHub, `units` and `slots` entries long).
+// Row width of a batch of n queries: a power of two up to 32 (a lane per
+// query), then whole 32-byte sectors (100 queries: 104 floats and not 128).
+inline int ppr_row_width(int n) {
+  if (n > 32) return (n + 7) / 8 * 8;
+  int w = 1;
+  while (w < n) w *= 2;
+  return w;
+}
+// The kernels' template argument for a row: its power of two.
+inline int ppr_row_class(int row) {
+  int c = 1;
+  while (c < row) c *= 2;
+  return c;
+}
+// Slices of 32 queries that a row's hub chunks are summed in.
+__host__ __device__ inline int ppr_slices(int row) { return (row + 31) / 32; }
+
+// Units longer than this go through the ring, a slice of 32 queries at a time
+// (ppr_long_units).  Short chains count while a round's rows are few (R-MAT-16,
+// 100 queries: 4.4 ms with 256, 4.9 with 1024, 6.6 with hub chunks only);
+// once they take longer than the chains, whole rows read by 16-byte words
+// move more (R-MAT-19, 100 queries: 24.4, 20.5 and 22.2 ms).
+constexpr int kPprLong[2] = {256, 1024};
+constexpr long long kPprFewBytes = 1500000000ll;  // gathered a round
+
+// The graph part of PprArgs, from a graph's PPR arrays (the block `mem`
+// holds unit records (4 words each) | slotFirst | slotCount | slotHub,
+// `units` and `slots` entries long).
 inline void ppr_args_graph(PprArgs &a, const int32_t *inSources, const int32_t *outDegree,
-                           const uint8_t *lastActive, const int32_t *mem, int32_t units,
-                           int32_t slots) {
+                           const int32_t *mem, int32_t units, const int32_t (&nLong)[2], int32_t slots,
+                           long long nEdges, int row) {
   const size_t nu = (size_t)(units > 0 ? units : 1), ns = (size_t)(slots > 0 ? slots : 1);
   a.inSources = inSources;
   a.outDegree = outDegree;
-  a.lastActive = lastActive;
   a.nUnits = units;
-  a.unitV = mem;
-  a.unitBeg = a.unitV + nu;
-  a.unitLen = a.unitBeg + nu;
-  a.unitSlot = a.unitLen + nu;
-  a.slotFirst = a.unitSlot + nu;
+  a.row = row;
+  a.nLong = nLong[4 * nEdges * row < kPprFewBytes ? 0 : 1];
+  a.unit = reinterpret_cast<const int4 *>(mem);
+  a.slotFirst = mem + 4 * nu;
   a.slotCount = a.slotFirst + ns;
   a.slotHub = a.slotCount + ns;
+}
+
+// Completes the unit records: the last round in which each vertex is active.
+static __global__ void ppr_unit_active_kernel(int4 *unit, int32_t nUnits, const uint8_t *lastActive) {
+  for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < nUnits; u += gridDim.x * blockDim.x)
+    unit[u].z |= (int)lastActive[unit[u].x] << 16;
 }
 
 __device__ __forceinline__ float ppr_contrib(float rank, int deg) {
@@ -208,25 +236,10 @@ static __global__ void ppr_active_step_kernel(int32_t nVertices, const int32_t *
   }
 }
 
-// Row width QP (queries per vertex row, a power of two 1..256) and how a
-// warp covers it: L lanes per unit (L = min(QP, 32)), G = 32 / L units per
-// warp, W = QP / L words of queries per lane (query of lane j, word k:
-// k * L + j), D edges gathered per step (their loads all in flight), M
-// source ids loaded per lane per step.
-template <int QP>
-struct PprShape {
-  static constexpr int L = QP < 32 ? QP : 32;
-  static constexpr int G = 32 / L;
-  static constexpr int W = QP / L;
-  static constexpr int D = W == 1 ? 32 : 32 / W;
-  static constexpr int M = D > L ? D / L : 1;
-};
-
 // rank := 1 at each query's source, 0 elsewhere (pagerank-style init of a
 // personalised run).
-template <int QP>
-__global__ void ppr_init_kernel(const PprArgs a) {
-  const size_t n = (size_t)a.nVertices * QP;
+static __global__ void ppr_init_kernel(const PprArgs a) {
+  const size_t n = (size_t)a.nVertices * a.row;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x) {
     a.rank[0][i] = 0.0f;
@@ -234,109 +247,302 @@ __global__ void ppr_init_kernel(const PprArgs a) {
   }
 }
 
-template <int QP>
-__global__ void ppr_sources_kernel(const PprArgs a) {
+static __global__ void ppr_sources_kernel(const PprArgs a) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= a.nQueries) return;
   const int s = a.sources[q];
-  a.rank[0][(size_t)s * QP + q] = 1.0f;
-  a.contrib[0][(size_t)s * QP + q] = ppr_contrib(1.0f, a.outDegree[s]);
+  a.rank[0][(size_t)s * a.row + q] = 1.0f;
+  a.contrib[0][(size_t)s * a.row + q] = ppr_contrib(1.0f, a.outDegree[s]);
 }
 
-// Round r: reads rank/contrib[r & 1], writes [(r + 1) & 1].  Groups of L
-// lanes take units longest first (the G groups of a warp get neighbouring
-// units, so similar lengths); a group loads D source ids per step (M per
-// lane, coalesced), issues the D gathered rows' loads, then each lane folds
-// its queries' D values in edge order.
+// This round's buffers (selects, not indexes, keep the parameters out of
+// local memory).
+struct PprRound {
+  const float *rk, *ct;
+  float *rk2, *ct2;
+  int r;
+};
+__device__ __forceinline__ PprRound ppr_buffers(const PprArgs &a, int r) {
+  const bool odd = (r & 1) != 0;
+  return {odd ? a.rank[1] : a.rank[0], odd ? a.contrib[1] : a.contrib[0], odd ? a.rank[0] : a.rank[1],
+          odd ? a.contrib[0] : a.contrib[1], r};
+}
+
+// Element idx (vertex v, query q) of the next rank and contribution.
+__device__ __forceinline__ void ppr_finish(const PprArgs &a, const PprRound &b, int v, int q, size_t idx, bool act,
+                                           float acc, int odeg) {
+  if (act) {
+    const float tele = (q < a.nQueries && a.sources[q] == v) ? a.teleport : 0.0f;
+    const float nr = __fadd_rn(tele, __fmul_rn(a.damp, acc));
+    b.rk2[idx] = nr;
+    b.ct2[idx] = ppr_contrib(nr, odeg);
+  } else {
+    b.rk2[idx] = __ldcg(b.rk + idx);
+    b.ct2[idx] = __ldcg(b.ct + idx);
+  }
+}
+
+// The left fold, in CSC order, of up to 32 neighbouring queries over the `len`
+// edges src[0..len) of a unit by one warp, lane q holding query q: the rows'
+// slices (C 16-byte words from `col` on, rows `row` floats apart) come through
+// a ring in shared memory, stages of 64 words with cp.async, and are added
+// from there.  A long unit's time is its chain; loads into registers leave one
+// batch of 16 or 32 rows in flight at a time and wait for all of it (two or
+// three L2 round trips of about 0.6 us for 32 edges, so that one 4,096-edge
+// chunk bounded every round of graphs up to R-MAT-18), the ring kPprStages
+// batches that arrive one by one.
+constexpr int kPprStages = 5;
+constexpr int kPprStageWords = 64;
+struct PprRing {
+  float4 word[kPprStages][kPprStageWords];
+};
+__device__ __forceinline__ float ppr_fold_ring(const int32_t *src, const float *col, size_t row, int C, int len,
+                                               PprRing &ring, int lane) {
+  const int SE = C > 4 ? 8 : C > 2 ? 16 : 32;  // edges of a stage: SE * C <= 64 words
+  const int e0 = lane / C, c0 = lane % C, e1 = (lane + 32) / C, c1 = (lane + 32) % C;
+  int blk = lane < len ? __ldg(src + lane) : 0;  // ids of the 32 edges being asked for
+  int next = 32 + lane < len ? __ldg(src + 32 + lane) : 0;
+  auto ask = [&](int t) {  // stage t
+    const int at = t * SE;
+    if (t > 0 && (at & 31) == 0) {  // the next 32 ids (warp-uniform)
+      blk = next;
+      next = at + 32 + lane < len ? __ldg(src + at + 32 + lane) : 0;
+    }
+    float4 *to = ring.word[t % kPprStages];
+    const int s0 = __shfl_sync(kFullMask, blk, (at + e0) & 31), s1 = __shfl_sync(kFullMask, blk, (at + e1) & 31);
+    if (e0 < SE && at + e0 < len) {
+      const unsigned d = (unsigned)__cvta_generic_to_shared(to + lane);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(col + (size_t)s0 * row + 4 * c0)
+                   : "memory");
+    }
+    if (e1 < SE && at + e1 < len) {
+      const unsigned d = (unsigned)__cvta_generic_to_shared(to + lane + 32);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(col + (size_t)s1 * row + 4 * c1)
+                   : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  const int stages = (len + SE - 1) / SE;
+  float acc = 0.0f;
+  for (int t = 0; t < kPprStages; ++t) ask(t);
+  for (int t = 0; t < stages; ++t) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kPprStages - 1) : "memory");
+    __syncwarp();
+    if (lane < 4 * C) {
+      const float *in = reinterpret_cast<const float *>(ring.word[t % kPprStages]) + lane;
+      const int n = min(SE, len - t * SE);
+      if (n == SE) {
+        for (int e = 0; e < SE; e += 8) {
+          float x[8];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) x[k] = in[(e + k) * 4 * C];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) acc = __fadd_rn(acc, x[k]);
+        }
+      } else {
+        for (int e = 0; e < n; ++e) acc = __fadd_rn(acc, in[e * 4 * C]);
+      }
+    }
+    __syncwarp();
+    ask(t + kPprStages);
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncwarp();
+  return acc;
+}
+
+// A hub chunk publishes its partial sums (this thread's: column q, counter
+// `counter`, lanes `mask` of the warp together, `lead` one of them); the last
+// of the vertex to arrive takes their sum in chunk order.  False: not the
+// last.
+__device__ __forceinline__ bool ppr_combine(const PprArgs &a, int slot, int q, bool mine, size_t counter,
+                                            unsigned mask, int leadLane, bool lead, float &acc) {
+  if (mine) a.partial[(size_t)slot * a.row + q] = acc;
+  __threadfence();
+  __syncwarp(mask);
+  unsigned last = 0u;
+  if (lead) {
+    const unsigned old = atomicAdd(a.arrive + counter, 1u);
+    last = (old + 1u) % (unsigned)a.slotCount[slot] == 0u ? 1u : 0u;
+  }
+  last = __shfl_sync(mask, last, leadLane);
+  if (!last) return false;
+  __threadfence();
+  const int first = a.slotFirst[slot], cnt = a.slotCount[slot];
+  float sum = 0.0f;
+  if (mine)
+    for (int c = 0; c < cnt; ++c) sum = __fadd_rn(sum, __ldcg(a.partial + (size_t)(first + c) * a.row + q));
+  acc = sum;
+  return true;
+}
+
+// The units [0, nLong), a slice of 32 queries each, a warp a slice.
+__device__ __forceinline__ void ppr_long_units(const PprArgs &a, const PprRound &b, PprRing &ring) {
+  const int lane = threadIdx.x & 31;
+  const long long warps = (long long)gridDim.x * (blockDim.x / 32);
+  const long long gw = (long long)(threadIdx.x / 32) * gridDim.x + blockIdx.x;
+  const int slices = ppr_slices(a.row);
+  for (long long i = gw; i < (long long)a.nLong * slices; i += warps) {
+    const int4 un = __ldg(a.unit + i / slices);
+    const int sl = (int)(i % slices), q = 32 * sl + lane, v = un.x, slot = un.w;
+    const bool act = (un.z >> 16) >= b.r;
+    const int len = act ? un.z & 0xffff : 0;
+    const bool mine = q < a.row;
+    const int odeg = __ldg(a.outDegree + v);
+    float acc = ppr_fold_ring(a.inSources + un.y, b.ct + 32 * sl, (size_t)a.row, min(a.row - 32 * sl, 32) / 4, len,
+                              ring, lane);
+    if (slot >= 0 &&
+        !ppr_combine(a, slot, q, mine, (size_t)a.slotHub[slot] * slices + sl, kFullMask, 0, lane == 0, acc))
+      continue;
+    if (mine) ppr_finish(a, b, v, q, (size_t)v * a.row + q, act, acc, odeg);
+  }
+}
+
+// Round r of rows of QP <= 32 floats: long units through the ring, then
+// groups of QP lanes take units (the groups of a warp neighbouring ones, so
+// similar lengths).  Work is dealt block-first, so that the longest units
+// spread over the SMs.  Rows of less than 16 bytes have no ring.
 template <int QP>
-__device__ __forceinline__ void ppr_round(const PprArgs &a, int r) {
-  using S = PprShape<QP>;
-  constexpr int L = S::L, G = S::G, W = S::W, D = S::D, M = S::M;
+__device__ __forceinline__ void ppr_round_narrow(const PprArgs &a, int r, PprRing &ring) {
+  constexpr int L = QP, G = 32 / L, M = 32 / L;
+  const PprRound b = ppr_buffers(a, r);
   const int lane = threadIdx.x & 31;
   const int grp = lane / L, j = lane % L;
   const long long warps = (long long)gridDim.x * (blockDim.x / 32);
-  const long long gw = (long long)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-  const bool odd = (r & 1) != 0;  // selects, not indexes (keeps the params out of local memory)
-  const float *rk = odd ? a.rank[1] : a.rank[0];
-  const float *ct = odd ? a.contrib[1] : a.contrib[0];
-  float *rk2 = odd ? a.rank[0] : a.rank[1];
-  float *ct2 = odd ? a.contrib[0] : a.contrib[1];
-  for (long long base = gw * G; base < a.nUnits; base += warps * G) {
+  const long long gw = (long long)(threadIdx.x / 32) * gridDim.x + blockIdx.x;
+  const unsigned mask = L == 32 ? kFullMask : (((1u << (L & 31)) - 1u) << (grp * L));
+  long long first = 0;
+  if constexpr (QP >= 4) {
+    ppr_long_units(a, b, ring);
+    first = a.nLong;
+  }
+  for (long long base = first + gw * G; base < a.nUnits; base += warps * G) {
     const long long u = base + grp;
-    const bool valid = u < a.nUnits;
-    const int v = valid ? a.unitV[u] : 0;
-    const int beg = valid ? a.unitBeg[u] : 0;
-    const int len = valid ? a.unitLen[u] : 0;
-    const bool isAct = valid && (int)a.lastActive[v] >= r;
-    const int maxLen = __reduce_max_sync(kFullMask, isAct ? len : 0);
-    float acc[W];
+    const int4 un = u < a.nUnits ? __ldg(a.unit + u) : make_int4(-1, 0, 0, -1);
+    const int v = un.x, slot = un.w;
+    const bool act = v >= 0 && (un.z >> 16) >= r;
+    const int len = act ? un.z & 0xffff : 0;
+    const int odeg = v >= 0 ? __ldg(a.outDegree + v) : 0;
+    const int maxLen = __reduce_max_sync(kFullMask, len);
+    const int32_t *src = a.inSources + un.y;
+    float acc = 0.0f;
+    int ids[M];
 #pragma unroll
-    for (int k = 0; k < W; ++k) acc[k] = 0.0f;
-    for (int o = 0; o < maxLen; o += D) {  // warp-uniform trip count
-      int ids[M];
+    for (int m = 0; m < M; ++m) ids[m] = m * L + j < len ? __ldg(src + m * L + j) : 0;
+    for (int o = 0; o < maxLen; o += 32) {  // warp-uniform
+      float c[32];
 #pragma unroll
-      for (int m = 0; m < M; ++m) {
-        const int t = m * L + j;
-        ids[m] = (t < D && o + t < len) ? __ldg(a.inSources + beg + o + t) : 0;
-      }
-      const int n = isAct ? min(D, len - o) : 0;  // this group's edges in the step
-      float c[D][W];
-#pragma unroll
-      for (int t = 0; t < D; ++t) {
-        const int sj = __shfl_sync(kFullMask, ids[t / L], t % L, L);
-#pragma unroll
-        for (int k = 0; k < W; ++k)
-          c[t][k] = t < n ? __ldcg(ct + (size_t)sj * QP + k * L + j) : 0.0f;
+      for (int t = 0; t < 32; ++t) {
+        const int s = __shfl_sync(kFullMask, ids[t / L], t % L, L);
+        c[t] = t < len - o ? b.ct[(size_t)s * QP + j] : 0.0f;
       }
 #pragma unroll
-      for (int t = 0; t < D; ++t)
+      for (int m = 0; m < M; ++m) ids[m] = o + 32 + m * L + j < len ? __ldg(src + o + 32 + m * L + j) : 0;
 #pragma unroll
-        for (int k = 0; k < W; ++k)
-          if (t < n) acc[k] = __fadd_rn(acc[k], c[t][k]);
+      for (int t = 0; t < 32; ++t)
+        if (t < len - o) acc = __fadd_rn(acc, c[t]);
     }
-    // hub chunks: publish the partial sums; the last chunk to arrive adds
-    // them in chunk order and finishes the vertex
-    const int slot = valid ? a.unitSlot[u] : -1;
-    unsigned arrived = 0u;
-    if (slot >= 0) {
+    if (v < 0) continue;
+    if (slot >= 0 && !ppr_combine(a, slot, j, true, (size_t)a.slotHub[slot], mask, grp * L, j == 0, acc)) continue;
+    ppr_finish(a, b, v, j, (size_t)v * QP + j, act, acc, odeg);
+  }
+}
+
+// Round r of wider rows (a.row floats, a multiple of 8 up to QP).  Long
+// units and hub chunks are taken a slice of 32 queries at a time, a lane per
+// query, so that their chains run in parallel; the others a whole row at a
+// time, four neighbouring queries a lane (one 16-byte load an edge and lane
+// instead of four 4-byte ones).
+template <int QP>
+__device__ __forceinline__ void ppr_round_wide(const PprArgs &a, int r, PprRing &ring) {
+  constexpr int L = QP / 4 < 32 ? QP / 4 : 32;  // lanes of a unit
+  constexpr int G = 32 / L, NV = QP / (4 * L);  // units a warp, 16-byte words a lane
+  constexpr int D = 8 / NV;                     // edges a step
+  const PprRound b = ppr_buffers(a, r);
+  const int lane = threadIdx.x & 31;
+  const long long warps = (long long)gridDim.x * (blockDim.x / 32);
+  const long long gw = (long long)(threadIdx.x / 32) * gridDim.x + blockIdx.x;
+  ppr_long_units(a, b, ring);
+  const int grp = lane / L, j = lane % L;
+  for (long long base = a.nLong + gw * G; base < a.nUnits; base += warps * G) {
+    const long long u = base + grp;
+    const int4 un = u < a.nUnits ? __ldg(a.unit + u) : make_int4(-1, 0, 0, -1);
+    const int v = un.x;
+    const bool act = v >= 0 && (un.z >> 16) >= r;
+    const int len = act ? un.z & 0xffff : 0;
+    const int odeg = v >= 0 ? __ldg(a.outDegree + v) : 0;
+    const int maxLen = __reduce_max_sync(kFullMask, len);
+    float4 acc[NV];
+    bool on[NV];
 #pragma unroll
-      for (int k = 0; k < W; ++k) a.partial[(size_t)slot * QP + k * L + j] = acc[k];
-      __threadfence();
-      __syncwarp(L == 32 ? kFullMask : (((1u << L) - 1u) << (grp * L)));
-      if (j == 0) {
-        const unsigned old = atomicAdd(a.arrive + a.slotHub[slot], 1u);
-        arrived = (old + 1u) % (unsigned)a.slotCount[slot] == 0u ? 1u : 0u;
-      }
+    for (int k = 0; k < NV; ++k) {
+      acc[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      on[k] = 4 * (j + L * k) < a.row;
     }
-    const unsigned last = __shfl_sync(kFullMask, arrived, grp * L);
-    if (!valid || (slot >= 0 && !last)) continue;
-    if (slot >= 0) {
-      __threadfence();
-      const int first = a.slotFirst[slot], cnt = a.slotCount[slot];
+    const int32_t *src = a.inSources + un.y;
+    int ids = j < len ? __ldg(src + j) : 0;
+    for (int o = 0; o < maxLen; o += L) {  // warp-uniform
+      const int next = o + L + j < len ? __ldg(src + o + L + j) : 0;
+      for (int d = 0; d < L && o + d < maxLen; d += D) {
+        const int n = len - o - d;  // edges from this step on (<= 0: none)
+        float4 c[D][NV];
 #pragma unroll
-      for (int k = 0; k < W; ++k) {
-        float sum = 0.0f;
-        for (int c = 0; c < cnt; ++c)
-          sum = __fadd_rn(sum, __ldcg(a.partial + (size_t)(first + c) * QP + k * L + j));
-        acc[k] = sum;
+        for (int t = 0; t < D; ++t) {
+          const int s = __shfl_sync(kFullMask, ids, d + t, L);
+          const float4 *row = reinterpret_cast<const float4 *>(b.ct + (size_t)s * a.row) + j;
+#pragma unroll
+          for (int k = 0; k < NV; ++k)
+            c[t][k] = t < n && on[k] ? row[L * k] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+#pragma unroll
+        for (int t = 0; t < D; ++t)
+          if (t < n) {
+#pragma unroll
+            for (int k = 0; k < NV; ++k) {
+              acc[k].x = __fadd_rn(acc[k].x, c[t][k].x);
+              acc[k].y = __fadd_rn(acc[k].y, c[t][k].y);
+              acc[k].z = __fadd_rn(acc[k].z, c[t][k].z);
+              acc[k].w = __fadd_rn(acc[k].w, c[t][k].w);
+            }
+          }
       }
+      ids = next;
     }
-    const int odeg = a.outDegree[v];
+    if (v < 0) continue;
 #pragma unroll
-    for (int k = 0; k < W; ++k) {
-      const int q = k * L + j;
-      const size_t idx = (size_t)v * QP + q;
-      if (isAct) {
-        const float tele = (q < a.nQueries && a.sources[q] == v) ? a.teleport : 0.0f;
-        const float nr = __fadd_rn(tele, __fmul_rn(a.damp, acc[k]));
-        rk2[idx] = nr;
-        ct2[idx] = ppr_contrib(nr, odeg);
+    for (int k = 0; k < NV; ++k) {
+      if (!on[k]) continue;
+      const int q = 4 * (j + L * k);
+      const size_t at = ((size_t)v * a.row + q) / 4;
+      float4 nr, nc;
+      if (act) {
+        const int4 s = __ldg(reinterpret_cast<const int4 *>(a.sources) + q / 4);
+        auto rank = [&](float x, int source, int qi) {
+          const float tele = (qi < a.nQueries && source == v) ? a.teleport : 0.0f;
+          return __fadd_rn(tele, __fmul_rn(a.damp, x));
+        };
+        nr = make_float4(rank(acc[k].x, s.x, q), rank(acc[k].y, s.y, q + 1), rank(acc[k].z, s.z, q + 2),
+                         rank(acc[k].w, s.w, q + 3));
+        nc = make_float4(ppr_contrib(nr.x, odeg), ppr_contrib(nr.y, odeg), ppr_contrib(nr.z, odeg),
+                         ppr_contrib(nr.w, odeg));
       } else {
-        rk2[idx] = __ldcg(rk + idx);
-        ct2[idx] = __ldcg(ct + idx);
+        nr = __ldcg(reinterpret_cast<const float4 *>(b.rk) + at);
+        nc = __ldcg(reinterpret_cast<const float4 *>(b.ct) + at);
       }
+      reinterpret_cast<float4 *>(b.rk2)[at] = nr;
+      reinterpret_cast<float4 *>(b.ct2)[at] = nc;
     }
   }
+}
+
+template <int QP>
+__device__ __forceinline__ void ppr_round(const PprArgs &a, int r) {
+  __shared__ PprRing rings[8];  // a warp's each (256 threads)
+  PprRing &ring = rings[threadIdx.x / 32];
+  if constexpr (QP <= 32)
+    ppr_round_narrow<QP>(a, r, ring);
+  else
+    ppr_round_wide<QP>(a, r, ring);
 }
 
 template <int QP>

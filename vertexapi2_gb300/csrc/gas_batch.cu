@@ -329,10 +329,14 @@ gas_status enqueue_batch(gas_batch *b, const CoreGraph &g, int kind, int32_t nQ,
 
 // ---- personalised PageRank batches
 // State of a batch with rows of QP queries: rank[2] | contrib[2] ([V][QP]
-// floats each) | partial ([slots][QP]) | arrive ([hubs]) | out ([QP][V]).
+// floats each) | partial ([slots][QP]) | arrive ([hubs][slices]) | out ([QP][V]).
+size_t ppr_arrivals(const gas_batch *b, int QP) {
+  return (size_t)std::max(b->ppr.hubs, 1) * gas::detail::ppr_slices(QP);
+}
+
 size_t ppr_state_bytes(const gas_batch *b, const CoreGraph &g, int QP) {
   const size_t V = (size_t)std::max(g.nV, 1);
-  return 4 * (5 * V * QP + (size_t)std::max(b->ppr.slots, 1) * QP + (size_t)std::max(b->ppr.hubs, 1)) + 256;
+  return 4 * (5 * V * QP + (size_t)std::max(b->ppr.slots, 1) * QP + ppr_arrivals(b, QP)) + 256;
 }
 
 gas::detail::PprArgs ppr_args(gas_batch *b, const CoreGraph &g, int32_t nQ, int QP) {
@@ -340,8 +344,8 @@ gas::detail::PprArgs ppr_args(gas_batch *b, const CoreGraph &g, int32_t nQ, int 
   memset(&a, 0, sizeof(a));
   a.nVertices = g.nV;
   a.nQueries = nQ;
-  gas::detail::ppr_args_graph(a, g.inSrc, b->ppr.outDegree, b->ppr.lastActive, b->ppr.mem,
-                              b->ppr.units, b->ppr.slots);
+  gas::detail::ppr_args_graph(a, g.inSrc, b->ppr.outDegree, b->ppr.mem, b->ppr.units, b->ppr.nLong,
+                              b->ppr.slots, g.nE, QP);
   const size_t V = (size_t)std::max(g.nV, 1);
   float *p = reinterpret_cast<float *>(b->pprState);
   a.rank[0] = p;
@@ -359,7 +363,7 @@ gas::detail::PprArgs ppr_args(gas_batch *b, const CoreGraph &g, int32_t nQ, int 
 float *ppr_out(gas_batch *b, const CoreGraph &g, int QP) {
   const size_t V = (size_t)std::max(g.nV, 1);
   return reinterpret_cast<float *>(b->pprState) + 4 * V * QP + (size_t)std::max(b->ppr.slots, 1) * QP +
-         (size_t)std::max(b->ppr.hubs, 1);
+         ppr_arrivals(b, QP);
 }
 
 template <int QP>
@@ -381,26 +385,6 @@ const void *ppr_run_fn_for(int QP) {
   }
 }
 
-template <int QP>
-void ppr_start(const gas::detail::PprArgs &a, int blocks, cudaStream_t s) {
-  gas::detail::ppr_init_kernel<QP><<<blocks, 256, 0, s>>>(a);
-  gas::detail::ppr_sources_kernel<QP><<<1, kMaxBatch, 0, s>>>(a);
-}
-
-void ppr_start_for(int QP, const gas::detail::PprArgs &a, int blocks, cudaStream_t s) {
-  switch (QP) {
-    case 1: ppr_start<1>(a, blocks, s); break;
-    case 2: ppr_start<2>(a, blocks, s); break;
-    case 4: ppr_start<4>(a, blocks, s); break;
-    case 8: ppr_start<8>(a, blocks, s); break;
-    case 16: ppr_start<16>(a, blocks, s); break;
-    case 32: ppr_start<32>(a, blocks, s); break;
-    case 64: ppr_start<64>(a, blocks, s); break;
-    case 128: ppr_start<128>(a, blocks, s); break;
-    default: ppr_start<256>(a, blocks, s); break;
-  }
-}
-
 // The whole PPR batch on b->stream: sources, arrival counters, initial
 // ranks, every round in one cooperative launch, query-major ranks in out.
 gas_status enqueue_ppr(gas_batch *b, const CoreGraph &g, int32_t nQ, int QP) {
@@ -408,13 +392,14 @@ gas_status enqueue_ppr(gas_batch *b, const CoreGraph &g, int32_t nQ, int QP) {
                                   cudaMemcpyHostToDevice, b->stream);
   gas::detail::PprArgs a = ppr_args(b, g, nQ, QP);
   if (e == cudaSuccess && b->ppr.hubs > 0)
-    e = cudaMemsetAsync(a.arrive, 0, 4 * (size_t)b->ppr.hubs, b->stream);
+    e = cudaMemsetAsync(a.arrive, 0, 4 * ppr_arrivals(b, QP), b->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(b->ctl, 0, kCtlBytes, b->stream);
   if (e != cudaSuccess) return cuda_fail(e, "PPR batch reset");
-  ppr_start_for(QP, a, 4 * b->sms, b->stream);
+  gas::detail::ppr_init_kernel<<<4 * b->sms, 256, 0, b->stream>>>(a);
+  gas::detail::ppr_sources_kernel<<<1, kMaxBatch, 0, b->stream>>>(a);
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "PPR batch init");
-  const void *fn = ppr_run_fn_for(QP);
+  const void *fn = ppr_run_fn_for(gas::detail::ppr_row_class(QP));
   int per = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, 256, 0);
   if (b->blocksPerSM > 0 && b->blocksPerSM < per) per = b->blocksPerSM;
@@ -434,8 +419,7 @@ gas_status enqueue_ppr(gas_batch *b, const CoreGraph &g, int32_t nQ, int QP) {
 
 gas_status run_one_ppr(gas_batch *b, const CoreGraph &g, int32_t nQ, const int32_t *sources,
                        float *results, int32_t *rounds) {
-  int QP = 1;
-  while (QP < nQ) QP *= 2;
+  const int QP = gas::detail::ppr_row_width(nQ);
   if (!b->ppr.mem) {
     gas_status st = gas::internal::build_ppr_graph(g, b->sms, b->pprRounds, &b->ppr);
     if (st) return st;

@@ -199,10 +199,11 @@ class Server {
 
 Batch::~Batch() {}
 
-// Queries per vertex row of a batch of n: BFS/SSSP at least 32 (a word of
-// query bits), PPR the next power of two.
+// Queries per vertex row of a batch of n: BFS/SSSP a power of two, at least
+// 32 (a word of query bits), PPR its own row width.
 int row_width(int kind, int n) {
-  int Q = kind == 2 ? 1 : 32;
+  if (kind == 2) return gas::detail::ppr_row_width(n);
+  int Q = 32;
   while (Q < n) Q *= 2;
   return Q;
 }
@@ -222,7 +223,8 @@ int64_t Server::state_bytes(const ServeGraph &g, int kind, int Q) const {
                         (use_pairs(g, kind, Q) ? 12 * V * Q : 0);
   if (kind == 0) return base + V * Q * 4 + 16 * V * W + lists;
   if (kind == 1) return base + V * Q * 4 + 12 * V * W + lists;
-  return base + V * Q * 16 + (int64_t)g.ppr.slots * Q * 4 + (int64_t)g.ppr.hubs * 4;
+  return base + V * Q * 16 + (int64_t)g.ppr.slots * Q * 4 +
+         (int64_t)g.ppr.hubs * gas::detail::ppr_slices(Q) * 4;
 }
 
 int64_t Server::available_bytes() {
@@ -328,13 +330,7 @@ void ppr_round_launch(const gas::detail::PprArgs &a, int r, int blocks, cudaStre
   gas::detail::ppr_round_kernel<QP><<<blocks, 256, 0, s>>>(a, r);
 }
 
-template <int QP>
-void ppr_start_launch(const gas::detail::PprArgs &a, int blocks, cudaStream_t s) {
-  gas::detail::ppr_init_kernel<QP><<<blocks, 256, 0, s>>>(a);
-  gas::detail::ppr_sources_kernel<QP><<<1, kMaxQ, 0, s>>>(a);
-}
-
-// FN<QP>(args...) for the batch's PPR row width QP (a power of two <= 256).
+// FN<QP>(args...) for the batch's PPR row class QP (a power of two <= 256).
 #define GAS_PPR_WIDTH(QPV, FN, ...)               \
   switch (QPV) {                                  \
     case 1: FN<1>(__VA_ARGS__); break;            \
@@ -386,7 +382,7 @@ void enqueue_round(Batch &b, int r, int blocks) {
 }
 
 void enqueue_ppr_round(Batch &b, int r, int blocks) {
-  GAS_PPR_WIDTH(b.Q, ppr_round_launch, b.pa, r, blocks, b.stream)
+  GAS_PPR_WIDTH(gas::detail::ppr_row_class(b.Q), ppr_round_launch, b.pa, r, blocks, b.stream)
 }
 
 int round_blocks(const Server &s, int64_t warpsOfWork) {
@@ -412,8 +408,10 @@ void Server::issue_chunk(int l, int rounds, bool final) {
       launches += 1;
     }
   } else if (b.kind == 2) {
-    const int G = 32 / std::min(b.Q, 32);  // units per warp
-    const int blocks = round_blocks(*this, (b.g->ppr.units + G - 1) / G);
+    const int cls = gas::detail::ppr_row_class(b.Q);
+    const int G = cls > 32 ? std::max(1, 128 / cls) : 32 / cls;  // units per warp
+    const int blocks = round_blocks(*this, (int64_t)gas::detail::ppr_slices(b.Q) * b.pa.nLong +
+                                               (b.g->ppr.units + G - 1) / G);
     for (int k = 0; k < rounds; ++k) enqueue_ppr_round(b, b.roundsIssued + k, blocks);
     b.roundsIssued += rounds;
     launches += rounds;
@@ -480,21 +478,23 @@ gas_status Server::launch(int l, const std::shared_ptr<Batch> &bp) {
     a.nVertices = V;
     a.nQueries = b.nQ;
     a.inSources = g.bg.g.inSrc;
-    gas::detail::ppr_args_graph(a, g.bg.g.inSrc, g.ppr.outDegree, g.ppr.lastActive, g.ppr.mem,
-                                g.ppr.units, g.ppr.slots);
+    gas::detail::ppr_args_graph(a, g.bg.g.inSrc, g.ppr.outDegree, g.ppr.mem, g.ppr.units, g.ppr.nLong,
+                                g.ppr.slots, g.bg.g.nE, b.Q);
     a.sources = b.sources;
     for (int k = 0; k < 2; ++k) {
       a.rank[k] = reinterpret_cast<float *>(take(Vs * b.Q * 4));
       a.contrib[k] = reinterpret_cast<float *>(take(Vs * b.Q * 4));
     }
     a.partial = reinterpret_cast<float *>(take((size_t)g.ppr.slots * b.Q * 4));
-    a.arrive = reinterpret_cast<unsigned *>(take((size_t)g.ppr.hubs * 4));
-    if (g.ppr.hubs > 0) cudaMemsetAsync(a.arrive, 0, (size_t)g.ppr.hubs * 4, b.stream);
+    const size_t arrivals = (size_t)g.ppr.hubs * gas::detail::ppr_slices(b.Q) * 4;
+    a.arrive = reinterpret_cast<unsigned *>(take(arrivals));
+    if (arrivals > 0) cudaMemsetAsync(a.arrive, 0, arrivals, b.stream);
     if (p - b.state > b.stateBytes) return fail(GAS_ERR_STATE, "batch state layout overflow");
     a.teleport = 0.15f;
     a.damp = 1.0f - a.teleport;  // as PPR::apply computes it, in float
     const int blocks = 4 * sms;
-    GAS_PPR_WIDTH(b.Q, ppr_start_launch, a, blocks, b.stream)
+    gas::detail::ppr_init_kernel<<<blocks, 256, 0, b.stream>>>(a);
+    gas::detail::ppr_sources_kernel<<<1, kMaxQ, 0, b.stream>>>(a);
   } else {
     gas::detail::BatchArgs &a = b.ba;
     memset(&a, 0, sizeof(a));
@@ -1059,18 +1059,21 @@ gas_status build_ppr_graph(const CoreGraph &cg, int sms, int rounds, PprGraph *o
     ++hubs;
   }
   const size_t nu = uv.size(), ns = sf.size();
-  // counting sort by length, longest first (stable)
-  std::vector<int64_t> pos((size_t)C + 2, 0);
-  for (size_t i = 0; i < nu; ++i) ++pos[(size_t)(C - ul[i]) + 1];
+  // counting sort by length, longest first (stable), after the hub chunks
+  std::vector<int64_t> pos((size_t)C + 3, 0);
+  auto key = [&](size_t i) { return us[i] >= 0 ? (size_t)0 : (size_t)(C - ul[i]) + 1; };
+  for (size_t i = 0; i < nu; ++i) ++pos[key(i) + 1];
   for (size_t k = 1; k < pos.size(); ++k) pos[k] += pos[k - 1];
-  std::vector<int32_t> mem(4 * std::max<size_t>(nu, 1) + 3 * std::max<size_t>(ns, 1), 0);
   const size_t nuA = std::max<size_t>(nu, 1), nsA = std::max<size_t>(ns, 1);
+  std::vector<int32_t> mem(4 * nuA + 3 * nsA, 0);
+  g.nLong[0] = g.nLong[1] = 0;
   for (size_t i = 0; i < nu; ++i) {
-    const size_t p = (size_t)pos[(size_t)(C - ul[i])]++;
-    mem[p] = uv[i];
-    mem[nuA + p] = ub[i];
-    mem[2 * nuA + p] = ul[i];
-    mem[3 * nuA + p] = us[i];
+    int32_t *rec = &mem[4 * (size_t)pos[key(i)]++];
+    rec[0] = uv[i];
+    rec[1] = ub[i];
+    rec[2] = ul[i];
+    rec[3] = us[i];
+    for (int k = 0; k < 2; ++k) g.nLong[k] += us[i] >= 0 || ul[i] > gas::detail::kPprLong[k];
   }
   for (size_t i = 0; i < ns; ++i) {
     mem[4 * nuA + i] = sf[i];
@@ -1080,20 +1083,24 @@ gas_status build_ppr_graph(const CoreGraph &cg, int sms, int rounds, PprGraph *o
   g.units = (int32_t)nu;
   g.slots = (int32_t)ns;
   g.hubs = hubs;
-  uint8_t *tmp = nullptr;
+  uint8_t *tmp = nullptr;  // two active sets | lastActive
   const size_t Vs = (size_t)std::max(V, 1);
   cudaError_t e = cudaMalloc(&g.outDegree, 4 * Vs);
   if (e == cudaSuccess) e = cudaMalloc(&g.mem, 4 * mem.size());
-  if (e == cudaSuccess) e = cudaMalloc(&g.lastActive, Vs);
-  if (e == cudaSuccess) e = cudaMalloc(&tmp, 2 * Vs);
+  if (e == cudaSuccess) e = cudaMalloc(&tmp, 3 * Vs);
   if (e == cudaSuccess) e = cudaMemcpy(g.outDegree, deg.data(), 4 * Vs, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(g.mem, mem.data(), 4 * mem.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemset(g.lastActive, 0, Vs);
+  uint8_t *lastActive = tmp + 2 * Vs;
+  if (e == cudaSuccess) e = cudaMemset(lastActive, 0, Vs);
   if (e == cudaSuccess) e = cudaMemset(tmp, 1, Vs);  // A0: every vertex
   for (int k = 1; k < rounds && e == cudaSuccess && V > 0; ++k) {
     uint8_t *cur = tmp + ((k - 1) & 1) * Vs, *nxt = tmp + (k & 1) * Vs;
     gas::detail::ppr_active_step_kernel<<<4 * sms, 256>>>(V, cg.inOff, cg.inSrc, cur, nxt,
-                                                           g.lastActive, k);
+                                                           lastActive, k);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess && nu > 0) {
+    gas::detail::ppr_unit_active_kernel<<<4 * sms, 256>>>(reinterpret_cast<int4 *>(g.mem), g.units, lastActive);
     e = cudaGetLastError();
   }
   // the legacy default stream: ordered after the memsets, not with the lanes
@@ -1108,7 +1115,6 @@ gas_status build_ppr_graph(const CoreGraph &cg, int sms, int rounds, PprGraph *o
 
 void free_ppr_graph(PprGraph *p) {
   if (p->outDegree) cudaFree(p->outDegree);
-  if (p->lastActive) cudaFree(p->lastActive);
   if (p->mem) cudaFree(p->mem);
   *p = PprGraph();
 }
