@@ -184,27 +184,31 @@ __device__ __forceinline__ void batch_unit(const BatchArgs &a, int u, int round,
         any |= m[k];
       }
       unsigned work = __ballot_sync(kFullMask, any != 0u);  // edges with a changed query
-      while (work) {  // warp-uniform; four edges' loads in flight per pass
-        int js[4];
+      // warp-uniform; the values of T edges in flight a lane (32 loads at
+      // most): a unit's time is one L2 round trip for each batch of them
+      // (R-MAT-18: 10 queries 4.06 -> 1.99 ms a run, 64 queries 8.36 -> 3.75,
+      // 256 queries 16.1 -> 13.6, from four edges in flight to T)
+      constexpr int T = W == 1 ? 16 : 32 / W;
+      while (work) {
+        int d[T][W];
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          js[t] = work ? __ffs(work) - 1 : -1;
+        for (int t = 0; t < T; ++t) {
+          const int js = work ? __ffs(work) - 1 : 0;
+          const bool on = work != 0u;
           if (work) work &= work - 1;
-        }
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          if (js[t] < 0) continue;
-          const int sj = __shfl_sync(kFullMask, s, js[t]);
-          const int wj = __shfl_sync(kFullMask, w, js[t]);
+          const int sj = __shfl_sync(kFullMask, s, js);
+          const int wj = __shfl_sync(kFullMask, w, js);
 #pragma unroll
           for (int k = 0; k < W; ++k) {
-            const unsigned mk = __shfl_sync(kFullMask, m[k], js[t]);
-            if ((mk >> lane) & 1u) {
-              const int d = __ldcg(a.value + (size_t)sj * Q + k * 32 + lane);
-              best[k] = min(best[k], d + wj);
-            }
+            const unsigned mk = __shfl_sync(kFullMask, m[k], js);
+            d[t][k] = kBatchInf;
+            if (on && ((mk >> lane) & 1u)) d[t][k] = __ldcg(a.value + (size_t)sj * Q + k * 32 + lane) + wj;
           }
         }
+#pragma unroll
+        for (int t = 0; t < T; ++t)
+#pragma unroll
+          for (int k = 0; k < W; ++k) best[k] = min(best[k], d[t][k]);
       }
     }
 #pragma unroll
