@@ -73,11 +73,11 @@ struct BatchArgs {
   int32_t delta;
   int32_t *thresh[2];      // [Q] by round parity
   unsigned *nearFlag[3];   // [W] queries with a new value below the bound (rotating)
-  // Pair frontier (graphs of small out-degree, V * Q < 2^31): the changed
-  // set is a list of (vertex, query) entries u * Q + q, one lane each,
-  // instead of vertex entries with query masks; every round pushes.
+  // Pair frontier (graphs of small out-degree, V * Q < 2^31): a thread per
+  // changed (vertex, query) instead of a warp per vertex entry; state
+  // query-major; every round pushes.  kPairsList: entries u * Q + q.
+  int32_t pairMode;        // PairMode
   uint32_t *pairs[3];      // [V * Q] each (rotating, counts in listCnt >> 32)
-  int32_t pairMode;
 };
 
 // Shared-memory view of the bucket bounds for one round (null when off).
@@ -378,17 +378,167 @@ __device__ __forceinline__ void batch_push_unit(const BatchArgs &a, int u, int c
   }
 }
 
-// Appends each lane's entry (when `want`) to a pair list: one atomic per
-// warp.  Warp-uniform call.
-__device__ __forceinline__ void warp_append_pair(bool want, uint32_t entry, uint32_t *list,
-                                                 unsigned long long *cnt) {
-  const int lane = threadIdx.x & 31;
-  const unsigned who = __ballot_sync(kFullMask, want);
-  if (!who) return;
-  unsigned long long base = 0ull;
-  if (lane == 0) base = atomicAdd(cnt, (unsigned long long)__popc(who) << 32);
-  base = __shfl_sync(kFullMask, base, 0) >> 32;
-  if (want) list[base + __popc(who & ((1u << lane) - 1u))] = entry;
+// ---- pair frontiers (graphs of small out-degree)
+// State is query-major (value[q][v], mask and seen words [w][v]), so that
+// the vertices of one query's wavefront touch neighbouring words.  The
+// changed set is the round's mask, or a list as well (below).
+//
+// From the mask: activation is one reduction into the next round's mask,
+// which also removes duplicates: no list, no counter that every warp contends
+// for, and nothing to wait for.  Each block owns groups of 32 consecutive
+// mask words (a warp reads one in a coalesced load), lists their set bits in
+// shared memory, zeroes the words (so the mask is clean when it next collects
+// bits) and relaxes a listed (vertex, query) a thread: a chain of four L2
+// round trips a round (mask; value and row bounds; row; atomic) where list
+// appends take seven.  64 SSSP queries, delta 512, from lists and from the
+// mask: 256 x 256 lattice 6.9 -> 3.4 ms, 506 x 506 16.2 -> 9.4, 1000 x 1000
+// 48 -> 35 (256 queries 193 -> 154); 64 BFS queries, 256 x 256 3.25 -> 2.06.
+//
+// From a list, for BFS over large masks: its rounds are short against the
+// passes over the mask (64 queries, 1000 x 1000: 21.7 ms from the mask, 19.1
+// from the list).
+constexpr long long kPairMaskWords = 1ll << 20;  // BFS: lists above
+enum PairMode { kPairsOff = 0, kPairsMask = 1, kPairsList = 2 };
+inline int pair_mode_of(bool bfs, long long nVertices, int W) {
+  return bfs && nVertices * W > kPairMaskWords ? kPairsList : kPairsMask;
+}
+constexpr int kPairList = 1024;  // pairs a block lists at a time
+constexpr int kPairWords = 8;    // mask words a thread reads a pass, half of them where that covers the mask
+
+// Blocks of a persistent run over the mask.  A round is a chain of round trips
+// and a grid barrier, which costs more the more blocks arrive: enough of them
+// to read the mask in one pass and for a wavefront of about 5 sqrt(V)
+// vertices a query, a pair a thread; whole blocks per SM (64 SSSP queries,
+// 256 x 256 lattice: 3.65, 3.42 and 3.96 ms at 4, 2 and 1 an SM; 506 x 506:
+// 9.4, 12.2, 19.6).
+inline int batch_pair_blocks(int32_t nVertices, int W, int nQ, int sms) {
+  double root = 1.0;
+  while (root * root < (double)nVertices) root *= 1.1;
+  const double words = (double)nVertices * W, front = 5.0 * root * nQ;
+  const double want = (words / kPairWords > front ? words / kPairWords : front) / 256;
+  const int perSM = (int)(want / (sms > 0 ? sms : 1) + 0.5);
+  return (perSM > 1 ? perSM : 1) * (sms > 0 ? sms : 1);
+}
+
+struct PairSmem {
+  uint32_t entry[kPairList];
+  unsigned warpTot[8];
+};
+
+// Relaxes the out-edges of pair (u, q) for query q alone.
+template <int W, int KIND>
+__device__ __forceinline__ void batch_pair(const BatchArgs &a, int u, int q, int round, unsigned *nxt,
+                                           unsigned long long &changed, const BatchBucket bk) {
+  const unsigned bit = 1u << (q & 31);
+  const int wq = q >> 5;
+  const size_t V = (size_t)a.nVertices;
+  const int eb = a.outOffsets[u], ee = a.outOffsets[u + 1];
+  unsigned *nw = nxt + (size_t)wq * V;
+  int du = 0;
+  if (KIND == kBatchSSSP) {
+    du = __ldcg(a.value + (size_t)q * V + u);
+    if (bk.bound && du >= bk.bound[q]) {  // not this bucket: keep (u, q) for later
+      atomicOr(nw + u, bit);
+      ++changed;
+      return;
+    }
+  }
+  constexpr int J = 4;  // edges in flight
+  for (int e0 = eb; e0 < ee; e0 += J) {
+    int v[J], x[J];
+#pragma unroll
+    for (int t = 0; t < J; ++t) {
+      v[t] = e0 + t < ee ? __ldg(a.outDests + e0 + t) : -1;
+      if (KIND == kBatchSSSP) x[t] = e0 + t < ee ? du + __ldg(a.weightsOut + e0 + t) : 0;
+    }
+    int old[J];
+#pragma unroll
+    for (int t = 0; t < J; ++t)
+      if (v[t] >= 0) {
+        if (KIND == kBatchBFS)
+          old[t] = (int)atomicOr(a.seen + (size_t)wq * V + v[t], bit);
+        else
+          old[t] = atomicMin(a.value + (size_t)q * V + v[t], x[t]);
+      }
+#pragma unroll
+    for (int t = 0; t < J; ++t) {
+      if (v[t] < 0) continue;
+      if (KIND == kBatchBFS) {
+        if ((unsigned)old[t] & bit) continue;
+        a.value[(size_t)q * V + v[t]] = round + 1;
+      } else {
+        if (x[t] >= old[t]) continue;
+        if (bk.bound && x[t] < bk.bound[q] && !(bk.near[wq] & bit)) atomicOr(bk.near + wq, bit);
+      }
+      atomicOr(nw + v[t], bit);  // result unused: a reduction
+      ++changed;
+    }
+  }
+}
+
+// One round over the pairs of mask `cur`.  Every thread of a 256-thread block
+// calls it.
+template <int W, int KIND>
+__device__ __forceinline__ void batch_pairs_round(const BatchArgs &a, int round, unsigned *cur, unsigned *nxt,
+                                                  PairSmem &sm, unsigned long long &changed, const BatchBucket bk) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long words = (long long)a.nVertices * W;
+  const long long half = (long long)gridDim.x * 32 * (kPairWords / 2) * 8;
+  for (long long base = 0; base < words; base += 2 * half) {  // block-uniform
+    const bool both = words - base > half;
+    // warp k of the block takes groups blockIdx.x + grid * (k + 8 j)
+    unsigned m[kPairWords];
+    int n = 0;
+#pragma unroll
+    for (int j = 0; j < kPairWords; ++j) {
+      const long long i = base + 32 * ((long long)blockIdx.x + (long long)gridDim.x * (warp + 8 * j)) + lane;
+      m[j] = (j < kPairWords / 2 || both) && i < words ? __ldcg(cur + i) : 0u;
+      if (m[j]) cur[i] = 0u;
+      n += __popc(m[j]);
+    }
+    int incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(kFullMask, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane == 31) sm.warpTot[warp] = (unsigned)incl;
+    __syncthreads();
+    int first = incl - n, total = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (k < warp) first += (int)sm.warpTot[k];
+      total += (int)sm.warpTot[k];
+    }
+    for (int at = 0; at < total; at += kPairList) {  // block-uniform
+      int pos = first - at;
+      if (pos < kPairList && pos + n > 0) {
+#pragma unroll
+        for (int j = 0; j < kPairWords; ++j) {
+          if (j >= kPairWords / 2 && !both) break;
+          const uint32_t i =
+              (uint32_t)(base + 32 * ((long long)blockIdx.x + (long long)gridDim.x * (warp + 8 * j)) + lane);
+          unsigned rest = m[j];
+          while (rest) {
+            const int p = __ffs(rest) - 1;
+            rest &= rest - 1u;
+            if (pos >= 0 && pos < kPairList) sm.entry[pos] = (i << 5) | (uint32_t)p;  // V * Q < 2^31
+            ++pos;
+          }
+        }
+      }
+      __syncthreads();
+      const int here = min(total - at, kPairList);
+      for (int k = threadIdx.x; k < here; k += 256) {
+        const uint32_t e = sm.entry[k], i = e >> 5;
+        const int w = W == 1 ? 0 : (int)(i / (uint32_t)a.nVertices);
+        batch_pair<W, KIND>(a, (int)(i - (uint32_t)w * (uint32_t)a.nVertices), 32 * w + (int)(e & 31u), round, nxt,
+                            changed, bk);
+      }
+      __syncthreads();  // the list is rewritten
+    }
+    __syncthreads();  // warpTot is rewritten
+  }
 }
 
 // Appends each lane's entries out[k] with want[k] (k < K) to a pair list:
@@ -417,46 +567,23 @@ __device__ __forceinline__ void warp_append_pairs(const bool (&want)[K], const u
     if (want[k]) list[pos++] = out[k];
 }
 
-// Pair-frontier push (state query-major: value[q][v], mask and seen words
-// [w][v], so that the pairs of one query's wavefront, which relax
-// neighbouring vertices, touch neighbouring words): lane i takes entry i of
-// the current pair list (when
-// `valid`), a changed (u, q), and relaxes u's out-edges for q alone; a
-// destination whose value changes is appended as (v, q) the first time its
-// query bit is set this round.  Warp-uniform (lanes step through their
-// edges together, up to the warp's largest out-degree).
-template <int W, int KIND>
-__device__ __forceinline__ void batch_pair_unit(const BatchArgs &a, bool valid, uint32_t entry,
-                                                int round, unsigned *cur, unsigned *nxt, uint32_t *listNext,
-                                                unsigned long long *cntNext,
-                                                unsigned long long &changed,
-                                                const BatchBucket bk) {
+// Pair-list push (BFS): lane i takes entry i of the current list (when
+// `valid`), a changed (u, q), and marks u's out-neighbours for q; one seen for
+// the first time is appended as (v, q).  Warp-uniform (lanes step through
+// their edges together, up to the warp's largest out-degree).
+template <int W>
+__device__ __forceinline__ void batch_pair_unit(const BatchArgs &a, bool valid, uint32_t entry, int round,
+                                                uint32_t *listNext, unsigned long long *cntNext,
+                                                unsigned long long &changed) {
   constexpr int Q = 32 * W;
   constexpr int LOGQ = W == 1 ? 5 : W == 2 ? 6 : W == 4 ? 7 : 8;
   const int u = valid ? (int)(entry >> LOGQ) : 0;
   const int q = (int)(entry & (Q - 1));
   const unsigned bit = 1u << (q & 31);
   const int wq = q >> 5;
-  const size_t V = (size_t)a.nVertices;  // pair batches keep their state query-major
-  int eb = valid ? a.outOffsets[u] : 0;
-  int deg = valid ? a.outOffsets[u + 1] - eb : 0;
-  int du = 0;
-  bool keep = false;
-  if (KIND == kBatchSSSP && valid) {
-    // Every bit of this round's mask belongs to a pair of this round's
-    // list, and nothing else touches the mask this round: each pair clears
-    // its word (idempotent zeros), so the mask is clean when it next
-    // collects pairs, without a pass over all vertices.
-    cur[(size_t)wq * V + u] = 0u;
-    du = __ldcg(a.value + (size_t)q * V + u);
-    if (bk.bound && du >= bk.bound[q]) {  // not this bucket: keep (u, q) for later
-      const unsigned old = atomicOr(nxt + (size_t)wq * V + u, bit);
-      keep = !(old & bit);
-      changed += 1;
-      deg = 0;
-    }
-  }
-  if (KIND == kBatchSSSP && bk.bound) warp_append_pair(keep, entry, listNext, cntNext);
+  const size_t V = (size_t)a.nVertices;
+  const int eb = valid ? a.outOffsets[u] : 0;
+  const int deg = valid ? a.outOffsets[u + 1] - eb : 0;
   // four out-edges a step, their appends to the next list in one atomic per
   // warp (the list counter is one word every warp of the grid contends for)
   constexpr int J = 4;
@@ -471,28 +598,31 @@ __device__ __forceinline__ void batch_pair_unit(const BatchArgs &a, bool valid, 
       out[t] = 0u;
       if (j < deg) {
         const int v = __ldg(a.outDests + eb + j);
-        if (KIND == kBatchBFS) {
-          const unsigned old = atomicOr(a.seen + (size_t)wq * V + v, bit);
-          if (!(old & bit)) {
-            a.value[(size_t)q * V + v] = round + 1;
-            want[t] = true;
-          }
-        } else {
-          const int cand = du + __ldg(a.weightsOut + eb + j);
-          const int old = atomicMin(a.value + (size_t)q * V + v, cand);
-          if (cand < old) {
-            const unsigned o2 = atomicOr(nxt + (size_t)wq * V + v, bit);
-            want[t] = !(o2 & bit);
-            if (bk.bound && cand < bk.bound[q] && !(bk.near[wq] & bit)) atomicOr(bk.near + wq, bit);
-          }
-        }
-        if (want[t]) {
+        const unsigned old = atomicOr(a.seen + (size_t)wq * V + v, bit);
+        if (!(old & bit)) {
+          a.value[(size_t)q * V + v] = round + 1;
+          want[t] = true;
           changed += 1;
           out[t] = ((uint32_t)v << LOGQ) | (uint32_t)q;
         }
       }
     }
     warp_append_pairs<J>(want, out, listNext, cntNext);
+  }
+}
+
+// One round over the pair list of round `round`, dealt to warps block-first.
+template <int W>
+__device__ __forceinline__ void batch_pair_list(const BatchArgs &a, int round, long long nList,
+                                                unsigned long long *cntNext, unsigned long long &changed) {
+  const uint32_t *pc = a.pairs[round % 3];
+  uint32_t *pn = a.pairs[(round + 1) % 3];
+  const long long threads = (long long)gridDim.x * blockDim.x;
+  const long long gwl = (long long)(threadIdx.x / 32) * gridDim.x + blockIdx.x;
+  for (long long base = gwl * 32; base < nList; base += threads) {
+    const long long i = base + (threadIdx.x & 31);
+    const bool valid = i < nList;
+    batch_pair_unit<W>(a, valid, valid ? __ldcg(pc + i) : 0u, round, pn, cntNext, changed);
   }
 }
 
@@ -517,17 +647,18 @@ __device__ __forceinline__ void batch_compact(const BatchArgs &a, const unsigned
   }
 }
 
-// PAIRS: the instantiation for pair-frontier batches (a.pairMode set),
-// which holds only the pair rounds: its smaller register budget (at most 40
-// a thread) keeps more warps, and so more of the latency-bound atomics, in
-// flight.  The other instantiation serves vertex-mask batches, at most 64
-// registers a thread so that 4 CTAs fit an SM: its pull and push rounds are
+// PAIRS: the instantiation for pair-frontier batches (a.pairMode), which
+// holds only their rounds; from lists (BFS only) with at most 40 registers a
+// thread, as more warps keep more of the latency-bound atomics in flight.  The
+// others take at most 64, so that 4 CTAs fit an SM: pull and push rounds are
 // latency-bound too (256 R-MAT-21 SSSP queries: 118 ms at 4 CTAs/SM, 170 ms
-// at the 2 a 128-register build allows).
-template <int W, int KIND, bool PAIRS = false>
-__global__ void __launch_bounds__(256, PAIRS ? 6 : 4) batch_run_kernel(const BatchArgs a) {
+// at the 2 a 128-register build allows, before pull units kept more loads in
+// flight).
+template <int W, int KIND, int PAIRS = kPairsOff>
+__global__ void __launch_bounds__(256, PAIRS == kPairsList ? 6 : 4) batch_run_kernel(const BatchArgs a) {
   __shared__ int32_t sBound[32 * W];
   __shared__ unsigned sNear[W];
+  __shared__ typename std::conditional<PAIRS == kPairsMask, PairSmem, char>::type sPairs;
   const long long warps = (long long)gridDim.x * (blockDim.x / 32);
   const long long gw = (long long)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
   // list entries are dealt to warps block-first (warp k of every block, then
@@ -572,21 +703,15 @@ __global__ void __launch_bounds__(256, PAIRS ? 6 : 4) batch_run_kernel(const Bat
       a.cnt[rn] = 0ull;
       a.listCnt[(r + 2) % 3] = 0ull;  // input of round r-1, appended in round r+1
     }
-    if (!PAIRS)  // pair rounds clear their own mask words (batch_pair_unit)
+    if (!PAIRS)  // pair rounds from the mask clear the words they read
       for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < maskWords;
            i += (size_t)gridDim.x * blockDim.x)
         clr[i] = 0u;
     unsigned long long changed = 0ull;
-    if constexpr (PAIRS) {
-      const uint32_t *pc = a.pairs[rc];
-      uint32_t *pn = a.pairs[rn];
-      const long long threads = (long long)gridDim.x * blockDim.x;
-      for (long long base = gwl * 32; base < nList; base += threads) {
-        const long long i = base + (threadIdx.x & 31);
-        const bool valid = i < nList;
-        batch_pair_unit<W, KIND>(a, valid, valid ? __ldcg(pc + i) : 0u, r, cur, nxt,
-                                 pn, cntNext, changed, bk);
-      }
+    if constexpr (PAIRS == kPairsMask) {
+      batch_pairs_round<W, KIND>(a, r, cur, nxt, sPairs, changed, bk);
+    } else if constexpr (PAIRS == kPairsList) {
+      batch_pair_list<W>(a, r, nList, cntNext, changed);
     } else if (push) {
       for (long long i = gwl; i < nList; i += warps)
         batch_push_unit<W, KIND>(a, listCur[i], listCurC[i], r, cur, nxt, listNext, listNextC,
@@ -629,32 +754,31 @@ static __global__ void batch_init_kernel(int kind, int32_t nVertices, int32_t Q,
 
 // Sources: value 0, their query bit, and the first list (each source
 // vertex once; inList was reset to -1).
-// With a pair list (pairs0 non-null) the first list is (s_q, q) per query,
-// and the state is query-major (value[q][v], mask and seen words [w][v]).
+// Pair batches keep their state query-major (value[q][v], mask and seen words
+// [w][v]); the first pair list is (s_q, q) per query.
 static __global__ void batch_sources_kernel(int kind, int32_t nQueries, int32_t Q, int32_t W,
                                             int32_t nVertices, const int32_t *sources, int32_t *value,
                                             unsigned *mask0, unsigned *seen,
                                             const int32_t *outOffsets, int32_t *inList,
                                             int32_t *list0, int32_t *list0C,
-                                            unsigned long long *listCnt0,
+                                            unsigned long long *listCnt0, int pairMode = kPairsOff,
                                             uint32_t *pairs0 = nullptr) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= nQueries) return;
   const int s = sources[q];
-  if (pairs0) {  // pair batches keep their state query-major
+  if (pairMode != kPairsOff) {
     value[(size_t)q * nVertices + s] = 0;
     atomicOr(mask0 + (size_t)(q / 32) * nVertices + s, 1u << (q % 32));
     if (kind == kBatchBFS) atomicOr(seen + (size_t)(q / 32) * nVertices + s, 1u << (q % 32));
-  } else {
-    value[(size_t)s * Q + q] = 0;
-    atomicOr(mask0 + (size_t)s * W + q / 32, 1u << (q % 32));
-    if (kind == kBatchBFS) atomicOr(seen + (size_t)s * W + q / 32, 1u << (q % 32));
-  }
-  if (pairs0) {
-    const unsigned long long pos = atomicAdd(listCnt0, 1ull << 32) >> 32;
-    pairs0[pos] = (uint32_t)s * (uint32_t)Q + (uint32_t)q;
+    if (pairMode == kPairsList) {
+      const unsigned long long pos = atomicAdd(listCnt0, 1ull << 32) >> 32;
+      pairs0[pos] = (uint32_t)s * (uint32_t)Q + (uint32_t)q;
+    }
     return;
   }
+  value[(size_t)s * Q + q] = 0;
+  atomicOr(mask0 + (size_t)s * W + q / 32, 1u << (q % 32));
+  if (kind == kBatchBFS) atomicOr(seen + (size_t)s * W + q / 32, 1u << (q % 32));
   if (atomicExch(inList + s, 0) != 0) {
     const unsigned d = (unsigned)(outOffsets[s + 1] - outOffsets[s]);
     const unsigned ne = d > 0u ? (d + kPushChunk - 1) / kPushChunk : 1u;

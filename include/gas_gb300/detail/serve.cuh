@@ -42,6 +42,7 @@ __global__ void __launch_bounds__(256) batch_round_kernel(const BatchArgs a, int
   if (ld_acquire(done)) return;
   __shared__ int32_t sBound[32 * W];
   __shared__ unsigned sNear[W];
+  __shared__ PairSmem sPairs;
   const long long warps = (long long)gridDim.x * (blockDim.x / 32);
   const long long gw = (long long)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
   // list entries are dealt to warps block-first (warp k of every block, then
@@ -76,21 +77,16 @@ __global__ void __launch_bounds__(256) batch_round_kernel(const BatchArgs a, int
     a.cnt[rn] = 0ull;
     a.listCnt[(r + 2) % 3] = 0ull;
   }
-  if (!a.pairMode)  // pair rounds clear their own mask words (batch_pair_unit)
+  if (!a.pairMode)  // pair rounds from the mask clear the words they read
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < maskWords;
          i += (size_t)gridDim.x * blockDim.x)
       clr[i] = 0u;
   unsigned long long changed = 0ull;
   if (a.pairMode) {
-    const uint32_t *pc = a.pairs[rc];
-    uint32_t *pn = a.pairs[rn];
-    const long long threads = (long long)gridDim.x * blockDim.x;
-    for (long long base = gwl * 32; base < nList; base += threads) {
-      const long long i = base + (threadIdx.x & 31);
-      const bool valid = i < nList;
-      batch_pair_unit<W, KIND>(a, valid, valid ? __ldcg(pc + i) : 0u, r, cur, nxt,
-                               pn, a.listCnt + rn, changed, bk);
-    }
+    if (KIND == kBatchSSSP || a.pairMode == kPairsMask)
+      batch_pairs_round<W, KIND>(a, r, cur, nxt, sPairs, changed, bk);
+    else
+      batch_pair_list<W>(a, r, nList, a.listCnt + rn, changed);
   } else if (push) {
     for (long long i = gwl; i < nList; i += warps)
       batch_push_unit<W, KIND>(a, a.list[rc][i], a.listC[rc][i], r, cur, nxt, a.list[rn],

@@ -50,7 +50,7 @@ struct gas_batch_s {
   int32_t delta = 0;   // SSSP bucket width (0 = Bellman-Ford rounds)
   int32_t frontier = -1;  // -1 automatic, 0 vertex masks, 1 (vertex, query) pairs
   int32_t maxOutDeg = 0;
-  uint32_t *pairs[3] = {nullptr, nullptr, nullptr};
+  uint32_t *pairs[3] = {nullptr, nullptr, nullptr};  // pair lists (BFS over large masks only)
   size_t pairCap = 0;
   int32_t *bucketMem = nullptr;  // thresh[2][256] | nearFlag[3][8]
   int32_t unitChunk = 0;
@@ -129,9 +129,9 @@ void free_state(gas_batch *b) {
 
 // Pair frontier for graphs whose out-degrees are small (a lane walks a
 // vertex's out-edges alone) and whose V * Q entries fit 32 bits.
-bool use_pairs(const gas_batch *b, const CoreGraph &g, int32_t Q) {
-  const bool allowed = b->maxOutDeg <= 64 && (long long)g.nV * Q < (1ll << 31);
-  return b->frontier == 0 ? false : allowed;
+int pair_mode(const gas_batch *b, const CoreGraph &g, int kind, int32_t Q) {
+  if (b->frontier == 0 || b->maxOutDeg > 64 || (long long)g.nV * Q >= (1ll << 31)) return gas::detail::kPairsOff;
+  return gas::detail::pair_mode_of(kind == gas::detail::kBatchBFS, g.nV, Q / 32);
 }
 
 gas_status ensure_pairs(gas_batch *b, const CoreGraph &g, int32_t Q) {
@@ -213,7 +213,15 @@ gas_status ensure_state(gas_batch *b, const CoreGraph &g, int32_t Q) {
 }
 
 template <int W, int KIND>
-gas_status launch_run(gas_batch *b, const CoreGraph &g, int32_t Q, int blocks, bool pairs) {
+const void *run_fn(int pairs) {
+  using namespace gas::detail;
+  return pairs == kPairsMask   ? (const void *)batch_run_kernel<W, KIND, kPairsMask>
+         : pairs == kPairsList ? (const void *)batch_run_kernel<W, kBatchBFS, kPairsList>
+                               : (const void *)batch_run_kernel<W, KIND, kPairsOff>;
+}
+
+template <int W, int KIND>
+gas_status launch_run(gas_batch *b, const CoreGraph &g, int32_t Q, int blocks, int pairs) {
   gas::detail::BatchArgs a;
   memset(&a, 0, sizeof(a));
   a.nVertices = g.nV;
@@ -249,44 +257,40 @@ gas_status launch_run(gas_batch *b, const CoreGraph &g, int32_t Q, int blocks, b
   a.thresh[1] = b->bucketMem + kMaxBatch;
   for (int k = 0; k < 3; ++k)
     a.nearFlag[k] = reinterpret_cast<unsigned *>(b->bucketMem + 2 * kMaxBatch + 8 * k);
-  a.pairMode = pairs ? 1 : 0;
-  for (int k = 0; k < 3; ++k) a.pairs[k] = pairs ? b->pairs[k] : nullptr;
+  a.pairMode = pairs;
+  for (int k = 0; k < 3; ++k) a.pairs[k] = b->pairs[k];
   void *args[] = {&a};
-  const void *fn = pairs ? (const void *)gas::detail::batch_run_kernel<W, KIND, true>
-                         : (const void *)gas::detail::batch_run_kernel<W, KIND, false>;
+  const void *fn = run_fn<W, KIND>(pairs);
   cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(256), args, 0, b->stream);
   return e == cudaSuccess ? GAS_OK : cuda_fail(e, "batch run launch");
 }
 
 template <int W>
 gas_status launch_run_kind(gas_batch *b, const CoreGraph &g, int kind, int32_t Q, int blocks,
-                           bool pairs) {
+                           int pairs) {
   return kind == gas::detail::kBatchBFS
              ? launch_run<W, gas::detail::kBatchBFS>(b, g, Q, blocks, pairs)
              : launch_run<W, gas::detail::kBatchSSSP>(b, g, Q, blocks, pairs);
 }
 
-int grid_blocks(gas_batch *b, int kind, int W, bool pairs) {
+int grid_blocks(gas_batch *b, const CoreGraph &g, int kind, int nQ, int W, int pairs) {
   int per = 0;
   const void *fn = nullptr;
-#define GAS_BATCH_FN(w)                                                                       \
-  if (W == w)                                                                                 \
-    fn = kind == gas::detail::kBatchBFS                                                       \
-             ? (pairs ? (const void *)gas::detail::batch_run_kernel<w, gas::detail::kBatchBFS, true> \
-                      : (const void *)gas::detail::batch_run_kernel<w, gas::detail::kBatchBFS, false>) \
-             : (pairs ? (const void *)gas::detail::batch_run_kernel<w, gas::detail::kBatchSSSP, true> \
-                      : (const void *)gas::detail::batch_run_kernel<w, gas::detail::kBatchSSSP, false>);
+#define GAS_BATCH_FN(w) \
+  if (W == w) fn = kind == gas::detail::kBatchBFS ? run_fn<w, gas::detail::kBatchBFS>(pairs) : run_fn<w, gas::detail::kBatchSSSP>(pairs);
   GAS_BATCH_FN(1) GAS_BATCH_FN(2) GAS_BATCH_FN(4) GAS_BATCH_FN(8)
 #undef GAS_BATCH_FN
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, 256, 0);
   if (b->blocksPerSM > 0 && b->blocksPerSM < per) per = b->blocksPerSM;
-  return std::max(per, 1) * std::max(b->sms, 1);
+  const int most = std::max(per, 1) * std::max(b->sms, 1);
+  if (pairs != gas::detail::kPairsMask || b->blocksPerSM > 0) return most;
+  return std::min(most, gas::detail::batch_pair_blocks(g.nV, W, nQ, b->sms));
 }
 
 // The whole batch on b->stream: sources (from pinned staging), state reset,
 // initial values, the persistent run, query-major results in outDev.
 gas_status enqueue_batch(gas_batch *b, const CoreGraph &g, int kind, int32_t nQ, int32_t Q,
-                         bool pairs) {
+                         int pairs) {
   const int W = Q / 32;
   const size_t V = (size_t)g.nV;
   cudaError_t e = cudaMemcpyAsync(b->srcDev, b->srcPinned, sizeof(int32_t) * nQ,
@@ -304,10 +308,10 @@ gas_status enqueue_batch(gas_batch *b, const CoreGraph &g, int kind, int32_t nQ,
   CtlView cv = ctl_view(b);
   gas::detail::batch_sources_kernel<<<(nQ + 127) / 128, 128, 0, b->stream>>>(
       kind, nQ, Q, W, g.nV, b->srcDev, b->value, b->mask[0], b->seen, g.outOff, b->inList,
-      b->list[0], b->listC[0], cv.listCnt, pairs ? b->pairs[0] : nullptr);
+      b->list[0], b->listC[0], cv.listCnt, pairs, b->pairs[0]);
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "batch init");
-  const int blocks = grid_blocks(b, kind, W, pairs);
+  const int blocks = grid_blocks(b, g, kind, nQ, W, pairs);
   gas_status st;
   switch (W) {
     case 1: st = launch_run_kind<1>(b, g, kind, Q, blocks, pairs); break;
@@ -502,8 +506,8 @@ gas_status run_one(gas_batch *b, const CoreGraph &g, int kind, int32_t nQ, const
   while (Q < nQ) Q *= 2;
   gas_status st = ensure_state(b, g, std::max(Q, 32));
   if (st) return st;
-  const bool pairs = use_pairs(b, g, Q);
-  if (pairs) {
+  const int pairs = pair_mode(b, g, kind, Q);
+  if (pairs == gas::detail::kPairsList) {
     st = ensure_pairs(b, g, Q);
     if (st) return st;
   }
@@ -513,7 +517,7 @@ gas_status run_one(gas_batch *b, const CoreGraph &g, int kind, int32_t nQ, const
     cudaGraphExec_t exec = nullptr;
     for (auto &c : b->graphs)
       if (c.kind == kind && c.W == Q / 32 && c.nQ == nQ && c.blocksPerSM == b->blocksPerSM &&
-          c.chunk == b->unitChunk && c.delta == b->delta && c.pairs == (int)pairs)
+          c.chunk == b->unitChunk && c.delta == b->delta && c.pairs == pairs)
         exec = c.exec;
     if (!exec) {
       cudaGraph_t graph = nullptr;
@@ -523,7 +527,7 @@ gas_status run_one(gas_batch *b, const CoreGraph &g, int kind, int32_t nQ, const
         if (cst == GAS_OK && ce == cudaSuccess && graph &&
             cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess) {
           b->graphs.push_back(
-              {kind, Q / 32, nQ, b->blocksPerSM, b->unitChunk, b->delta, (int)pairs, exec});
+              {kind, Q / 32, nQ, b->blocksPerSM, b->unitChunk, b->delta, pairs, exec});
         } else {
           exec = nullptr;
           b->useGraphs = false;  // this runtime cannot capture the batch: launch directly
@@ -795,7 +799,8 @@ gas_status gas_batch_autotune(gas_batch *b, int32_t program, int32_t nQueries,
     }
     int32_t Q = 32;
     while (Q < nq) Q *= 2;
-    if (!use_pairs(b, g, Q)) {
+    if (pair_mode(b, g, program == GAS_PROGRAM_BFS ? gas::detail::kBatchBFS : gas::detail::kBatchSSSP, Q) ==
+        gas::detail::kPairsOff) {
       const int32_t alphas[] = {2, 10, 50};
       st = tune(alphas, 3, gas_batch_set_policy, b->alpha);
       if (st) return st;

@@ -123,9 +123,9 @@ struct Batch {
   Ctl *ctl = nullptr;              // inside `state`
   gas::detail::BatchArgs ba;
   gas::detail::PprArgs pa;
-  bool pairs = false;             // (vertex, query) pair frontier
-  bool persistent = false;        // every round in one cooperative launch
+  int pairs = gas::detail::kPairsOff;  // (vertex, query) pair frontier
   int64_t pairsSeen = 0;          // largest pair list seen at a chunk's end
+  bool persistent = false;        // every round in one cooperative launch
   int32_t delta = 0;              // SSSP distance buckets
   int roundsIssued = 0;
   int chunk = kFirstChunk;
@@ -210,8 +210,10 @@ int row_width(int kind, int n) {
 
 // (vertex, query) pair frontier for graphs of small out-degree whose V * Q
 // pair ids fit 32 bits (as gas_batch chooses it)
-bool use_pairs(const ServeGraph &g, int kind, int Q) {
-  return kind != 2 && g.maxOutDeg <= 64 && (long long)std::max(g.bg.g.nV, 1) * Q < (1ll << 31);
+int pair_mode(const ServeGraph &g, int kind, int Q) {
+  const long long V = std::max(g.bg.g.nV, 1);
+  if (kind == 2 || g.maxOutDeg > 64 || V * Q >= (1ll << 31)) return gas::detail::kPairsOff;
+  return gas::detail::pair_mode_of(kind == 0, V, Q / 32);
 }
 
 int64_t Server::state_bytes(const ServeGraph &g, int kind, int Q) const {
@@ -220,7 +222,7 @@ int64_t Server::state_bytes(const ServeGraph &g, int kind, int Q) const {
   // each rounded up to 256 bytes
   const int64_t base = 256 + 4 * kMaxQ + 4 * (2 * kMaxQ + 24) + 24 * 256;
   const int64_t lists = 24 * gas::detail::batch_list_capacity(V, g.bg.g.nE) + 4 * V +
-                        (use_pairs(g, kind, Q) ? 12 * V * Q : 0);
+                        (pair_mode(g, kind, Q) == gas::detail::kPairsList ? 12 * V * Q : 0);
   if (kind == 0) return base + V * Q * 4 + 16 * V * W + lists;
   if (kind == 1) return base + V * Q * 4 + 12 * V * W + lists;
   return base + V * Q * 16 + (int64_t)g.ppr.slots * Q * 4 +
@@ -346,11 +348,14 @@ void ppr_round_launch(const gas::detail::PprArgs &a, int r, int blocks, cudaStre
 
 // The batch engine's persistent kernel for a pair-frontier batch of a row
 // width and program.
-const void *batch_run_fn(int W, bool bfs) {
-#define GAS_RUN_W(w)                                                                             \
-  case w:                                                                                        \
-    return bfs ? (const void *)gas::detail::batch_run_kernel<w, gas::detail::kBatchBFS, true>    \
-               : (const void *)gas::detail::batch_run_kernel<w, gas::detail::kBatchSSSP, true>;
+const void *batch_run_fn(int W, bool bfs, int pairs) {
+  using namespace gas::detail;
+#define GAS_RUN_W(w)                                                                                   \
+  case w:                                                                                              \
+    if (pairs == kPairsMask)                                                                           \
+      return bfs ? (const void *)batch_run_kernel<w, kBatchBFS, kPairsMask>                            \
+                 : (const void *)batch_run_kernel<w, kBatchSSSP, kPairsMask>;                          \
+    return (const void *)batch_run_kernel<w, kBatchBFS, kPairsList>;
   switch (W) {
     GAS_RUN_W(1)
     GAS_RUN_W(2)
@@ -416,8 +421,10 @@ void Server::issue_chunk(int l, int rounds, bool final) {
     b.roundsIssued += rounds;
     launches += rounds;
   } else {
-    int blocks = round_blocks(*this, std::max<int64_t>(b.g->bg.nUnits, V));
-    if (b.pairs) {
+    // pair rounds from the mask: a warp for each 128 of its words
+    int blocks = round_blocks(*this, b.pairs == gas::detail::kPairsMask ? (int64_t)V * b.W / 128 + 1
+                                                                        : std::max<int64_t>(b.g->bg.nUnits, V));
+    if (b.pairs == gas::detail::kPairsList) {
       // pair rounds walk the pair list only: a grid for about twice the
       // largest list seen so far (the rounds grid-stride past it), so that
       // a small batch's rounds need few block slots on a busy device
@@ -520,9 +527,9 @@ gas_status Server::launch(int l, const std::shared_ptr<Batch> &bp) {
     }
     a.inList = reinterpret_cast<int32_t *>(take(Vs * 4));
     a.seen = b.kind == 0 ? reinterpret_cast<unsigned *>(take(Vs * W * 4)) : nullptr;
-    a.pairMode = b.pairs ? 1 : 0;
+    a.pairMode = b.pairs;
     for (int k = 0; k < 3; ++k)
-      a.pairs[k] = b.pairs ? reinterpret_cast<uint32_t *>(take(Vs * b.Q * 4)) : nullptr;
+      a.pairs[k] = b.pairs == gas::detail::kPairsList ? reinterpret_cast<uint32_t *>(take(Vs * b.Q * 4)) : nullptr;
     a.delta = b.kind == 1 ? b.delta : 0;
     for (int k = 0; k < 2; ++k) a.thresh[k] = reinterpret_cast<int32_t *>(take(4 * kMaxQ));
     for (int k = 0; k < 3; ++k) a.nearFlag[k] = reinterpret_cast<unsigned *>(take(4 * 8));
@@ -542,7 +549,7 @@ gas_status Server::launch(int l, const std::shared_ptr<Batch> &bp) {
                                                                     a.thresh[0], a.delta);
     gas::detail::batch_sources_kernel<<<(b.nQ + 127) / 128, 128, 0, b.stream>>>(
         kb, b.nQ, b.Q, b.W, V, b.sources, a.value, a.mask[0], a.seen, g.bg.g.outOff, a.inList,
-        a.list[0], a.listC[0], a.listCnt, b.pairs ? a.pairs[0] : nullptr);
+        a.list[0], a.listC[0], a.listCnt, b.pairs, a.pairs[0]);
   }
   launches += 2;  // init + sources
   e = cudaGetLastError();
@@ -557,10 +564,12 @@ gas_status Server::launch(int l, const std::shared_ptr<Batch> &bp) {
     // their grids fit the device together; the other lanes' kernels are
     // ordinary and finite, so a partly placed grid waits for their blocks
     // to finish, and every grid-barrier wait in it is bounded.
-    const void *fn = batch_run_fn(b.W, b.kind == 0);
+    const void *fn = batch_run_fn(b.W, b.kind == 0, b.pairs);
     int per = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, 256, 0);
-    const int blocks = std::max(1, per * sms / 3);
+    int blocks = std::max(1, per * sms / 3);
+    if (b.pairs == gas::detail::kPairsMask)
+      blocks = std::min(blocks, gas::detail::batch_pair_blocks(V, b.W, b.nQ, sms));
     void *args[] = {&b.ba};
     e = cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(256), args, 0, b.stream);
     if (e == cudaSuccess) {
@@ -742,7 +751,7 @@ bool Server::admit() {
       bp->nQ = nQ;
       bp->Q = row_width(kind, nQ);
       bp->W = std::max(bp->Q / 32, 1);
-      bp->pairs = use_pairs(*g, kind, bp->Q);
+      bp->pairs = pair_mode(*g, kind, bp->Q);
       // distance buckets for SSSP on pair-frontier (high-diameter) graphs
       bp->delta = (kind == 1 && bp->pairs) ? 4 * std::max(g->maxWeight, 1) : 0;
       bp->stateBytes = state_bytes(*g, kind, bp->Q);
