@@ -208,18 +208,29 @@ __device__ __forceinline__ void group_edges(const DenseCtx &a, int v, int beg, i
     const int e = tBeg + sl - 4;
     edge_acc<P>(a, v, __ldg(a.inSources + e), edge_ptr<P>(a.edgeData, e), known, x);
   }
+  // without a gather the vertex needs no further edge once it is known active
   if constexpr (W == 32) {
     known = known || __any_sync(kFullMask, x.act != 0u);
-    for (int q0 = qb; q0 < qe; q0 += 32) {
+    for (int q0 = qb; q0 < qe && (a.haveGather || !known); q0 += 32) {
       if (q0 + sl < qe) quad_acc<P>(a, v, q0 + sl, known, x);
       known = known || __any_sync(kFullMask, x.act != 0u);
     }
   } else {
     static_assert(W * 8 >= 64, "a group walks at most 64 edges in two steps");
 #pragma unroll
-    for (int k = 0; k < 2; ++k)
+    for (int k = 0; k < 2; ++k) {
+      if (!a.haveGather) {  // uniform
+        const unsigned act = __ballot_sync(kFullMask, x.act != 0u);
+        known = known || ((act >> ((threadIdx.x & 31) / W * W)) & ((1u << W) - 1u)) != 0u;
+        if (known) {
+          x.act = 1u;
+          continue;
+        }
+      }
       if (qb + sl + W * k < qe) quad_acc<P>(a, v, qb + sl + W * k, known, x);
+    }
   }
+  if (known) x.act = 1u;
 }
 
 struct DenseCounts {
@@ -371,7 +382,7 @@ __device__ void dense_warp_unit(const DenseCtx &a, long long u, DenseCounts &c) 
     unsigned act = 0u;
 #pragma unroll
     for (int k = 0; k < GAS_TPV_MAX_DEGREE; ++k)
-      if (beg + k < end) {
+      if (beg + k < end && (a.haveGather || !act)) {
         act |= (a.skipBits || bit_test(a.prevBits, src[k])) ? 1u : 0u;
         if (a.haveGather)
           g = P::gatherReduce(g, P::gatherMap(vd + v, vd + src[k], edge_ptr<P>(a.edgeData, beg + k)));
