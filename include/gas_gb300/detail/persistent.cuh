@@ -604,15 +604,22 @@ __global__ void __launch_bounds__(kGNT, MinBlocks) run_persistent_kernel(const g
       compact_active<kGNT, kGVT>(front_bits(ra, ra.stampBase + r), a.inOffsets, a.nVertices,
                                  ra.frontL[cur], ra.maxGatherTiles, a.capacity, a.errWord, sm.g.app);
   }
-  if (versioned) {  // the newest values into the run's current buffer
+  // The result goes into the vertex data array here, not in a copy that the
+  // host would have to wait for (the last round ended with a grid barrier:
+  // nobody reads that array any more).
+  if (versioned) {
     FusedCtx f;
     f.cells = ra.fusedCells;
-    f.vd = vdBuf[vcur];
+    f.vd = vdBuf[0];
     fused_fold<P>(f, a.nVertices);
+  } else if (vcur == 1) {
+    typedef typename P::VertexData VD;
+    const VD *from = reinterpret_cast<const VD *>(vdBuf[1]);
+    VD *to = reinterpret_cast<VD *>(vdBuf[0]);
+    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < a.nVertices; v += gridDim.x * blockDim.x) to[v] = from[v];
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     *ra.roundsOut = r;
-    if (ra.vcurOut) *ra.vcurOut = vcur;
     if (ra.denseEndOut) *ra.denseEndOut = denseEnd ? 1 : 0;
   }
 }

@@ -143,7 +143,6 @@ typedef struct {
                                  ret/out-edges, dense work units taken, unused */
   int32_t denseAlpha;         /* next round dense when out-edges*alpha > E; 0 = never */
   int32_t allActive;          /* round 0 is every vertex (setActive(0, V)) */
-  int32_t *vcurOut;           /* 1 when the final vertex data is in vertexAlt */
   /* degree bins of the dense pass (fixed per graph): warp work units are
    * [large-vertex chunks | warp-per-vertex | 8-lane groups | thread-per-vertex] */
   const int32_t *binMid;      /* in-degree 65..1024: one warp each          */

@@ -86,19 +86,25 @@ struct ListCtl {
   unsigned pad;
 };
 
+// What the host reads back after a run comes first, in one copy.
 struct Ctl {
-  ListCtl f[2];  // frontier lists
-  ListCtl s[2];  // scatter lists
+  unsigned err;     // device error bits (kept across set_active)
+  int32_t rounds;   // rounds executed by the last persistent run
+  int32_t denseEnd; // 1 when that run stopped before a dense round (gas_run_args::denseEndOut)
+  int32_t pad;
+  ListCtl f[2];     // frontier lists
+  ListCtl s[2];     // scatter lists
   unsigned tile[2];
   unsigned bar[2];  // persistent-kernel grid barrier: arrival word, unused
-  int32_t rounds;   // rounds executed by the last persistent run
-  int32_t vcur;     // 1 when that run's result is in the alternate buffer
-  int32_t denseEnd; // 1 when that run stopped before a dense round (gas_run_args::denseEndOut)
-  int32_t pad0;
   unsigned long long dense[3][4];  // per-round counters of dense rounds (kDenseCntStride)
-  unsigned err;     // device error bits (kept across set_active)
-  unsigned pad;
   int32_t resume[4];  // hand-over of a leading dense-rounds kernel (gas_run_args::resume)
+};
+
+// The part of Ctl that the host reads, as it lies there.
+struct CtlHead {
+  unsigned err;
+  int32_t rounds, denseEnd, pad;
+  ListCtl f[2];
 };
 
 enum DirtyBit : unsigned {
@@ -141,7 +147,7 @@ __global__ void ell_rows_kernel(int32_t nV, const int32_t *off, const int32_t *i
 // The counters, barrier words and round-0 bitmaps a persistent run starts
 // from, zeroed by one launch instead of one memset each.
 struct ZeroSegments {
-  static constexpr int kMax = 8;
+  static constexpr int kMax = 9;
   uint32_t *ptr[kMax];
   int32_t words[kMax];
   int32_t n;
@@ -246,6 +252,7 @@ struct gas_core_s {
   int32_t round = 0;
   // run bookkeeping
   unsigned long long *pinned = nullptr;
+  CtlHead *head = nullptr;          // page-locked: control words read back
   cudaEvent_t ev[kRing] = {};
   cudaEvent_t t0 = nullptr, t1 = nullptr;
   float lastMs = 0.f;
@@ -475,19 +482,28 @@ gas_status materialize(gas_core *c) {
   return GAS_OK;
 }
 
+// Queues the copy of the control words the host reads (c->head, valid after
+// a synchronisation).
+cudaError_t fetch_head(gas_core *c) {
+  static_assert(offsetof(CtlHead, f) == offsetof(Ctl, f), "CtlHead is Ctl's first part");
+  return cudaMemcpyAsync(c->head, c->ctl, sizeof(CtlHead), cudaMemcpyDeviceToHost, c->stream);
+}
+
+// The device error bits of a fetched head.
+gas_status head_error(gas_core *c) {
+  const unsigned err = c->head->err;
+  if (!err) return GAS_OK;
+  cudaMemsetAsync(&c->ctl->err, 0, sizeof(unsigned), c->stream);
+  if (err & GAS_DEVERR_TIMEOUT)
+    return fail(GAS_ERR_TIMEOUT, "a bounded device wait (tile look-back) timed out");
+  return fail(GAS_ERR_STATE, "device list capacity exceeded (error bits 0x%x)", err);
+}
+
 gas_status check_device_error(gas_core *c) {
-  unsigned err = 0;
-  cudaError_t e = cudaMemcpyAsync(&err, &c->ctl->err, sizeof(err), cudaMemcpyDeviceToHost,
-                                  c->stream);
+  cudaError_t e = fetch_head(c);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return cuda_fail(e, "device sync");
-  if (err) {
-    cudaMemsetAsync(&c->ctl->err, 0, sizeof(unsigned), c->stream);
-    if (err & GAS_DEVERR_TIMEOUT)
-      return fail(GAS_ERR_TIMEOUT, "a bounded device wait (tile look-back) timed out");
-    return fail(GAS_ERR_STATE, "device list capacity exceeded (error bits 0x%x)", err);
-  }
-  return GAS_OK;
+  return head_error(c);
 }
 
 }  // namespace
@@ -570,11 +586,13 @@ gas_status gas_core_create(int32_t device, void *stream, gas_core **out) {
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, gas::detail::scatter_activate_kernel,
                                                 gas::detail::kSNT, 0);
   c->scatterGrid = std::max(1, per) * std::max(1, c->numSMs);
-  e = cudaMallocHost((void **)&c->pinned, sizeof(unsigned long long) * kRing);
+  // one page-locked block: the round counts' ring, the control words
+  e = cudaMallocHost((void **)&c->pinned, sizeof(unsigned long long) * kRing + sizeof(CtlHead));
   if (e != cudaSuccess) {
     delete c;
     return cuda_fail(e, "cudaMallocHost");
   }
+  c->head = reinterpret_cast<CtlHead *>(c->pinned + kRing);
   for (int k = 0; k < kRing; ++k) cudaEventCreateWithFlags(&c->ev[k], cudaEventDisableTiming);
   cudaEventCreate(&c->t0);
   cudaEventCreate(&c->t1);
@@ -838,13 +856,13 @@ gas_status gas_core_upload_vertex_data(gas_core *c, const void *host) {
 gas_status gas_core_download_vertex_data(gas_core *c, void *host) {
   if (!c || !host) return fail(GAS_ERR_INVALID, "download_vertex_data: null argument");
   if (!c->haveGraph) return fail(GAS_ERR_STATE, "no graph set");
-  gas_status st = check_device_error(c);
-  if (st) return st;
-  if (c->nV == 0) return GAS_OK;
-  cudaError_t e = cudaMemcpyAsync(host, c->vd, (size_t)c->vertexBytes * c->nV,
-                                  cudaMemcpyDeviceToHost, c->stream);
+  // the error bits of the work before the copy come back with it; the data
+  // is the caller's only if there are none
+  cudaError_t e = fetch_head(c);
+  if (e == cudaSuccess && c->nV > 0)
+    e = cudaMemcpyAsync(host, c->vd, (size_t)c->vertexBytes * c->nV, cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  return e == cudaSuccess ? GAS_OK : cuda_fail(e, "vertex data download");
+  return e == cudaSuccess ? head_error(c) : cuda_fail(e, "vertex data download");
 }
 
 gas_status gas_core_download_edge_data(gas_core *c, void *host) {
@@ -879,7 +897,7 @@ gas_status gas_core_set_active(gas_core *c, int32_t start, int32_t end) {
     return fail(GAS_ERR_INVALID, "active range [%d, %d) outside [0, %d]", start, end, c->nV);
   gas_status st = set_device(c);
   if (st) return st;
-  cudaError_t e = cudaMemsetAsync(c->ctl, 0, offsetof(Ctl, err), c->stream);  // keep err
+  cudaError_t e = cudaMemsetAsync(&c->ctl->rounds, 0, sizeof(Ctl) - offsetof(Ctl, rounds), c->stream);  // keep err
   if (e != cudaSuccess) return cuda_fail(e, "set_active reset");
   c->dirty = 0;
   c->densePending = false;
@@ -920,14 +938,9 @@ gas_status gas_core_count_active(gas_core *c, int32_t *n) {
     *n = c->countCache;
     return GAS_OK;
   }
-  gas_status st = check_device_error(c);
+  gas_status st = check_device_error(c);  // brings the counts too
   if (st) return st;
-  unsigned long long v = 0;
-  cudaError_t e = cudaMemcpyAsync(&v, &c->ctl->f[c->cur].cnt, 8, cudaMemcpyDeviceToHost,
-                                  c->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  if (e != cudaSuccess) return cuda_fail(e, "count_active");
-  *n = (int32_t)std::min<unsigned long long>(v >> 32, (unsigned long long)c->nV);
+  *n = (int32_t)std::min<unsigned long long>(c->head->f[c->cur].cnt >> 32, (unsigned long long)c->nV);
   c->countCache = *n;
   c->countValid = true;
   return GAS_OK;
@@ -1229,7 +1242,8 @@ gas_status gas_core_run_persistent(gas_core *c, int32_t maxIters, int32_t haveGa
     seg(c->chunkArrive, sizeof(unsigned) * std::max(c->nChunkVertices, 1));
     seg(&c->ctl->s[0], sizeof(c->ctl->s));
     seg(&c->ctl->f[c->cur ^ 1], sizeof(ListCtl));
-    seg(&c->ctl->bar[0], sizeof(c->ctl->bar) + sizeof(int32_t));
+    seg(&c->ctl->bar[0], sizeof(c->ctl->bar));
+    seg(&c->ctl->rounds, 2 * sizeof(int32_t));
     seg(round_bits(c, ra.stampBase), sizeof(uint32_t) * std::max(c->bitWords, 1));
     if (c->frontBits)
       seg(c->frontBits + (size_t)((unsigned)(ra.stampBase + 1) % 3u) * c->bitWords,
@@ -1285,7 +1299,6 @@ gas_status gas_core_run_persistent(gas_core *c, int32_t maxIters, int32_t haveGa
   ra.denseAlpha = ra.edgeScatter ? 0 : c->denseAlpha;  // Program::scatter walks list rounds
   ra.allActive =
       (c->rangeMode && c->rstart == 0 && c->rcount == c->nV && ra.denseAlpha > 0) ? 1 : 0;
-  ra.vcurOut = &c->ctl->vcur;
   ra.resume = &c->ctl->resume[0];
   ra.denseEndOut = &c->ctl->denseEnd;
 
@@ -1298,17 +1311,11 @@ gas_status gas_core_run_persistent(gas_core *c, int32_t maxIters, int32_t haveGa
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "persistent run launch");
   cudaEventRecord(c->t1, c->stream);
-  int32_t rv[4] = {0, 0, 0, 0};  // rounds, vcur, denseEnd, pad (adjacent in Ctl)
-  A(cudaMemcpyAsync(rv, &c->ctl->rounds, sizeof(rv), cudaMemcpyDeviceToHost, c->stream));
+  A(fetch_head(c));
   A(cudaStreamSynchronize(c->stream));
   if (e != cudaSuccess) return cuda_fail(e, "persistent run");
-  const int32_t rounds = rv[0];
-  if (rv[1]) {  // the result ended in the alternate buffer of the dense rounds
-    A(cudaMemcpyAsync(c->vd, c->valt, (size_t)c->vertexBytes * c->nV, cudaMemcpyDeviceToDevice,
-                      c->stream));
-    A(cudaStreamSynchronize(c->stream));
-    if (e != cudaSuccess) return cuda_fail(e, "persistent run copy-back");
-  }
+  const CtlHead head = *c->head;
+  const int32_t rounds = head.rounds;
   cudaEventElapsedTime(&c->lastMs, c->t0, c->t1);
   const int32_t R = rounds;
   if (R & 1) {
@@ -1324,12 +1331,12 @@ gas_status gas_core_run_persistent(gas_core *c, int32_t maxIters, int32_t haveGa
   c->pendingCommit = false;
   c->haveScatList = false;
   c->countValid = false;
-  if (rv[2] && R > 0) {  // the next frontier is the last round's stamps
+  if (head.denseEnd && R > 0) {  // the next frontier is the last round's stamps
     c->densePending = true;
     c->densePendStamp = c->stamp;  // the last round's stamp
   }
   if (iterations) *iterations = R;
-  return check_device_error(c);
+  return head_error(c);
 }
 
 gas_status gas_core_round_stats(gas_core *c, int32_t capacity, int64_t *active,
