@@ -295,7 +295,7 @@ __device__ __forceinline__ void fused_list_round(const gas_gather_args &a, const
 template <int NT>
 struct FusedBitsSmem {
   int32_t vid[NT * 32];
-  ScanU64Smem<NT> scan;
+  int32_t warpTot[NT / 32];
 };
 
 // A fused round whose frontier is bitmap `bits` (nWords words), owned by
@@ -344,11 +344,27 @@ __device__ __forceinline__ void fused_bits_round(const gas_gather_args &a, const
     // the first pass's units may have been loaded already (read together
     // with the previous round's counts)
     const uint32_t packed = (k0 == 0 && haveFirst) ? first : fused_units<NT>(bits, nWords, k0);
-    const unsigned long long mine = (unsigned long long)__popc(packed);
-    unsigned long long excl, total;
-    block_exclusive_scan_u64<NT>(mine, excl, total, sm.scan);
-    if (total == 0ull) continue;  // block-uniform (the scan ends with a barrier)
-    int off = (int)excl;
+    // positions: a warp scan, then the warps' totals (one block barrier)
+    const int mine = __popc(packed);
+    int incl = mine;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int o = __shfl_up_sync(kFullMask, incl, d);
+      if (lane >= d) incl += o;
+    }
+    if (lane == 31) sm.warpTot[warp] = incl;
+    __syncthreads();
+    int off = incl - mine, total = 0;
+#pragma unroll
+    for (int k = 0; k < NT / 32; ++k) {
+      const int n = sm.warpTot[k];
+      if (k < warp) off += n;
+      total += n;
+    }
+    if (total == 0) {  // block-uniform
+      __syncthreads();  // warpTot is rewritten by the next pass
+      continue;
+    }
     uint32_t rest = packed;
     while (rest) {
       const int p = __ffs(rest) - 1;
@@ -358,14 +374,16 @@ __device__ __forceinline__ void fused_bits_round(const gas_gather_args &a, const
     }
     __syncthreads();
     if (f.width == 4) {  // two listed vertices a thread, their loads interleaved
-      for (int i = threadIdx.x; i < (int)total; i += 2 * NT) {
-        const int vs[2] = {sm.vid[i], i + NT < (int)total ? sm.vid[i + NT] : -1};
+      for (int i = threadIdx.x; i < total; i += 2 * NT) {
+        const int vs[2] = {sm.vid[i], i + NT < total ? sm.vid[i + NT] : -1};
         fused_vertices<P, 2, 4>(a, f, vs, c);
       }
     } else {
-      for (int i = threadIdx.x; i < (int)total; i += NT) fused_vertex<P>(a, f, sm.vid[i], c);
+      for (int i = threadIdx.x; i < total; i += NT) fused_vertex<P>(a, f, sm.vid[i], c);
     }
-    __syncthreads();  // sm.vid is rewritten by the next pass
+    // the lists are rewritten by the next pass (after the last one the round's
+    // grid barrier separates them)
+    if (k0 + 4 * (NT / 32) < perBlock) __syncthreads();
   }
 }
 
