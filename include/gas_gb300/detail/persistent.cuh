@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(PullThreads<P>::value, 1) run_dense_kernel(con
   constexpr bool kMessage = PullSource<P>::kMessage;
   extern __shared__ __align__(16) unsigned char pullSmem[];
   Src *hot = reinterpret_cast<Src *>(pullSmem);
-  uint32_t *hotPrev = reinterpret_cast<uint32_t *>(pullSmem + kHotBytes);
+  uint32_t *hotPrev = reinterpret_cast<uint32_t *>(pullSmem + pull_table_bytes<P>(ra.nHot));
   VD *vd = reinterpret_cast<VD *>(ra.g.vertexData);
   // messages alternate between the two spare vertex buffers, vertex data
   // between its own and the first of them

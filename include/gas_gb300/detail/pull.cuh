@@ -109,9 +109,16 @@ struct PullThreads {
 // The table's entries for values of `bytes` bytes: whole bitmap words.
 __host__ __device__ constexpr int pull_hot_capacity(int bytes) { return kHotBytes / bytes / 128 * 128; }
 
+// Shared memory of a table of nHot slots (slot 0 included): the values, then
+// their bits.  A launch takes what its graph's table needs; what it leaves is
+// L1 for the other gathers.
 template <class P>
-constexpr size_t pull_smem_bytes() {
-  return (size_t)kHotBytes + (size_t)pull_hot_capacity((int)sizeof(typename PullSource<P>::type)) / 8;
+__host__ __device__ constexpr size_t pull_table_bytes(int nHot) {
+  return ((size_t)nHot * sizeof(typename PullSource<P>::type) + 15) / 16 * 16;
+}
+template <class P>
+constexpr size_t pull_smem_bytes(int nHot) {
+  return pull_table_bytes<P>(nHot) + (size_t)(nHot + 31) / 32 * 4;
 }
 
 // What changes from round to round, in shared memory: finishing a vertex

@@ -232,29 +232,31 @@ class EngineGPU {
   // Fused rounds of an apply-only run (BFS: no gather) also use 1 CTA per SM.
   static constexpr int kFusedApplyBlocksPerSM = 1;
   // A run that starts with every vertex active runs its leading dense rounds
-  // in run_dense_kernel (one CTA and about 132 KB of shared memory per SM), then resumes here.
+  // in run_dense_kernel (one CTA per SM, up to 132 KB of shared memory), then resumes here.
 
   static gas_status launchRun(void *user, const gas_run_args *ra, void *stream) {
     EngineGPU *self = static_cast<EngineGPU *>(user);
     if (ra->allActive && ra->resume && ra->pullIds && !ra->denseFirst && self->runBlocksPerSM_ == 0) {
       const void *dk = ra->pullWide ? (const void *)detail::run_dense_kernel<Program, true>
                                     : (const void *)detail::run_dense_kernel<Program, false>;
-      const size_t smem = detail::pull_smem_bytes<Program>();
+      const size_t most = detail::pull_smem_bytes<Program>(
+          detail::pull_hot_capacity((int)sizeof(typename detail::PullSource<Program>::type)));
       if (self->denseGrid_ == 0 || self->denseWide_ != ra->pullWide) {
         self->denseWide_ = ra->pullWide;
         int dev = 0, sms = 0, per = 0, coop = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-        cudaFuncSetAttribute(dk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, dk, detail::PullThreads<Program>::value, smem);
+        cudaFuncSetAttribute(dk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, dk, detail::PullThreads<Program>::value, most);
         cudaGetLastError();
         self->denseGrid_ = (coop && per > 0 && sms > 0) ? sms : -1;
       }
       if (self->denseGrid_ > 0) {
         void *dargs[] = {const_cast<gas_run_args *>(ra)};
         cudaError_t e = cudaLaunchCooperativeKernel(dk, dim3(self->denseGrid_), dim3(detail::PullThreads<Program>::value),
-                                                    dargs, smem, (cudaStream_t)stream);
+                                                    dargs, detail::pull_smem_bytes<Program>(ra->nHot),
+                                                    (cudaStream_t)stream);
         if (e == cudaSuccess) {
           gas_run_args rest = *ra;
           rest.denseFirst = 1;

@@ -398,16 +398,27 @@ __global__ void out_degree_key_kernel(const int32_t *outOff, int32_t nV, uint32_
     key[v] = 65535u - (uint32_t)min(outOff[v + 1] - outOff[v], 65535);
 }
 
+// The least out-degree of a hot vertex.  Each slot costs every SM its share of
+// the table's fill in every round, and saves an SM outDeg / 152 gathers.
+// Without a least degree, 10, 32, 64, 128, 256 (run(), us): CC 200 x 200
+// lattice 2910, 1920 and the same from there on (its degree-4 half was hot);
+// CC, 60,000 vertices, 1.7 M edges 133, 123, 115, 115, 113, 111; PageRank of
+// 30,000 and 150,000 vertices 515, 525, 496, 496, 492, 488 and 1016, 998,
+// 961, 957, 957, 955, of 9,001 240, 263, 257, 257, 257, 257; SSSP of 60,000
+// 275, 261, 250, 248, 248, 250.  Graphs of a million vertices fill the table
+// with higher degrees than these.
+constexpr int kHotMinOut = 64;
+
 // order: the vertices by falling out-degree.  The hot ones: as many whole
-// degree classes as fit `capacity` slots, of which the first stays unused
-// (one block).
+// degree classes of at least kHotMinOut as fit `capacity` slots, of which the
+// first stays unused (one block).
 __global__ void hot_pick_kernel(const uint32_t *order, const int32_t *outOff, int32_t nV, int32_t capacity,
                                 gas::internal::HotInfo *info, int32_t *hotVertex) {
   __shared__ int sHot;
   const int most = capacity - 1;
   auto deg = [&](int k) { return outOff[order[k] + 1] - outOff[order[k]]; };
   if (threadIdx.x == 0) {
-    const int minOut = nV > most ? max(1, deg(most) + 1) : 1;
+    const int minOut = max(kHotMinOut, nV > most ? deg(most) + 1 : 1);
     int lo = 0, hi = min(nV, most);  // the first k of a smaller degree
     while (lo < hi) {
       const int mid = (lo + hi) >> 1;
