@@ -291,8 +291,22 @@ __global__ void __launch_bounds__(PullThreads<P>::value, 1) run_dense_kernel(con
   const long long E = ra.g.nEdges;
   int r = 0, pending = 0, ended = 0;
   PullFirst first;
-  if constexpr (kMessage) {  // the round-0 messages
+  // The round-0 messages, and the hot sources' values side by side: filled
+  // from the vertices themselves, every SM would gather all of them.  (Message
+  // Programs update vertex data in place from round 0 on, so it is read here
+  // alone.)
+  if constexpr (kMessage) {
     for (int v = gtid; v < ra.g.nVertices; v += stride) buf[0][v] = P::gatherMap(vd + v, vd + v, nullptr);
+  }
+  for (int k = gtid + 1; k < ra.nHot; k += stride) {
+    const VD *x = vd + ra.hotVertex[k];
+    if constexpr (kMessage)
+      reinterpret_cast<Src *>(ra.hotVal[0])[k] = P::gatherMap(x, x, nullptr);
+    else
+      reinterpret_cast<Src *>(ra.hotVal[0])[k] = *x;
+  }
+  for (int k = threadIdx.x; k < hotWords; k += blockDim.x) hotPrev[k] = 0u;
+  if (kMessage || ra.nHot > 1) {
     if (!grid_barrier(ra.barrier, ra.g.errWord)) ended = 1;
   }
   for (; !ended;) {
@@ -305,19 +319,13 @@ __global__ void __launch_bounds__(PullThreads<P>::value, 1) run_dense_kernel(con
     clear_ahead(ra, stamp);
     for (int i = gtid; i < hotWords; i += stride) ra.hotBits[(unsigned)(stamp + 1) % 3u][i] = 0u;
     // the hot sources' values and bits as of the previous round's end
-    if (r == 0) {
-      if (threadIdx.x < (unsigned)hotWords) hotPrev[threadIdx.x] = 0u;
-      // (from buf[0]: message Programs already update vertex data in place
-      // where other blocks have started the round)
-#pragma unroll 8
-      for (int k = threadIdx.x + 1; k < ra.nHot; k += blockDim.x) hot[k] = load_cg(buf[0] + ra.hotVertex[k]);
-    } else if (ra.nHot > 1) {
+    if (ra.nHot > 1) {
       const int4 *from = reinterpret_cast<const int4 *>(ra.hotVal[r & 1]);
       const int quads = (int)(((size_t)ra.nHot * sizeof(Src) + 15) / 16);
 #pragma unroll 8
       for (int k = threadIdx.x; k < quads; k += blockDim.x) reinterpret_cast<int4 *>(hot)[k] = __ldcg(from + k);
       const uint32_t *bits = ra.hotBits[(unsigned)(stamp - 1) % 3u];
-      for (int k = threadIdx.x; k < hotWords; k += blockDim.x) hotPrev[k] = __ldcg(bits + k);
+      for (int k = threadIdx.x; k < hotWords && r > 0; k += blockDim.x) hotPrev[k] = __ldcg(bits + k);
     }
     unsigned long long *cnt = ra.denseCnt + kDenseCntStride * (r % 3);
     if (threadIdx.x == 0) {

@@ -259,7 +259,7 @@ struct PullStep {
 // Loads the step whose ids are s4 (its values; its edge data from *eds),
 // tests its hot sources' bits while some vertex of the warp is not known to
 // be active, then fetches the next ids if there are any.
-template <class P, int W>
+template <class P, int W, bool WIDE>
 __device__ __forceinline__ void pull_step(const PullCtx<P> &a, const gas_run_args &ra, int4 &s4, const int4 *&ids,
                                           const int4 *&eds, bool more, bool &hit, bool &allHit, PullStep<P> &x) {
   const int s[4] = {s4.x, s4.y, s4.z, s4.w};
@@ -278,7 +278,14 @@ __device__ __forceinline__ void pull_step(const PullCtx<P> &a, const gas_run_arg
   if (!allHit) {
     if (!hit) {
       bool h = false;
-      if (ra.nHot > 1) {
+      if constexpr (WIDE) {  // hot and cold ones alike, in flight with the values
+        const uint32_t *bits = a.round->prevBits;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int k = s[j] & 0x7fffffff;
+          h |= ((s[j] < 0 ? a.hotPrev : bits)[k >> 5] >> (k & 31)) & 1u;  // slot 0's bit is never set
+        }
+      } else if (ra.nHot > 1) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) h = h || (s[j] < 0 && hot_bit<P>(a, s[j]));
       } else {  // no hot sources (a lattice): pull_cold would find them all
@@ -312,7 +319,7 @@ __device__ __forceinline__ typename P::GatherResult pull_edge(const PullCtx<P> &
 }
 
 // In-degree <= 8, one lane a vertex: a left fold from gatherZero.
-template <class P>
+template <class P, bool WIDE>
 __device__ __forceinline__ bool pull_serial(const PullCtx<P> &a, const gas_run_args &ra, const PullUnit &u, int4 s4,
                                             EdgeAcc<typename P::GatherResult> &x) {
   const int lane = threadIdx.x & 31, v = u.rec.x;
@@ -322,7 +329,7 @@ __device__ __forceinline__ bool pull_serial(const PullCtx<P> &a, const gas_run_a
   const int4 *eds = static_cast<const int4 *>(ra.pullEds) + u.base + lane;
   for (int t = 0; t < u.quads; ++t) {  // warp-uniform
     PullStep<P> st;
-    pull_step<P, 1>(a, ra, s4, ids, eds, t + 1 < u.quads, hit, allHit, st);
+    pull_step<P, 1, WIDE>(a, ra, s4, ids, eds, t + 1 < u.quads, hit, allHit, st);
     if (ra.g.haveGather) {
 #pragma unroll
       for (int j = 0; j < 4; ++j)
@@ -330,13 +337,13 @@ __device__ __forceinline__ bool pull_serial(const PullCtx<P> &a, const gas_run_a
           x.val = P::gatherReduce(x.val, pull_edge<P>(a, ra, v, st, j, u.rec.y + 4 * t + j));
     }
   }
-  if (!allHit && ra.nHot > 1) hit = pull_cold<P, 1>(a, ra, u, u.quads, hit);
+  if (!WIDE && !allHit && ra.nHot > 1) hit = pull_cold<P, 1>(a, ra, u, u.quads, hit);
   return hit;
 }
 
 // W lanes a vertex, the quads of its in-edges dealt round-robin, folded as
 // they come.
-template <class P, int W>
+template <class P, int W, bool WIDE>
 __device__ __forceinline__ bool pull_any(const PullCtx<P> &a, const gas_run_args &ra, const PullUnit &u, int sl,
                                          int4 s4, EdgeAcc<typename P::GatherResult> &x) {
   const int lane = threadIdx.x & 31, v = u.rec.x;
@@ -348,7 +355,7 @@ __device__ __forceinline__ bool pull_any(const PullCtx<P> &a, const gas_run_args
   x.has = ra.g.haveGather && rem > 0 ? 1u : 0u;
   for (int t = 0; t < u.quads; ++t, rem -= 4 * W) {  // warp-uniform
     PullStep<P> st;
-    pull_step<P, W>(a, ra, s4, ids, eds, t + 1 < u.quads, hit, allHit, st);
+    pull_step<P, W, WIDE>(a, ra, s4, ids, eds, t + 1 < u.quads, hit, allHit, st);
     if (ra.g.haveGather) {
       const int pos = u.rec.y + u.rec.z - rem;
 #pragma unroll
@@ -359,7 +366,7 @@ __device__ __forceinline__ bool pull_any(const PullCtx<P> &a, const gas_run_args
         }
     }
   }
-  if (!allHit && ra.nHot > 1) hit = pull_cold<P, W>(a, ra, u, u.quads, hit);
+  if (!WIDE && !allHit && ra.nHot > 1) hit = pull_cold<P, W>(a, ra, u, u.quads, hit);
   return hit;
 }
 
@@ -367,7 +374,7 @@ __device__ __forceinline__ bool pull_any(const PullCtx<P> &a, const gas_run_args
 // group_edges gives it: per such lane its unaligned edge if it has one, then
 // its quads, then the lanes' results combined in pairs, pairs of pairs, ...
 // x: the lane's result; returns whether its vertex is active (group-uniform).
-template <class P, int W, int VL>
+template <class P, int W, int VL, bool WIDE>
 __device__ __forceinline__ bool pull_ordered(const PullCtx<P> &a, const gas_run_args &ra, const PullUnit &u, int sl,
                                              int4 s4, EdgeAcc<typename P::GatherResult> &x) {
   typedef typename P::GatherResult GR;
@@ -400,7 +407,7 @@ __device__ __forceinline__ bool pull_ordered(const PullCtx<P> &a, const gas_run_
       pos = sl < 4 ? u.rec.y + sl : tailPos + sl - 4;
     }
     PullStep<P> st;
-    pull_step<P, W>(a, ra, s4, ids, eds, h + 1 < ENDS || u.quads > 0, hit, allHit, st);
+    pull_step<P, W, WIDE>(a, ra, s4, ids, eds, h + 1 < ENDS || u.quads > 0, hit, allHit, st);
     if (ra.g.haveGather) {
 #pragma unroll
       for (int j = 0; j < (VL == 1 ? 1 : 3); ++j)
@@ -427,7 +434,7 @@ __device__ __forceinline__ bool pull_ordered(const PullCtx<P> &a, const gas_run_
 #pragma unroll 1
     for (int l = 0; l < layers; ++l, q += LAYER) {  // warp-uniform
       PullStep<P> st;
-      pull_step<P, W>(a, ra, s4, ids, eds, --left > 0, hit, allHit, st);
+      pull_step<P, W, WIDE>(a, ra, s4, ids, eds, --left > 0, hit, allHit, st);
       if (q < rg.quads && ra.g.haveGather) {
         const int pos = 4 * (rg.first + q);
         const GR m = pull_edge<P>(a, ra, v, st, 0, pos);
@@ -458,7 +465,7 @@ __device__ __forceinline__ bool pull_ordered(const PullCtx<P> &a, const gas_run_
       x.has = has ? 1u : 0u;
     }
   }
-  if (!allHit && ra.nHot > 1) hit = pull_cold<P, W>(a, ra, u, steps, hit);
+  if (!WIDE && !allHit && ra.nHot > 1) hit = pull_cold<P, W>(a, ra, u, steps, hit);
   return hit;
 }
 
@@ -577,21 +584,21 @@ __device__ __forceinline__ void pull_unit(const PullCtx<P> &a, const gas_run_arg
     typename P::VertexData own;  // on its way while the edges are gathered
     if (mine) own = pull_own<P>(a, ra, v);
     if (u >= n.small) {
-      act = pull_serial<P>(a, ra, pu, s4, x);
+      act = pull_serial<P, WIDE>(a, ra, pu, s4, x);
     } else {
       constexpr int M = pull_mid_lanes(WIDE), S = pull_small_lanes(WIDE);
       if (u >= n.mid) {
         if constexpr (kAny)
-          act = pull_any<P, S>(a, ra, pu, lane % S, s4, x);
+          act = pull_any<P, S, WIDE>(a, ra, pu, lane % S, s4, x);
         else
-          act = pull_ordered<P, S, kSmallLanes / S>(a, ra, pu, lane % S, s4, x);
+          act = pull_ordered<P, S, kSmallLanes / S, WIDE>(a, ra, pu, lane % S, s4, x);
         if (S > 1 && ra.g.haveGather) pull_combine<P, S>(x);
         mine = mine && lane % S == 0;
       } else {
         if constexpr (kAny)
-          act = pull_any<P, M>(a, ra, pu, lane % M, s4, x);
+          act = pull_any<P, M, WIDE>(a, ra, pu, lane % M, s4, x);
         else
-          act = pull_ordered<P, M, 32 / M>(a, ra, pu, lane % M, s4, x);
+          act = pull_ordered<P, M, 32 / M, WIDE>(a, ra, pu, lane % M, s4, x);
         if (ra.g.haveGather) pull_combine<P, M>(x);
         mine = mine && lane % M == 0;
       }
@@ -603,9 +610,9 @@ __device__ __forceinline__ void pull_unit(const PullCtx<P> &a, const gas_run_arg
   {
     bool act;
     if constexpr (kAny)
-      act = pull_any<P, 32>(a, ra, pu, lane, s4, x);
+      act = pull_any<P, 32, WIDE>(a, ra, pu, lane, s4, x);
     else
-      act = pull_ordered<P, 32, 1>(a, ra, pu, lane, s4, x);
+      act = pull_ordered<P, 32, 1, WIDE>(a, ra, pu, lane, s4, x);
     // a chunk publishes its partial; the vertex's last to arrive combines
     const int ch = u;
     if (ra.g.haveGather) pull_combine<P, 32>(x);
