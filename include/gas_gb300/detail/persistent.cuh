@@ -268,7 +268,7 @@ constexpr long long kMarkPullFactor = 4;
 // 1 the run is over, 2 stopped at maxRounds before a dense round); the
 // rounds, stamps, resets and statistics are the main kernel's own.
 template <class P, bool WIDE>
-__global__ void __launch_bounds__(PullThreads<P>::value, 1) run_dense_kernel(const gas_run_args ra) {
+__global__ void __launch_bounds__(PullThreads<P, WIDE>::value, 1) run_dense_kernel(const gas_run_args ra) {
   typedef typename P::VertexData VD;
   typedef typename PullSource<P>::type Src;
   constexpr bool kMessage = PullSource<P>::kMessage;
@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(PullThreads<P>::value, 1) run_dense_kernel(con
   const int stride = gridDim.x * blockDim.x, gtid = blockIdx.x * blockDim.x + threadIdx.x;
   const long long E = ra.g.nEdges;
   int r = 0, pending = 0, ended = 0;
-  PullFirst first;
+  __shared__ PullKept<WIDE ? kWideThreads : 1> kept;
   // The round-0 messages, and the hot sources' values side by side: filled
   // from the vertices themselves, every SM would gather all of them.  (Message
   // Programs update vertex data in place from round 0 on, so it is read here
@@ -344,8 +344,10 @@ __global__ void __launch_bounds__(PullThreads<P>::value, 1) run_dense_kernel(con
     __syncthreads();
     a.cur = round.cur;
     a.allActive = r == 0;
-    if (WIDE && r == 0) first = pull_first<WIDE>(ra, units, pull_first_unit());
-    const DenseCounts counts = pull_pass<P, WIDE>(a, ra, units, first);
+    if constexpr (WIDE) {
+      if (r == 0) keep_first(kept, pull_first<WIDE>(ra, units, pull_first_unit()));
+    }
+    const DenseCounts counts = pull_pass<P, WIDE>(a, ra, units, kept);
     if (!counts_barrier(ra.barrier, ra.g.errWord, counts, cnt)) {
       ended = 1;
       break;

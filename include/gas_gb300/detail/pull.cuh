@@ -100,10 +100,15 @@ struct PullSource {
 
 // Threads of the CTA, by the registers a thread needs: with the table in
 // place of L1 a spill is an L2 round trip (SSSP R-MAT-18 0.54 ms at 1,024
-// threads with 88 bytes of spills, 0.45 at 896 without).
-template <class P>
+// threads with 88 bytes of spills, 0.45 at 896 without).  The wide form keeps
+// more: of 640, 768 and 896 threads (none spills at 768), 768 is 1 to 2 %
+// ahead over R-MAT graphs of 4,096..150,000 vertices (PageRank 60,000: 644,
+// 564, 619 us; 9,001: 386, 390, 416).
+constexpr int kWideThreads = 768;
+template <class P, bool WIDE>
 struct PullThreads {
-  static constexpr int value = (ProgramReduceAnyOrder<P>::value ? 896 : 768) + (PullSource<P>::kMessage ? 128 : 0);
+  static constexpr int value =
+      WIDE ? kWideThreads : (ProgramReduceAnyOrder<P>::value ? 896 : 768) + (PullSource<P>::kMessage ? 128 : 0);
 };
 
 // The table's entries for values of `bytes` bytes: whole bitmap words.
@@ -675,11 +680,29 @@ __host__ __device__ __forceinline__ PullUnits pull_units(const gas_run_args &ra,
 }
 
 // A warp's first unit and its ids.  They are the same in every round; the
-// wide form, whose rounds are a chain of few loads, keeps them.
+// wide form, whose rounds are a chain of few loads, keeps them in shared
+// memory (in registers they were spilled, and local memory is an L2 round
+// trip once a barrier has invalidated L1).
 struct PullFirst {
   PullUnit unit;
   int4 ids;
 };
+template <int NT>
+struct PullKept {
+  int4 rec[NT], ids[NT];
+  int2 at[NT];
+};
+template <int NT>
+__device__ __forceinline__ void keep_first(PullKept<NT> &k, const PullFirst &f) {
+  k.rec[threadIdx.x] = f.unit.rec;
+  k.ids[threadIdx.x] = f.ids;
+  k.at[threadIdx.x] = make_int2(f.unit.base, f.unit.quads);
+}
+template <int NT>
+__device__ __forceinline__ PullFirst kept_first(const PullKept<NT> &k) {
+  const int2 at = k.at[threadIdx.x];
+  return {{at.x, at.y, k.rec[threadIdx.x]}, k.ids[threadIdx.x]};
+}
 template <bool WIDE>
 __device__ __forceinline__ PullFirst pull_first(const gas_run_args &ra, const volatile PullUnits &n, int u) {
   PullFirst f = {{0, 0, make_int4(-1, 0, 0, 0)}, make_int4(kNoEdge, kNoEdge, kNoEdge, kNoEdge)};
@@ -702,7 +725,7 @@ __device__ __forceinline__ int pull_first_unit() {
 // ahead.
 template <class P, bool WIDE>
 __device__ DenseCounts pull_pass(const PullCtx<P> &a, const gas_run_args &ra, const volatile PullUnits &n,
-                                 const PullFirst &first) {
+                                 const PullKept<WIDE ? kWideThreads : 1> &kept) {
   DenseCounts c = {0u, 0u, 0u, 0u};
   const int lane = threadIdx.x & 31;
   const int warps = (int)(gridDim.x * (blockDim.x / 32));
@@ -712,7 +735,11 @@ __device__ DenseCounts pull_pass(const PullCtx<P> &a, const gas_run_args &ra, co
   const int dealt = n.total < 4 * warps ? 4 * warps : n.total / 4 * 3 / warps * warps;
   int u = pull_first_unit();
   const PullUnit noUnit = {0, 0, make_int4(-1, 0, 0, 0)};
-  const PullFirst f = WIDE ? first : pull_first<WIDE>(ra, n, u);
+  PullFirst f;
+  if constexpr (WIDE)
+    f = kept_first(kept);
+  else
+    f = pull_first<WIDE>(ra, n, u);
   PullUnit pu = f.unit;
   int4 s4 = f.ids;
   int next = n.total;  // lane 0: the next batch, asked for one unit early

@@ -239,6 +239,8 @@ class EngineGPU {
     if (ra->allActive && ra->resume && ra->pullIds && !ra->denseFirst && self->runBlocksPerSM_ == 0) {
       const void *dk = ra->pullWide ? (const void *)detail::run_dense_kernel<Program, true>
                                     : (const void *)detail::run_dense_kernel<Program, false>;
+      const int threads =
+          ra->pullWide ? detail::PullThreads<Program, true>::value : detail::PullThreads<Program, false>::value;
       const size_t most = detail::pull_smem_bytes<Program>(
           detail::pull_hot_capacity((int)sizeof(typename detail::PullSource<Program>::type)));
       if (self->denseGrid_ == 0 || self->denseWide_ != ra->pullWide) {
@@ -248,14 +250,14 @@ class EngineGPU {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
         cudaFuncSetAttribute(dk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, dk, detail::PullThreads<Program>::value, most);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, dk, threads, most);
         cudaGetLastError();
         self->denseGrid_ = (coop && per > 0 && sms > 0) ? sms : -1;
       }
       if (self->denseGrid_ > 0) {
         void *dargs[] = {const_cast<gas_run_args *>(ra)};
-        cudaError_t e = cudaLaunchCooperativeKernel(dk, dim3(self->denseGrid_), dim3(detail::PullThreads<Program>::value),
-                                                    dargs, detail::pull_smem_bytes<Program>(ra->nHot),
+        cudaError_t e = cudaLaunchCooperativeKernel(dk, dim3(self->denseGrid_), dim3(threads), dargs,
+                                                    detail::pull_smem_bytes<Program>(ra->nHot),
                                                     (cudaStream_t)stream);
         if (e == cudaSuccess) {
           gas_run_args rest = *ra;
