@@ -52,6 +52,7 @@ struct BatchArgs {
   int32_t *inList;            // [V] round stamp of list membership
   int32_t alpha;              // push when out-degree total * alpha <= nEdges
   int32_t nQueries;       // padded to 32 * W
+  int32_t nLive;          // queries among them
   const int32_t *inSources;
   const int32_t *weights;  // CSC order (SSSP)
   const int32_t *unitV;
@@ -133,98 +134,197 @@ __device__ __forceinline__ void warp_append(bool want, int v, int d, int32_t *li
   }
 }
 
-template <int W, int KIND>
-__device__ __forceinline__ void batch_unit(const BatchArgs &a, int u, int round,
-                                           const unsigned *cur, unsigned *nxt,
-                                           unsigned long long &changed) {
+// Row i of W-word rows (16-byte aligned from W = 4 on, as the buffers are),
+// zero unless ok.  Wide loads: past L1 every load is its own L2 request.
+template <int W>
+__device__ __forceinline__ void load_words(const unsigned *rows, int i, bool ok, unsigned (&m)[W]) {
+  const unsigned *p = rows + (size_t)i * W;
+#pragma unroll
+  for (int k = 0; k < W; ++k) m[k] = 0u;
+  if (!ok) return;
+  if constexpr (W % 4 == 0) {
+#pragma unroll
+    for (int k = 0; k < W; k += 4) {
+      const uint4 x = __ldcg(reinterpret_cast<const uint4 *>(p + k));
+      m[k] = x.x;
+      m[k + 1] = x.y;
+      m[k + 2] = x.z;
+      m[k + 3] = x.w;
+    }
+  } else if constexpr (W == 2) {
+    const uint2 x = __ldcg(reinterpret_cast<const uint2 *>(p));
+    m[0] = x.x;
+    m[1] = x.y;
+  } else {
+#pragma unroll
+    for (int k = 0; k < W; ++k) m[k] = __ldcg(p + k);
+  }
+}
+
+// Pull round of a BFS batch, a warp a unit: units u0, u0 + stride, ...  A
+// lane looks up each of the next 32 (vertex, range, and whether the vertex
+// still has a query to be reached: most have none from the third round on),
+// then the warp walks those that do, the next one's first sources in flight,
+// and ends a unit once every query has reached its vertex.  A vertex of one
+// unit belongs to this warp alone: its seen row is read with the sources and
+// written back plainly, where an atomic would be one more L2 round trip.
+// Bound by L2: the masks of a round, one 32-byte sector an edge.  A run, with
+// eight 4-byte loads an edge and every unit walked -> now: 256 queries on
+// R-MAT-18 (6.1 M edges) 1.63 -> 0.69 ms, 64 queries 0.65 -> 0.36, 10 queries
+// 0.29 -> 0.24; 200 queries on R-MAT-16 0.61 -> 0.28.
+template <int W>
+__device__ __forceinline__ void batch_bfs_pull(const BatchArgs &a, long long u0, long long stride, int round,
+                                               const unsigned *cur, unsigned *nxt, unsigned long long &changed) {
+  const int lane = threadIdx.x & 31;
+  const int Q = W * 32;
+  // this lane's word of a row: its live queries (lanes past W: none)
+  const int liveBits = lane < W ? a.nLive - 32 * lane : 0;
+  const unsigned live = liveBits >= 32 ? kFullMask : liveBits > 0 ? (1u << liveBits) - 1u : 0u;
+  for (long long base = u0; base < a.nUnits; base += 32 * stride) {  // warp-uniform
+    const long long u = base + lane * stride;
+    int v = -1, beg = 0, end = 0;
+    if (u < a.nUnits) {
+      v = __ldg(a.unitV + u);
+      beg = __ldg(a.unitBeg + u);
+      end = __ldg(a.unitEnd + u);
+      if ((u > 0 && __ldg(a.unitV + u - 1) == v) || (u + 1 < a.nUnits && __ldg(a.unitV + u + 1) == v))
+        end = -end;  // (a unit's end is above 0) one of several of its vertex
+    }
+    unsigned row[W];
+    load_words<W>(a.seen, v, v >= 0, row);
+    bool need = false;
+#pragma unroll
+    for (int k = 0; k < W; ++k) need |= (~row[k] & __shfl_sync(kFullMask, live, k)) != 0u;
+    unsigned work = __ballot_sync(kFullMask, need && v >= 0);
+    if (!work) continue;
+    int j = __ffs(work) - 1;
+    int nb = __shfl_sync(kFullMask, beg, j), ne = __shfl_sync(kFullMask, end, j);
+    int sn = nb + lane < abs(ne) ? __ldg(a.inSources + nb + lane) : -1;
+    while (work) {
+      work &= work - 1u;
+      const int cv = __shfl_sync(kFullMask, v, j);
+      const bool split = ne < 0;
+      const int ce = abs(ne);
+      int e0 = nb, s = sn;
+      const unsigned seen = lane < W ? __ldcg(a.seen + (size_t)cv * W + lane) : 0u;
+      if (work) {
+        j = __ffs(work) - 1;
+        nb = __shfl_sync(kFullMask, beg, j);
+        ne = __shfl_sync(kFullMask, end, j);
+        sn = nb + lane < abs(ne) ? __ldg(a.inSources + nb + lane) : -1;
+      }
+      unsigned acc[W], mine = 0u;
+#pragma unroll
+      for (int k = 0; k < W; ++k) acc[k] = 0u;
+      for (;;) {  // 64 edges
+        unsigned m[W];
+        const int s1 = e0 + 32 + lane < ce ? __ldg(a.inSources + e0 + 32 + lane) : -1;
+        load_words<W>(cur, s, s >= 0, m);
+#pragma unroll
+        for (int k = 0; k < W; ++k) acc[k] |= m[k];
+        if (e0 + 32 < ce) {
+          const int s2 = e0 + 64 + lane < ce ? __ldg(a.inSources + e0 + 64 + lane) : -1;
+          load_words<W>(cur, s1, s1 >= 0, m);
+#pragma unroll
+          for (int k = 0; k < W; ++k) acc[k] |= m[k];
+          s = s2;
+        }
+#pragma unroll
+        for (int k = 0; k < W; ++k) {
+          const unsigned all = __reduce_or_sync(kFullMask, acc[k]);
+          if (lane == k) mine = all;
+        }
+        e0 += 64;
+        if (e0 >= ce || __all_sync(kFullMask, (live & ~(mine | seen)) == 0u)) break;
+      }
+      unsigned fresh = mine & ~seen;
+      if (split) {
+        if (fresh) fresh &= ~atomicOr(a.seen + (size_t)cv * W + lane, fresh);
+        if (fresh) atomicOr(nxt + (size_t)cv * W + lane, fresh);
+      } else if (fresh) {
+        a.seen[(size_t)cv * W + lane] = seen | fresh;
+        nxt[(size_t)cv * W + lane] = fresh;
+      }
+      changed += __popc(fresh);
+#pragma unroll
+      for (int k = 0; k < W; ++k)
+        if ((__shfl_sync(kFullMask, fresh, k) >> lane) & 1u) a.value[(size_t)cv * Q + k * 32 + lane] = round + 1;
+    }
+  }
+}
+
+// One unit of a pull round of an SSSP batch.
+template <int W>
+__device__ __forceinline__ void batch_sssp_unit(const BatchArgs &a, int u, const unsigned *cur, unsigned *nxt,
+                                                unsigned long long &changed) {
   const int lane = threadIdx.x & 31;
   const int v = a.unitV[u];
   const int beg = a.unitBeg[u], end = a.unitEnd[u];
   const int Q = W * 32;
-  if (KIND == kBatchBFS) {
-    unsigned acc[W];
+  int best[W];
 #pragma unroll
-    for (int k = 0; k < W; ++k) acc[k] = 0u;
-    for (int e0 = beg; e0 < end; e0 += 32) {
-      const int e = e0 + lane;
-      const int s = e < end ? __ldg(a.inSources + e) : -1;
-      unsigned m[W];
+  for (int k = 0; k < W; ++k) best[k] = kBatchInf;
+  for (int e0 = beg; e0 < end; e0 += 32) {
+    // lane j loads edge e0+j: source, weight and its changed-query mask
+    const int e = e0 + lane;
+    const bool ok = e < end;
+    const int s = ok ? __ldg(a.inSources + e) : 0;
+    const int w = ok ? __ldg(a.weights + e) : 0;
+    unsigned m[W], any = 0u;
+    load_words<W>(cur, s, ok, m);
 #pragma unroll
-      for (int k = 0; k < W; ++k) m[k] = s >= 0 ? __ldcg(cur + (size_t)s * W + k) : 0u;
+    for (int k = 0; k < W; ++k) any |= m[k];
+    unsigned work = __ballot_sync(kFullMask, any != 0u);  // edges with a changed query
+    // warp-uniform; the values of T edges in flight a lane (32 loads at
+    // most): a unit's time is one L2 round trip for each batch of them
+    // (R-MAT-18: 10 queries 4.06 -> 1.99 ms a run, 64 queries 8.36 -> 3.75,
+    // 256 queries 16.1 -> 13.6, from four edges in flight to T)
+    constexpr int T = W == 1 ? 16 : 32 / W;
+    while (work) {
+      int d[T][W];
 #pragma unroll
-      for (int k = 0; k < W; ++k) acc[k] |= __reduce_or_sync(kFullMask, m[k]);
-    }
+      for (int t = 0; t < T; ++t) {
+        const int js = work ? __ffs(work) - 1 : 0;
+        const bool on = work != 0u;
+        if (work) work &= work - 1;
+        const int sj = __shfl_sync(kFullMask, s, js);
+        const int wj = __shfl_sync(kFullMask, w, js);
 #pragma unroll
-    for (int k = 0; k < W; ++k) {
-      if (!acc[k]) continue;  // warp-uniform
-      unsigned fresh = 0u;
-      if (lane == 0) {
-        const unsigned old = atomicOr(a.seen + (size_t)v * W + k, acc[k]);
-        fresh = acc[k] & ~old;
-        if (fresh) atomicOr(nxt + (size_t)v * W + k, fresh);
-      }
-      fresh = __shfl_sync(kFullMask, fresh, 0);
-      if ((fresh >> lane) & 1u) a.value[(size_t)v * Q + k * 32 + lane] = round + 1;
-      if (lane == 0) changed += __popc(fresh);
-    }
-  } else {
-    int best[W];
-#pragma unroll
-    for (int k = 0; k < W; ++k) best[k] = kBatchInf;
-    for (int e0 = beg; e0 < end; e0 += 32) {
-      // lane j loads edge e0+j: source, weight and its changed-query mask
-      const int e = e0 + lane;
-      const bool ok = e < end;
-      const int s = ok ? __ldg(a.inSources + e) : 0;
-      const int w = ok ? __ldg(a.weights + e) : 0;
-      unsigned m[W], any = 0u;
-#pragma unroll
-      for (int k = 0; k < W; ++k) {
-        m[k] = ok ? __ldcg(cur + (size_t)s * W + k) : 0u;
-        any |= m[k];
-      }
-      unsigned work = __ballot_sync(kFullMask, any != 0u);  // edges with a changed query
-      // warp-uniform; the values of T edges in flight a lane (32 loads at
-      // most): a unit's time is one L2 round trip for each batch of them
-      // (R-MAT-18: 10 queries 4.06 -> 1.99 ms a run, 64 queries 8.36 -> 3.75,
-      // 256 queries 16.1 -> 13.6, from four edges in flight to T)
-      constexpr int T = W == 1 ? 16 : 32 / W;
-      while (work) {
-        int d[T][W];
-#pragma unroll
-        for (int t = 0; t < T; ++t) {
-          const int js = work ? __ffs(work) - 1 : 0;
-          const bool on = work != 0u;
-          if (work) work &= work - 1;
-          const int sj = __shfl_sync(kFullMask, s, js);
-          const int wj = __shfl_sync(kFullMask, w, js);
-#pragma unroll
-          for (int k = 0; k < W; ++k) {
-            const unsigned mk = __shfl_sync(kFullMask, m[k], js);
-            d[t][k] = kBatchInf;
-            if (on && ((mk >> lane) & 1u)) d[t][k] = __ldcg(a.value + (size_t)sj * Q + k * 32 + lane) + wj;
-          }
+        for (int k = 0; k < W; ++k) {
+          const unsigned mk = __shfl_sync(kFullMask, m[k], js);
+          d[t][k] = kBatchInf;
+          if (on && ((mk >> lane) & 1u)) d[t][k] = __ldcg(a.value + (size_t)sj * Q + k * 32 + lane) + wj;
         }
-#pragma unroll
-        for (int t = 0; t < T; ++t)
-#pragma unroll
-          for (int k = 0; k < W; ++k) best[k] = min(best[k], d[t][k]);
       }
-    }
 #pragma unroll
-    for (int k = 0; k < W; ++k) {
-      bool improved = false;
-      if (best[k] < kBatchInf) {
-        const int old = atomicMin(a.value + (size_t)v * Q + k * 32 + lane, best[k]);
-        improved = best[k] < old;
-      }
-      const unsigned word = __ballot_sync(kFullMask, improved);
-      if (lane == 0 && word) {
-        atomicOr(nxt + (size_t)v * W + k, word);
-        changed += __popc(word);
-      }
+      for (int t = 0; t < T; ++t)
+#pragma unroll
+        for (int k = 0; k < W; ++k) best[k] = min(best[k], d[t][k]);
     }
   }
+#pragma unroll
+  for (int k = 0; k < W; ++k) {
+    bool improved = false;
+    if (best[k] < kBatchInf) {
+      const int old = atomicMin(a.value + (size_t)v * Q + k * 32 + lane, best[k]);
+      improved = best[k] < old;
+    }
+    const unsigned word = __ballot_sync(kFullMask, improved);
+    if (lane == 0 && word) {
+      atomicOr(nxt + (size_t)v * W + k, word);
+      changed += __popc(word);
+    }
+  }
+}
+
+// A pull round: units u0, u0 + stride, ... (one warp).
+template <int W, int KIND>
+__device__ __forceinline__ void batch_pull_round(const BatchArgs &a, long long u0, long long stride, int round,
+                                                 const unsigned *cur, unsigned *nxt, unsigned long long &changed) {
+  if constexpr (KIND == kBatchBFS)
+    batch_bfs_pull<W>(a, u0, stride, round, cur, nxt, changed);
+  else
+    for (long long u = u0; u < a.nUnits; u += stride) batch_sssp_unit<W>(a, (int)u, cur, nxt, changed);
 }
 
 // Push round: a warp per list entry (u, chunk), lanes over the chunk's
@@ -239,8 +339,7 @@ __device__ __forceinline__ void batch_push_unit(const BatchArgs &a, int u, int c
   const int lane = threadIdx.x & 31;
   const int Q = W * 32;
   unsigned m[W];
-#pragma unroll
-  for (int k = 0; k < W; ++k) m[k] = __ldcg(cur + (size_t)u * W + k);
+  load_words<W>(cur, u, true, m);
   int du[W];
   if (KIND == kBatchSSSP) {
 #pragma unroll
@@ -637,10 +736,10 @@ __device__ __forceinline__ void batch_compact(const BatchArgs &a, const unsigned
   for (long long base = gw * 32; base < a.nVertices; base += warps * 32) {
     const long long v = base + lane;
     unsigned any = 0u;
-    if (v < a.nVertices) {
+    unsigned m[W];
+    load_words<W>(nxt, (int)v, v < a.nVertices, m);
 #pragma unroll
-      for (int k = 0; k < W; ++k) any |= __ldcg(nxt + (size_t)v * W + k);
-    }
+    for (int k = 0; k < W; ++k) any |= m[k];
     const bool want = any != 0u;
     warp_append(want, (int)v, want ? a.outOffsets[v + 1] - a.outOffsets[v] : 0, listNext,
                 listNextC, cntNext);
@@ -717,8 +816,7 @@ __global__ void __launch_bounds__(256, PAIRS == kPairsList ? 6 : 4) batch_run_ke
         batch_push_unit<W, KIND>(a, listCur[i], listCurC[i], r, cur, nxt, listNext, listNextC,
                                  cntNext, changed, bk);
     } else {
-      for (long long u = gw; u < a.nUnits; u += warps)
-        batch_unit<W, KIND>(a, (int)u, r, cur, nxt, changed);
+      batch_pull_round<W, KIND>(a, gw, warps, r, cur, nxt, changed);
     }
     (void)clr;
     changed = warp_sum_u64(changed);

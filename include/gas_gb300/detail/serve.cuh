@@ -92,8 +92,7 @@ __global__ void __launch_bounds__(256) batch_round_kernel(const BatchArgs a, int
       batch_push_unit<W, KIND>(a, a.list[rc][i], a.listC[rc][i], r, cur, nxt, a.list[rn],
                                a.listC[rn], a.listCnt + rn, changed, bk);
   } else {
-    for (long long u = gw; u < a.nUnits; u += warps)
-      batch_unit<W, KIND>(a, (int)u, r, cur, nxt, changed);
+    batch_pull_round<W, KIND>(a, gw, warps, r, cur, nxt, changed);
   }
   changed = warp_sum_u64(changed);
   if ((threadIdx.x & 31) == 0 && changed) atomicAdd(a.cnt + rc, changed);

@@ -221,7 +221,7 @@ const void *run_fn(int pairs) {
 }
 
 template <int W, int KIND>
-gas_status launch_run(gas_batch *b, const CoreGraph &g, int32_t Q, int blocks, int pairs) {
+gas_status launch_run(gas_batch *b, const CoreGraph &g, int32_t nQ, int32_t Q, int blocks, int pairs) {
   gas::detail::BatchArgs a;
   memset(&a, 0, sizeof(a));
   a.nVertices = g.nV;
@@ -236,6 +236,7 @@ gas_status launch_run(gas_batch *b, const CoreGraph &g, int32_t Q, int blocks, i
   a.inList = b->inList;
   a.alpha = b->alpha;
   a.nQueries = Q;
+  a.nLive = nQ;
   a.inSources = g.inSrc;
   a.weights = reinterpret_cast<const int32_t *>(g.edgeData);
   a.unitV = b->unitV;
@@ -266,11 +267,11 @@ gas_status launch_run(gas_batch *b, const CoreGraph &g, int32_t Q, int blocks, i
 }
 
 template <int W>
-gas_status launch_run_kind(gas_batch *b, const CoreGraph &g, int kind, int32_t Q, int blocks,
-                           int pairs) {
+gas_status launch_run_kind(gas_batch *b, const CoreGraph &g, int kind, int32_t nQ, int32_t Q,
+                           int blocks, int pairs) {
   return kind == gas::detail::kBatchBFS
-             ? launch_run<W, gas::detail::kBatchBFS>(b, g, Q, blocks, pairs)
-             : launch_run<W, gas::detail::kBatchSSSP>(b, g, Q, blocks, pairs);
+             ? launch_run<W, gas::detail::kBatchBFS>(b, g, nQ, Q, blocks, pairs)
+             : launch_run<W, gas::detail::kBatchSSSP>(b, g, nQ, Q, blocks, pairs);
 }
 
 int grid_blocks(gas_batch *b, const CoreGraph &g, int kind, int nQ, int W, int pairs) {
@@ -314,10 +315,10 @@ gas_status enqueue_batch(gas_batch *b, const CoreGraph &g, int kind, int32_t nQ,
   const int blocks = grid_blocks(b, g, kind, nQ, W, pairs);
   gas_status st;
   switch (W) {
-    case 1: st = launch_run_kind<1>(b, g, kind, Q, blocks, pairs); break;
-    case 2: st = launch_run_kind<2>(b, g, kind, Q, blocks, pairs); break;
-    case 4: st = launch_run_kind<4>(b, g, kind, Q, blocks, pairs); break;
-    default: st = launch_run_kind<8>(b, g, kind, Q, blocks, pairs); break;
+    case 1: st = launch_run_kind<1>(b, g, kind, nQ, Q, blocks, pairs); break;
+    case 2: st = launch_run_kind<2>(b, g, kind, nQ, Q, blocks, pairs); break;
+    case 4: st = launch_run_kind<4>(b, g, kind, nQ, Q, blocks, pairs); break;
+    default: st = launch_run_kind<8>(b, g, kind, nQ, Q, blocks, pairs); break;
   }
   if (st) return st;
   if (pairs) {  // query-major already: the first nQ rows are the results

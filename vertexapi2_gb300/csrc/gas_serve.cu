@@ -512,6 +512,7 @@ gas_status Server::launch(int l, const std::shared_ptr<Batch> &bp) {
     a.weightsOut = g.bg.weightsOut;
     a.alpha = 10;
     a.nQueries = b.Q;
+    a.nLive = b.nQ;
     a.inSources = g.bg.g.inSrc;
     a.weights = reinterpret_cast<const int32_t *>(g.bg.g.edgeData);
     a.unitV = g.bg.unitV;
