@@ -58,8 +58,14 @@ constexpr int kPullBatch = 2;                 // work units a warp takes at a ti
 // 207 with dense.cuh's pass).
 __host__ __device__ constexpr int pull_mid_lanes(bool wide) { return wide ? 32 : 8; }
 __host__ __device__ constexpr int pull_small_lanes(bool wide) { return wide ? kSmallLanes : 1; }
-// Narrow units a graph needs for the narrow form: two for each warp of the chip.
-constexpr long long kPullNarrowUnits = 2ll * 152 * 28;
+// Narrow units a graph needs for the narrow form: two for each warp of the
+// chip, one for Programs that reduce in any order, whose narrow units are the
+// shorter chains.  Measured at one and at two (run(), us): SSSP, 300,000
+// vertices 414, 472, 200,000 332, 369, 100,000 281, 279; CC 300,000 144, 162;
+// PageRank 400,000 1744, 1598, 200,000 and 1,000,000 the same.
+__host__ __device__ constexpr long long pull_narrow_units(bool anyOrder) {
+  return (anyOrder ? 1ll : 2ll) * 152 * 28;
+}
 constexpr int kHotBytes = GAS_PULL_HOT_BYTES; // shared memory for hot values
 constexpr int kNoEdge = (int)0x80000000;      // stands for no edge: table slot 0, which no vertex has
 

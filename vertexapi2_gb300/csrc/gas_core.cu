@@ -766,7 +766,7 @@ gas_status gas_core_set_graph(gas_core *c, int32_t nV, int32_t nE, const int32_t
     // the slices of the leading dense rounds' kernel; their extents are
     // wanted before the rest of the memory can be sized
     c->pullWide = pl.wide = bins.nChunks + bins.nMid / (32 / gas::detail::pull_mid_lanes(false)) + bins.nSmall / 32 <
-                            gas::detail::kPullNarrowUnits;
+                            gas::detail::pull_narrow_units(c->pullAnyOrder);
     const size_t listed = ((size_t)pull_slice_count(bins, pl.wide) + 1) * sizeof(int2);
     const size_t sliceBytes = (listed + 255) & ~(size_t)255;
     int2 *dSlices = reinterpret_cast<int2 *>(sx.keys[0]);
