@@ -371,6 +371,19 @@ __device__ __forceinline__ bool ppr_combine(const PprArgs &a, int slot, int q, b
   return true;
 }
 
+// The warps that take a long unit and no other: the round lasts as long as
+// the longest of their chains, and short units dealt to them come on top.
+// Where long units would keep more than three quarters of the warps from the
+// short ones, every warp takes both.  20 rounds, with results, us, every warp
+// both -> up to half -> up to three quarters: R-MAT-12, 4 queries 470, 385,
+// 385; R-MAT-16, 16 queries 1962, 1821, 1821, 100 queries 4384, 4424, 3589;
+// 20,000 vertices, 200 queries 3378, 2698, 2698; R-MAT-19, 40 queries 11322,
+// 10239, 10252, 100 queries 20175, 20122, 20138.
+__device__ __forceinline__ long long ppr_long_warps(const PprArgs &a, long long warps) {
+  const long long n = (long long)a.nLong * ppr_slices(a.row);
+  return 4 * n <= 3 * warps ? n : 0;
+}
+
 // The units [0, nLong), a slice of 32 queries each, a warp a slice.
 __device__ __forceinline__ void ppr_long_units(const PprArgs &a, const PprRound &b, PprRing &ring) {
   const int lane = threadIdx.x & 31;
@@ -411,7 +424,8 @@ __device__ __forceinline__ void ppr_round_narrow(const PprArgs &a, int r, PprRin
     ppr_long_units(a, b, ring);
     first = a.nLong;
   }
-  for (long long base = first + gw * G; base < a.nUnits; base += warps * G) {
+  const long long busy = QP >= 4 ? ppr_long_warps(a, warps) : 0;
+  for (long long base = first + (gw - busy) * G; gw >= busy && base < a.nUnits; base += (warps - busy) * G) {
     const long long u = base + grp;
     const int4 un = u < a.nUnits ? __ldg(a.unit + u) : make_int4(-1, 0, 0, -1);
     const int v = un.x, slot = un.w;
@@ -459,7 +473,8 @@ __device__ __forceinline__ void ppr_round_wide(const PprArgs &a, int r, PprRing 
   const long long gw = (long long)(threadIdx.x / 32) * gridDim.x + blockIdx.x;
   ppr_long_units(a, b, ring);
   const int grp = lane / L, j = lane % L;
-  for (long long base = a.nLong + gw * G; base < a.nUnits; base += warps * G) {
+  const long long busy = ppr_long_warps(a, warps);
+  for (long long base = a.nLong + (gw - busy) * G; gw >= busy && base < a.nUnits; base += (warps - busy) * G) {
     const long long u = base + grp;
     const int4 un = u < a.nUnits ? __ldg(a.unit + u) : make_int4(-1, 0, 0, -1);
     const int v = un.x;
