@@ -205,6 +205,7 @@ struct gas_core_s {
   // layout of the leading dense rounds' kernel (pull.cuh), kept when the
   // Program's source values have pullEntry > 0 bytes
   int32_t pullEntry = 0;
+  bool pullKept = false;  // the graph holds that layout's records (memory allowed it)
   bool pullQuadEd = false;      // its gathers read 4-byte edge data
   bool pullAnyOrder = false;    // its reductions may take any order
   bool pullWide = false;        // this graph's layout has more lanes a vertex
@@ -347,7 +348,7 @@ size_t carve_arena(gas_core *c, unsigned char *base, bool edgeMap, int32_t maxHu
   bytes(&c->valt, (size_t)c->vertexBytes * V);
   take(&c->retBits, 4 * 3 * (size_t)c->bitWords);
   take(&c->bins, 4 * V);
-  if (c->pullEntry > 0) {
+  if (c->pullKept) {
     take(&c->slotOf, 4 * V);
     take(&c->hotVertex, GAS_PULL_HOT_BYTES);
     take(&c->pullRec, 16 * V);
@@ -649,6 +650,11 @@ gas_status gas_core_set_graph(gas_core *c, int32_t nV, int32_t nE, const int32_t
   const size_t sortBytes = sort_scratch_bytes(nV, nE, nullptr, nullptr);
   unsigned char *work = nullptr;
   cudaError_t e = cudaMalloc((void **)&work, 256 + 2 * listBytes + edBytes + sortBytes);
+  if (e == cudaErrorMemoryAllocation && c->arena) {  // the previous graph's memory makes room
+    cudaGetLastError();
+    free_graph(c);
+    e = cudaMalloc((void **)&work, 256 + 2 * listBytes + edBytes + sortBytes);
+  }
   if (e != cudaSuccess) return give_up(cuda_fail(e, "setGraph edge list upload"));
   struct Release {
     unsigned char *p;
@@ -693,12 +699,19 @@ gas_status gas_core_set_graph(gas_core *c, int32_t nV, int32_t nE, const int32_t
   const int32_t maxHubs = nE / (gas::detail::kChunkEdges + 1);
   const int32_t maxChunks = nE / gas::detail::kChunkEdges + maxHubs;
 
-  const size_t need = carve_arena(c, nullptr, edgeMap, maxHubs, maxChunks);
+  c->pullKept = c->pullEntry > 0;
+  size_t need = carve_arena(c, nullptr, edgeMap, maxHubs, maxChunks);
   if (c->arenaBytes < need || c->arenaBytes / 4 > need) {  // too small, or mostly idle
     if (c->arena) cudaFree(c->arena);
     c->arena = nullptr;
     c->arenaBytes = 0;
-    A(cudaMalloc((void **)&c->arena, need));
+    e = cudaMalloc((void **)&c->arena, need);
+    if (e == cudaErrorMemoryAllocation && c->pullKept) {  // a graph that fits without the layout
+      cudaGetLastError();
+      c->pullKept = false;
+      need = carve_arena(c, nullptr, edgeMap, maxHubs, maxChunks);
+      e = cudaMalloc((void **)&c->arena, need);
+    }
     if (e != cudaSuccess) return give_up(cuda_fail(e, "setGraph device allocation"));
     c->arenaBytes = need;
   }
@@ -723,7 +736,7 @@ gas_status gas_core_set_graph(gas_core *c, int32_t nV, int32_t nE, const int32_t
   HotInfo *dHot = reinterpret_cast<HotInfo *>(dCounts + 1);
   A(cudaMemsetAsync(dHot, 0, sizeof(HotInfo), c->stream));
   PullLayout pl = {c->slotOf, c->hotVertex, c->pullRec, c->chunkRec, c->pullAnyOrder, false};
-  if (st == GAS_OK && e == cudaSuccess && c->pullEntry > 0)
+  if (st == GAS_OK && e == cudaSuccess && c->pullKept)
     st = device_pull_records(c->stream, nV, c->inOff, c->outOff, c->bins, hubs, dCounts, maxChunks,
                              gas::detail::pull_hot_capacity(c->pullEntry), pl, dHot, sx);
   if (st) return give_up(st);
@@ -762,7 +775,7 @@ gas_status gas_core_set_graph(gas_core *c, int32_t nV, int32_t nE, const int32_t
   c->binTiny = c->binSmall + bins.nSmall;
   c->nChunks = bins.nChunks;
   c->nChunkVertices = bins.nHub;
-  if (c->pullEntry > 0) {
+  if (c->pullKept) {
     // the slices of the leading dense rounds' kernel; their extents are
     // wanted before the rest of the memory can be sized
     c->pullWide = pl.wide = bins.nChunks + bins.nMid / (32 / gas::detail::pull_mid_lanes(false)) + bins.nSmall / 32 <
@@ -780,17 +793,23 @@ gas_status gas_core_set_graph(gas_core *c, int32_t nV, int32_t nE, const int32_t
       if (c->pullMem) cudaFree(c->pullMem);
       c->pullMem = nullptr;
       c->pullBytes = 0;
-      A(cudaMalloc((void **)&c->pullMem, want));
-      if (e != cudaSuccess) return give_up(cuda_fail(e, "setGraph device allocation"));
-      c->pullBytes = want;
+      if (cudaMalloc((void **)&c->pullMem, want) != cudaSuccess) {
+        cudaGetLastError();
+        c->pullMem = nullptr;
+        c->pullKept = false;  // the main kernel runs every round
+      } else {
+        c->pullBytes = want;
+      }
     }
-    c->pullSlices = reinterpret_cast<int2 *>(c->pullMem);
-    c->pullIds = reinterpret_cast<int4 *>(c->pullMem + sliceBytes);
-    c->pullEds = eds ? reinterpret_cast<int4 *>(c->pullMem + sliceBytes + idBytes) : nullptr;
-    if (nV > 0) A(cudaMemcpyAsync(c->pullSlices, dSlices, listed, cudaMemcpyDeviceToDevice, c->stream));
-    st = device_pull_fill(c->stream, bins, pl, c->pullSlices, c->inSrc, static_cast<const int32_t *>(c->ed),
-                          c->pullIds, c->pullEds);
-    if (st) return give_up(st);
+    if (c->pullKept) {
+      c->pullSlices = reinterpret_cast<int2 *>(c->pullMem);
+      c->pullIds = reinterpret_cast<int4 *>(c->pullMem + sliceBytes);
+      c->pullEds = eds ? reinterpret_cast<int4 *>(c->pullMem + sliceBytes + idBytes) : nullptr;
+      if (nV > 0) A(cudaMemcpyAsync(c->pullSlices, dSlices, listed, cudaMemcpyDeviceToDevice, c->stream));
+      st = device_pull_fill(c->stream, bins, pl, c->pullSlices, c->inSrc, static_cast<const int32_t *>(c->ed),
+                            c->pullIds, c->pullEds);
+      if (st) return give_up(st);
+    }
     A(cudaStreamSynchronize(c->stream));
     if (e != cudaSuccess) return give_up(cuda_fail(e, "setGraph build"));
   }
