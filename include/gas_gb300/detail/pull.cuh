@@ -16,11 +16,12 @@
 //   * the values of the graph's hot sources -- the vertices of highest
 //     out-degree, which hold 59 % (R-MAT-22) to 76 % (R-MAT-20) of the edges
 //     -- and their frontier bits are in shared memory, where 32 random reads
-//     take about 4 cycles: one CTA of 1,024 threads per SM, filled from a
-//     compact array at the start of a round (29 MB from L2 over the chip).
+//     take about 4 cycles: one CTA of 768 to 1,024 threads per SM, filled from
+//     a compact array at the start of a round (at most 20 MB from L2 over the
+//     chip).
 //     pullIds holds a hot source as its table slot;
 //   * bits of cold sources are tested only for vertices that no hot
-//     in-neighbour has made active;
+//     in-neighbour has made active (the wide form tests them all at once);
 //   * Programs that say gatherFromSource have gatherMap evaluated once per
 //     source and round instead of once per edge (PageRank: an IEEE division,
 //     and 4 bytes a gather instead of 8), and their vertex data updated in
