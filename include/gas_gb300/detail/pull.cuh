@@ -121,6 +121,37 @@ struct PullThreads {
 // The table's entries for values of `bytes` bytes: whole bitmap words.
 __host__ __device__ constexpr int pull_hot_capacity(int bytes) { return kHotBytes / bytes / 128 * 128; }
 
+// The hot vertices: as many whole degree classes of at least kHotMinOut as fit
+// `most` slots.  deg(k): the out-degree of the k-th of nV vertices sorted by
+// min(out-degree, kHotDegreeCap), the largest first (the sort's keys have 16
+// bits; equal keys come by vertex id).  The cut is made on those capped
+// degrees alone, so that the first `count` vertices are the ones of
+// out-degree >= minOut: pull_finish tells a hot vertex by its degree.  Where
+// more than `most` reach the cap, none is hot.
+constexpr int kHotDegreeCap = 65535;
+struct HotCut {
+  int count, minOut;
+};
+template <class Deg>
+__host__ __device__ inline HotCut hot_cut(const Deg &deg, int nV, int most, int least) {
+  auto capped = [&](int k) {
+    const int d = deg(k);
+    return d < kHotDegreeCap ? d : kHotDegreeCap;
+  };
+  int minOut = nV > most ? capped(most) + 1 : 1;
+  if (minOut > kHotDegreeCap) return {0, 0x7fffffff};
+  if (minOut < least) minOut = least;
+  int lo = 0, hi = nV < most ? nV : most;  // the first k of a smaller degree
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (capped(mid) >= minOut)
+      lo = mid + 1;
+    else
+      hi = mid;
+  }
+  return {lo, minOut};
+}
+
 // Shared memory of a table of nHot slots (slot 0 included): the values, then
 // their bits.  A launch takes what its graph's table needs; what it leaves is
 // L1 for the other gathers.

@@ -395,7 +395,8 @@ __global__ void hub_chunks_kernel(const int32_t *bins, const int32_t *inOff,
 __global__ void out_degree_key_kernel(const int32_t *outOff, int32_t nV, uint32_t *key) {
   for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < nV;
        v += (long long)gridDim.x * blockDim.x)
-    key[v] = 65535u - (uint32_t)min(outOff[v + 1] - outOff[v], 65535);
+    key[v] = (uint32_t)(gas::detail::kHotDegreeCap -
+                        min(outOff[v + 1] - outOff[v], gas::detail::kHotDegreeCap));
 }
 
 // The least out-degree of a hot vertex.  Each slot costs every SM its share of
@@ -409,27 +410,18 @@ __global__ void out_degree_key_kernel(const int32_t *outOff, int32_t nV, uint32_
 // with higher degrees than these.
 constexpr int kHotMinOut = 64;
 
-// order: the vertices by falling out-degree.  The hot ones: as many whole
-// degree classes of at least kHotMinOut as fit `capacity` slots, of which the
-// first stays unused (one block).
+// order: the vertices by falling out-degree (out_degree_key_kernel).  The hot
+// ones (hot_cut) take the slots below `capacity`, of which the first stays
+// unused (one block).
 __global__ void hot_pick_kernel(const uint32_t *order, const int32_t *outOff, int32_t nV, int32_t capacity,
                                 gas::internal::HotInfo *info, int32_t *hotVertex) {
   __shared__ int sHot;
-  const int most = capacity - 1;
-  auto deg = [&](int k) { return outOff[order[k] + 1] - outOff[order[k]]; };
   if (threadIdx.x == 0) {
-    const int minOut = max(kHotMinOut, nV > most ? deg(most) + 1 : 1);
-    int lo = 0, hi = min(nV, most);  // the first k of a smaller degree
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      if (deg(mid) >= minOut)
-        lo = mid + 1;
-      else
-        hi = mid;
-    }
-    sHot = lo;
-    info->nHot = lo + 1;
-    info->minOut = minOut;
+    const gas::detail::HotCut cut = gas::detail::hot_cut(
+        [&](int k) { return outOff[order[k] + 1] - outOff[order[k]]; }, nV, capacity - 1, kHotMinOut);
+    sHot = cut.count;
+    info->nHot = cut.count + 1;
+    info->minOut = cut.minOut;
   }
   __syncthreads();
   for (int k = threadIdx.x; k < sHot; k += blockDim.x) hotVertex[k + 1] = (int32_t)order[k];
