@@ -107,7 +107,11 @@ typedef struct {
 
 /* Arguments of one persistent run() launch: every round of gather/apply,
  * commit + scatter/activate and frontier swap in a single cooperative
- * kernel, the phases separated by bounded grid barriers. */
+ * kernel, the phases separated by bounded grid barriers.
+ *
+ * The kernels that read it are compiled into the caller's binary with this
+ * header, so a field keeps its place and its meaning: new ones go to the end,
+ * and one that newer kernels have no use for is still filled in and heeded. */
 typedef struct {
   gas_gather_args g;          /* graph, vertex data, carry arrays, ...      */
   const int32_t *outDests;    /* CSR destinations [nEdges]                  */
@@ -143,6 +147,9 @@ typedef struct {
                                  ret/out-edges, dense work units taken, unused */
   int32_t denseAlpha;         /* next round dense when out-edges*alpha > E; 0 = never */
   int32_t allActive;          /* round 0 is every vertex (setActive(0, V)) */
+  int32_t *vcurOut;           /* 1 when the final vertex data is in vertexAlt: the
+                                 library copies it then (the present kernels leave
+                                 it in vertexData, and 0 here) */
   /* degree bins of the dense pass (fixed per graph): warp work units are
    * [large-vertex chunks | warp-per-vertex | 8-lane groups | thread-per-vertex] */
   const int32_t *binMid;      /* in-degree 65..1024: one warp each          */

@@ -90,8 +90,8 @@ struct ListCtl {
 struct Ctl {
   unsigned err;     // device error bits (kept across set_active)
   int32_t rounds;   // rounds executed by the last persistent run
-  int32_t denseEnd; // 1 when that run stopped before a dense round (gas_run_args::denseEndOut)
-  int32_t pad;
+  int32_t vcur;     // 1 when its result is in the alternate buffer (gas_run_args::vcurOut)
+  int32_t denseEnd; // 1 when it stopped before a dense round (gas_run_args::denseEndOut)
   ListCtl f[2];     // frontier lists
   ListCtl s[2];     // scatter lists
   unsigned tile[2];
@@ -103,7 +103,7 @@ struct Ctl {
 // The part of Ctl that the host reads, as it lies there.
 struct CtlHead {
   unsigned err;
-  int32_t rounds, denseEnd, pad;
+  int32_t rounds, vcur, denseEnd;
   ListCtl f[2];
 };
 
@@ -1262,7 +1262,7 @@ gas_status gas_core_run_persistent(gas_core *c, int32_t maxIters, int32_t haveGa
     seg(&c->ctl->s[0], sizeof(c->ctl->s));
     seg(&c->ctl->f[c->cur ^ 1], sizeof(ListCtl));
     seg(&c->ctl->bar[0], sizeof(c->ctl->bar));
-    seg(&c->ctl->rounds, 2 * sizeof(int32_t));
+    seg(&c->ctl->rounds, 3 * sizeof(int32_t));  // and vcur, denseEnd
     seg(round_bits(c, ra.stampBase), sizeof(uint32_t) * std::max(c->bitWords, 1));
     if (c->frontBits)
       seg(c->frontBits + (size_t)((unsigned)(ra.stampBase + 1) % 3u) * c->bitWords,
@@ -1318,6 +1318,7 @@ gas_status gas_core_run_persistent(gas_core *c, int32_t maxIters, int32_t haveGa
   ra.denseAlpha = ra.edgeScatter ? 0 : c->denseAlpha;  // Program::scatter walks list rounds
   ra.allActive =
       (c->rangeMode && c->rstart == 0 && c->rcount == c->nV && ra.denseAlpha > 0) ? 1 : 0;
+  ra.vcurOut = &c->ctl->vcur;
   ra.resume = &c->ctl->resume[0];
   ra.denseEndOut = &c->ctl->denseEnd;
 
@@ -1335,6 +1336,10 @@ gas_status gas_core_run_persistent(gas_core *c, int32_t maxIters, int32_t haveGa
   if (e != cudaSuccess) return cuda_fail(e, "persistent run");
   const CtlHead head = *c->head;
   const int32_t rounds = head.rounds;
+  if (head.vcur) {  // a kernel that leaves the result in the alternate buffer
+    e = cudaMemcpyAsync(c->vd, c->valt, (size_t)c->vertexBytes * c->nV, cudaMemcpyDeviceToDevice, c->stream);
+    if (e != cudaSuccess) return cuda_fail(e, "persistent run copy-back");
+  }
   cudaEventElapsedTime(&c->lastMs, c->t0, c->t1);
   const int32_t R = rounds;
   if (R & 1) {
