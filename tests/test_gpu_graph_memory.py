@@ -1,0 +1,138 @@
+"""set_graph near the end of device memory: a graph that fits on its own is
+taken, whatever an engine keeps from its last graph, whether or not the layout
+of the leading dense rounds would fit beside it, and with no more than its own
+arrays or its adjacency and the build's working memory."""
+from __future__ import annotations
+
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from vertexapi2_gb300 import GASEngine
+from vertexapi2_gb300 import programs as P
+from vertexapi2_gb300._lib import PROGRAM_CC, load
+
+pytestmark = pytest.mark.gpu
+
+MB = 1 << 20
+SLACK = 16 * MB  # the device allocates in blocks of 2 MB
+LEFT = 4096 * MB
+
+
+class Memory:
+    """Leaves a chosen number of free bytes."""
+
+    def __init__(self, torch):
+        self.torch = torch
+        torch.zeros(1, device="cuda")
+        torch.cuda.synchronize()
+        self.fine = None
+        self.coarse = self.block(self.free() - LEFT)
+
+    def free(self):
+        return self.torch.cuda.mem_get_info(0)[0]
+
+    def block(self, n):
+        return self.torch.empty(max(n, 1) // (2 * MB) * 2 * MB, dtype=self.torch.uint8, device="cuda")
+
+    def leave(self, n):
+        self.release()
+        self.fine = self.block(self.free() - n)
+        assert abs(self.free() - n) <= 4 * MB
+
+    def release(self):
+        self.fine = None
+        self.torch.cuda.empty_cache()
+
+
+@pytest.fixture
+def memory(gpu):
+    torch = pytest.importorskip("torch")
+    if torch.cuda.mem_get_info(0)[0] < LEFT + 64 * MB:
+        pytest.skip("device memory in use")
+    m = Memory(torch)
+    yield m
+    m.coarse = None
+    m.release()
+
+
+def i32(a):
+    return a.ctypes.data_as(C.POINTER(C.c_int32))
+
+
+def bare_set_graph(nv, s, d, vertex_bytes=4):
+    """Status of set_graph on an engine that keeps no layout, and the bytes it
+    holds then."""
+    import torch
+    lib, core = load(), C.c_void_p()
+    assert lib.gas_core_create(0, None, C.byref(core)) == 0
+    free = torch.cuda.mem_get_info(0)[0]
+    st = lib.gas_core_set_graph(core, nv, s.size, i32(s), i32(d), None, 0, vertex_bytes, 4)
+    held = free - torch.cuda.mem_get_info(0)[0]
+    lib.gas_core_destroy(core)
+    return st, held
+
+
+def least_free(memory, nv, s, d):
+    """Free bytes (to 2 MB) in which the graph fits without the layout."""
+    lo, hi = 0, LEFT // (2 * MB)
+    while lo + 1 < hi:
+        mid = (lo + hi) // 2
+        memory.leave(mid * 2 * MB)
+        if bare_set_graph(nv, s, d)[0] == 0:
+            hi = mid
+        else:
+            lo = mid
+    memory.release()
+    return hi * 2 * MB
+
+
+def random_graph(nv, ne, seed):
+    rng = np.random.default_rng(seed)
+    return rng.integers(0, nv, ne, dtype=np.int32), rng.integers(0, nv, ne, dtype=np.int32)
+
+
+def ring(nv):
+    """Degrees of 2: a graph of the fused rounds."""
+    v = np.arange(nv, dtype=np.int32)
+    n = np.roll(v, -1)
+    return np.concatenate([v, n]), np.concatenate([n, v])
+
+
+def labels(e, nv, s, d):
+    vd = P.cc_init(nv)
+    e.set_graph(nv, vd, s, d)
+    e.set_active(0, nv)
+    e.run(4)
+    e.get_results()
+    return vd
+
+
+@pytest.mark.parametrize("kind", ["random", "ring"])
+@pytest.mark.parametrize("before", ["new engine", "other graph before"])
+def test_a_graph_that_fits_is_taken(memory, kind, before):
+    nv, (s, d) = (1 << 20, random_graph(1 << 20, 1 << 24, 1)) if kind == "random" else (3 << 20, ring(3 << 20))
+    other = random_graph(1 << 19, 3 << 23, 2)
+    with GASEngine(PROGRAM_CC) as e:
+        ref = labels(e, nv, s, d)
+    least = least_free(memory, nv, s, d)
+    with GASEngine(PROGRAM_CC) as e:
+        held = memory.free()
+        if before != "new engine":
+            labels(e, 1 << 19, *other)
+        held -= memory.free()
+        memory.leave(least + SLACK - held)
+        assert np.array_equal(labels(e, nv, s, d), ref)
+        assert np.array_equal(labels(e, nv, s, d), ref)
+        memory.release()
+        assert np.array_equal(labels(e, nv, s, d), ref)
+
+
+def test_state_may_take_the_build_memory(memory):
+    nv = 1 << 20
+    s, d = random_graph(nv, 1 << 24, 3)
+    st, held = bare_set_graph(nv, s, d, 256)
+    assert st == 0
+    memory.leave(held + SLACK)
+    assert bare_set_graph(nv, s, d, 256)[0] == 0

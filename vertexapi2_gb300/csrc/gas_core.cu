@@ -160,6 +160,14 @@ __global__ void zero_segments_kernel(ZeroSegments z) {
       z.ptr[s][i] = 0u;
 }
 
+// Device memory that outlives a graph: the next one reuses it when it fits.  A
+// cudaMalloc / cudaFree pair costs about 100 us, and a graph has some fifty
+// arrays.
+struct Block {
+  unsigned char *p = nullptr;
+  size_t bytes = 0;
+};
+
 struct gas_core_s {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -182,11 +190,10 @@ struct gas_core_s {
   bool fusedRounds = true;      // one-phase rounds when every degree is <= 8
   bool edgeScatterOn = false;   // keep csr2csc and run scatter-capable rounds
   bool edgeScatterReady = false;  // a scatter list awaits the Program's scatter
-  // One allocation holds the arrays whose sizes follow from V and E (the
-  // next set_graph reuses it when it fits): a cudaMalloc / cudaFree pair
-  // costs about 100 us, and there are some fifty arrays.
-  unsigned char *arena = nullptr;
-  size_t arenaBytes = 0;
+  // adjacency, edge data, degree bins; vertex-sized state and lists; the
+  // fused rounds' arrays; the leading dense rounds' layout (records and
+  // tables, then slices), which a graph can do without
+  Block graphMem, stateMem, fusedMem, layoutMem, sliceMem;
   int32_t *inOff = nullptr, *inSrc = nullptr, *outOff = nullptr, *outDst = nullptr;
   void *ed = nullptr;
   void *vd = nullptr, *vnew = nullptr, *vsaved = nullptr, *valt = nullptr;
@@ -205,12 +212,9 @@ struct gas_core_s {
   // layout of the leading dense rounds' kernel (pull.cuh), kept when the
   // Program's source values have pullEntry > 0 bytes
   int32_t pullEntry = 0;
-  bool pullKept = false;  // the graph holds that layout's records (memory allowed it)
   bool pullQuadEd = false;      // its gathers read 4-byte edge data
   bool pullAnyOrder = false;    // its reductions may take any order
   bool pullWide = false;        // this graph's layout has more lanes a vertex
-  unsigned char *pullMem = nullptr;  // slices | ids | edge data, reused as the arena is
-  size_t pullBytes = 0;
   int2 *pullSlices = nullptr;
   int4 *pullIds = nullptr, *pullEds = nullptr;
   int32_t *slotOf = nullptr, *hotVertex = nullptr;
@@ -272,20 +276,49 @@ static uint32_t *round_bits(gas_core_s *c, int32_t stamp) {
 
 namespace {
 
-// Drops the graph; the arena stays for the next one unless `all`.
+void give_back(Block &b) {
+  if (b.p) cudaFree(b.p);
+  b = Block();
+}
+
+// At least `need` bytes, the ones there already unless they are too few or
+// mostly idle.
+cudaError_t reserve(Block &b, size_t need) {
+  if (b.bytes >= need && b.bytes / 4 <= need) return cudaSuccess;
+  give_back(b);
+  const cudaError_t e = cudaMalloc((void **)&b.p, need);
+  if (e == cudaSuccess)
+    b.bytes = need;
+  else
+    b.p = nullptr;
+  return e;
+}
+
+// No layout of the leading dense rounds: the main kernel runs every round.
+void forget_layout(gas_core *c) {
+  c->pullSlices = nullptr;
+  c->pullIds = c->pullEds = c->pullRec = c->chunkRec = nullptr;
+  c->slotOf = c->hotVertex = nullptr;
+  c->hotVal[0] = c->hotVal[1] = nullptr;
+  c->hotBits = nullptr;
+  c->nHot = c->hotMinOut = c->nZero = 0;
+}
+void drop_layout(gas_core *c) {
+  forget_layout(c);
+  give_back(c->layoutMem);
+  give_back(c->sliceMem);
+}
+
+// Drops the graph; its blocks stay for the next one unless `all`.
 void free_graph(gas_core *c, bool all = true) {
-  void *ptrs[] = {c->vsaved, c->frontBits, c->csrPerm, c->fcell, c->ellIn, c->ellOut, c->ellEd};
-  for (void *p : ptrs)
-    if (p) cudaFree(p);
-  if (all && c->arena) {
-    cudaFree(c->arena);
-    c->arena = nullptr;
-    c->arenaBytes = 0;
-  }
-  if (all && c->pullMem) {
-    cudaFree(c->pullMem);
-    c->pullMem = nullptr;
-    c->pullBytes = 0;
+  if (c->vsaved) cudaFree(c->vsaved);
+  if (c->csrPerm) cudaFree(c->csrPerm);
+  forget_layout(c);
+  if (all) {
+    drop_layout(c);
+    give_back(c->graphMem);
+    give_back(c->stateMem);
+    give_back(c->fusedMem);
   }
   c->cscPerm = c->csrPerm = nullptr;
   c->csr2csc = nullptr;
@@ -301,12 +334,6 @@ void free_graph(gas_core *c, bool all = true) {
   c->chunkVertex = c->chunkBegin = c->chunkFirst = c->chunkCount = c->chunkSlot = nullptr;
   c->chunkArrive = c->chunkFlags = nullptr;
   c->chunkVal = nullptr;
-  c->pullSlices = nullptr;
-  c->pullIds = c->pullEds = c->pullRec = c->chunkRec = nullptr;
-  c->slotOf = c->hotVertex = nullptr;
-  c->hotVal[0] = c->hotVal[1] = nullptr;
-  c->hotBits = nullptr;
-  c->nHot = c->hotMinOut = c->nZero = 0;
   c->nMid = c->nSmall = c->nTiny = c->nChunks = c->nChunkVertices = 0;
   for (int k = 0; k < 2; ++k) {
     c->fvid[k] = c->fpre[k] = c->fbeg[k] = c->fsplit[k] = nullptr;
@@ -321,50 +348,56 @@ void free_graph(gas_core *c, bool all = true) {
   c->haveGraph = false;
 }
 
-// Lays the V- and E-sized arrays out in the arena at `base` (null: only the
-// size is wanted), each on a 256-byte boundary.
-size_t carve_arena(gas_core *c, unsigned char *base, bool edgeMap, int32_t maxHubs, int32_t maxChunks) {
+// Lays arrays out from `base`, each on a 256-byte boundary (null: only the
+// size is wanted, the arrays become null).
+struct Carver {
+  unsigned char *base;
   size_t used = 0;
-  auto take = [&](auto **p, size_t bytes) {
-    *p = reinterpret_cast<std::remove_reference_t<decltype(**p)> *>(base + used);
+  template <class T>
+  void operator()(T **p, size_t bytes) {
+    *p = base ? reinterpret_cast<T *>(base + used) : nullptr;
     used += (std::max<size_t>(bytes, 1) + 255) & ~(size_t)255;
-  };
-  auto bytes = [&](void **p, size_t n) {
-    *p = base + used;
-    used += (std::max<size_t>(n, 1) + 255) & ~(size_t)255;
-  };
-  const size_t V = (size_t)c->nV, E = (size_t)c->nE, gb = (size_t)((c->gatherBytes + 15) / 16 * 16);
+  }
+  void operator()(void **p, size_t bytes) {
+    unsigned char *q;
+    (*this)(&q, bytes);
+    *p = q;
+  }
+};
+
+// What the build writes: adjacency, edge data, degree bins, chunks.
+size_t carve_graph(gas_core *c, unsigned char *base, bool edgeMap, int32_t maxChunks) {
+  Carver take{base};
+  const size_t V = (size_t)c->nV, E = (size_t)c->nE;
   take(&c->inOff, 4 * (V + 1));
   // whole 16-byte quads: the dense pass reads source ids (and 4-byte edge
   // data) four at a time, up to the quad that holds a vertex's last edge
   take(&c->inSrc, 4 * (E + 4));
   take(&c->outOff, 4 * (V + 1));
   take(&c->outDst, 4 * E);
-  if (c->edgeBytes > 0) bytes(&c->ed, (size_t)c->edgeBytes * (E + 4));
+  if (c->edgeBytes > 0) take(&c->ed, (size_t)c->edgeBytes * (E + 4));
   if (c->edgeBytes > 0) take(&c->cscPerm, 4 * E);
   if (edgeMap) take(&c->csr2csc, 4 * E);
-  bytes(&c->vd, (size_t)c->vertexBytes * V);
-  bytes(&c->vnew, (size_t)c->vertexBytes * V);
-  bytes(&c->valt, (size_t)c->vertexBytes * V);
-  take(&c->retBits, 4 * 3 * (size_t)c->bitWords);
   take(&c->bins, 4 * V);
-  if (c->pullKept) {
-    take(&c->slotOf, 4 * V);
-    take(&c->hotVertex, GAS_PULL_HOT_BYTES);
-    take(&c->pullRec, 16 * V);
-    take(&c->chunkRec, 16 * (size_t)maxChunks);
-    bytes(&c->hotVal[0], GAS_PULL_HOT_BYTES);
-    bytes(&c->hotVal[1], GAS_PULL_HOT_BYTES);
-    take(&c->hotBits, 4 * 3 * (size_t)kHotWords);
-  }
   take(&c->chunkVertex, 4 * (size_t)maxChunks);
   take(&c->chunkBegin, 4 * (size_t)maxChunks);
   take(&c->chunkFirst, 4 * (size_t)maxChunks);
   take(&c->chunkCount, 4 * (size_t)maxChunks);
   take(&c->chunkSlot, 4 * (size_t)maxChunks);
+  return take.used;
+}
+
+// What only the rounds use.
+size_t carve_state(gas_core *c, unsigned char *base, int32_t maxHubs, int32_t maxChunks) {
+  Carver take{base};
+  const size_t V = (size_t)c->nV, gb = (size_t)((c->gatherBytes + 15) / 16 * 16);
+  take(&c->vd, (size_t)c->vertexBytes * V);
+  take(&c->vnew, (size_t)c->vertexBytes * V);
+  take(&c->valt, (size_t)c->vertexBytes * V);
+  take(&c->retBits, 4 * 3 * (size_t)c->bitWords);
   take(&c->chunkFlags, 4 * (size_t)maxChunks);
   take(&c->chunkArrive, 4 * (size_t)maxHubs);
-  bytes(&c->chunkVal, gb * maxChunks);
+  take(&c->chunkVal, gb * maxChunks);
   for (int k = 0; k < 2; ++k) {
     take(&c->fvid[k], 4 * V);
     take(&c->fpre[k], 4 * V);
@@ -377,11 +410,37 @@ size_t carve_arena(gas_core *c, unsigned char *base, bool edgeMap, int32_t maxHu
   }
   take(&c->rsplit, 4 * (size_t)c->maxGatherTiles);
   take(&c->mark, 4 * V);
-  bytes(&c->carryVal, gb * c->maxGatherTiles);
+  take(&c->carryVal, gb * c->maxGatherTiles);
   take(&c->carryFlag, 4 * (size_t)c->maxGatherTiles);
   take(&c->ctl, sizeof(Ctl));
   take(&c->stats, 16 * (size_t)kMaxRounds);
-  return used;
+  return take.used;
+}
+
+// The fused rounds' cells, rows of ellWidth entries and active-set bitmaps.
+size_t carve_fused(gas_core *c, unsigned char *base) {
+  Carver take{base};
+  const size_t V = (size_t)std::max(c->nV, 1), cells = V * c->ellWidth;
+  take(&c->fcell, (size_t)GAS_FUSED_CELL_BYTES(c->vertexBytes) * V);
+  take(&c->ellIn, 4 * cells);
+  take(&c->ellOut, 4 * cells);
+  if (c->edgeBytes > 0) take(&c->ellEd, (size_t)c->edgeBytes * cells);
+  take(&c->frontBits, 4 * 3 * (size_t)c->bitWords);
+  return take.used;
+}
+
+// The leading dense rounds' records and tables.
+size_t carve_layout(gas_core *c, unsigned char *base, int32_t maxChunks) {
+  Carver take{base};
+  const size_t V = (size_t)c->nV;
+  take(&c->slotOf, 4 * V);
+  take(&c->hotVertex, GAS_PULL_HOT_BYTES);
+  take(&c->pullRec, 16 * V);
+  take(&c->chunkRec, 16 * (size_t)maxChunks);
+  take(&c->hotVal[0], GAS_PULL_HOT_BYTES);
+  take(&c->hotVal[1], GAS_PULL_HOT_BYTES);
+  take(&c->hotBits, 4 * 3 * (size_t)kHotWords);
+  return take.used;
 }
 
 gas_status set_device(gas_core *c) {
@@ -563,6 +622,235 @@ bool core_graph(gas_core_s *c, CoreGraph *out) {
 }  // namespace internal
 }  // namespace gas
 
+namespace {
+
+// The layout of the leading dense rounds (pull.cuh), from the CSC and the
+// bins, with the build's working memory; without it (c->pullIds null) the main
+// kernel runs every round.
+gas_status build_layout(gas_core *c, const DegreeBins &bins, const HubChunks &hubs, DegreeBins *dCounts,
+                        int32_t maxChunks, const SortScratch &sx) {
+  cudaError_t e = reserve(c->layoutMem, carve_layout(c, nullptr, maxChunks));
+  if (e != cudaSuccess) return cuda_fail(e, "layout of the dense rounds");
+  carve_layout(c, c->layoutMem.p, maxChunks);
+  PullLayout pl = {c->slotOf, c->hotVertex, c->pullRec, c->chunkRec, c->pullAnyOrder, false};
+  HotInfo *dHot = reinterpret_cast<HotInfo *>(dCounts + 1), hot = {0, 0};
+  e = cudaMemsetAsync(dHot, 0, sizeof(HotInfo), c->stream);
+  if (e != cudaSuccess) return cuda_fail(e, "layout of the dense rounds");
+  gas_status st = device_pull_records(c->stream, c->nV, c->inOff, c->outOff, c->bins, hubs, dCounts, maxChunks,
+                                      gas::detail::pull_hot_capacity(c->pullEntry), pl, dHot, sx);
+  if (st) return st;
+  e = cudaMemcpyAsync(&hot, dHot, sizeof(hot), cudaMemcpyDeviceToHost, c->stream);
+  if (e != cudaSuccess) return cuda_fail(e, "layout of the dense rounds");
+  // the slices' extents are wanted before the rest of the memory can be sized
+  c->pullWide = pl.wide = bins.nChunks + bins.nMid / (32 / gas::detail::pull_mid_lanes(false)) + bins.nSmall / 32 <
+                          gas::detail::pull_narrow_units(c->pullAnyOrder);
+  const size_t listed = ((size_t)pull_slice_count(bins, pl.wide) + 1) * sizeof(int2);
+  const size_t sliceBytes = (listed + 255) & ~(size_t)255;
+  int2 *dSlices = reinterpret_cast<int2 *>(sx.keys[0]);
+  long long quads = 0;
+  st = device_pull_slices(c->stream, bins, pl, dSlices, &quads, sx);  // waits
+  if (st) return st;
+  const bool eds = c->pullQuadEd && c->edgeBytes == 4;
+  const size_t idBytes = ((size_t)quads * 16 + 256) & ~(size_t)255;
+  e = reserve(c->sliceMem, sliceBytes + idBytes * (eds ? 2 : 1));
+  if (e != cudaSuccess) return cuda_fail(e, "layout of the dense rounds");
+  c->pullSlices = reinterpret_cast<int2 *>(c->sliceMem.p);
+  c->pullEds = eds ? reinterpret_cast<int4 *>(c->sliceMem.p + sliceBytes + idBytes) : nullptr;
+  int4 *ids = reinterpret_cast<int4 *>(c->sliceMem.p + sliceBytes);
+  e = cudaMemcpyAsync(c->pullSlices, dSlices, listed, cudaMemcpyDeviceToDevice, c->stream);
+  if (e != cudaSuccess) return cuda_fail(e, "layout of the dense rounds");
+  st = device_pull_fill(c->stream, bins, pl, c->pullSlices, c->inSrc, static_cast<const int32_t *>(c->ed), ids,
+                        c->pullEds);
+  if (st) return st;
+  c->pullIds = ids;
+  c->nZero = bins.nZero;
+  c->nHot = hot.nHot;
+  c->hotMinOut = hot.nHot > 1 ? hot.minOut : 0x7fffffff;
+  return GAS_OK;
+}
+
+// set_graph's work.  The graph's own arrays come first, the layout of the
+// leading dense rounds last: it never keeps a graph from fitting, and neither
+// does the build's working memory once the adjacency stands.  On failure the
+// caller frees everything.
+gas_status build_graph(gas_core *c, int32_t nV, int32_t nE, const int32_t *srcs, const int32_t *dsts,
+                       const void *edgeData, int32_t edgeBytes, int32_t vertexBytes, int32_t gatherBytes) {
+  // the edge list, the edge data in edge-list order, the sorts, the bins' counts
+  const size_t listBytes = ((size_t)std::max(nE, 1) * 4 + 255) & ~(size_t)255;
+  const size_t edBytes = ((size_t)edgeBytes * std::max(nE, 1) + 255) & ~(size_t)255;
+  const size_t sortBytes = sort_scratch_bytes(nV, nE, nullptr, nullptr);
+  struct Work {
+    unsigned char *p = nullptr;
+    void release() {
+      if (p) cudaFree(p);
+      p = nullptr;
+    }
+    ~Work() { release(); }
+  } work;
+  cudaError_t e = cudaMalloc((void **)&work.p, 256 + 2 * listBytes + edBytes + sortBytes);
+  if (e != cudaSuccess) {
+    work.p = nullptr;
+    return cuda_fail(e, "setGraph edge list upload");
+  }
+  DegreeBins *dCounts = reinterpret_cast<DegreeBins *>(work.p);
+  int32_t *dS = reinterpret_cast<int32_t *>(work.p + 256);
+  int32_t *dD = reinterpret_cast<int32_t *>(work.p + 256 + listBytes);
+  unsigned char *dEd = work.p + 256 + 2 * listBytes;
+  SortScratch sx;
+  sort_scratch_bytes(nV, nE, &sx, dEd + edBytes);
+  auto A = [&](cudaError_t r) {
+    if (e == cudaSuccess) e = r;
+  };
+
+  // the edge list on the device: id check, then CSC (gather) and CSR
+  // (scatter) by stable radix sorts (gas_graph_build.cu)
+  if (nE > 0) {
+    A(cudaMemcpyAsync(dS, srcs, sizeof(int32_t) * nE, cudaMemcpyHostToDevice, c->stream));
+    A(cudaMemcpyAsync(dD, dsts, sizeof(int32_t) * nE, cudaMemcpyHostToDevice, c->stream));
+    if (edgeBytes > 0)
+      A(cudaMemcpyAsync(dEd, edgeData, (size_t)edgeBytes * nE, cudaMemcpyHostToDevice, c->stream));
+    if (e != cudaSuccess) return cuda_fail(e, "setGraph edge list upload");
+  }
+  EdgeCheck check;
+  gas_status st = device_check_edges(c->stream, nV, nE, dS, dD, work.p, &check);
+  if (st == GAS_OK && check.firstBad >= 0)
+    st = fail(GAS_ERR_INVALID, "edge %lld (%d -> %d) has a vertex id outside [0, %d)", check.firstBad,
+              srcs[check.firstBad], dsts[check.firstBad], nV);
+  if (st) return st;
+
+  c->nV = nV;
+  c->nE = nE;
+  c->edgeBytes = edgeBytes;
+  c->vertexBytes = vertexBytes;
+  c->gatherBytes = gatherBytes;
+  c->maxGatherTiles = (int32_t)(((long long)nV + nE) / GAS_GATHER_TILE + 2);
+  c->maxScatTiles = (int32_t)(((long long)nV + nE) / GAS_SCATTER_TILE + 2);
+  c->bitWords = (nV + 31) / 32;
+  const bool edgeMap = c->edgeScatterOn && edgeBytes > 0;
+  // bounds on the vertices of more than kChunkEdges in-edges and their chunks
+  const int32_t maxHubs = nE / (gas::detail::kChunkEdges + 1);
+  const int32_t maxChunks = nE / gas::detail::kChunkEdges + maxHubs;
+
+  e = reserve(c->graphMem, carve_graph(c, nullptr, edgeMap, maxChunks));
+  if (e != cudaSuccess) return cuda_fail(e, "setGraph device allocation");
+  carve_graph(c, c->graphMem.p, edgeMap, maxChunks);
+  if (c->keepCsrPerm || edgeMap) A(dalloc(&c->csrPerm, (size_t)nE));
+  if (e != cudaSuccess) return cuda_fail(e, "setGraph device allocation");
+  const size_t stateBytes = carve_state(c, nullptr, maxHubs, maxChunks);
+  e = reserve(c->stateMem, stateBytes);
+  const bool tight = e == cudaErrorMemoryAllocation;  // it has to wait for the working memory
+  if (tight) {
+    cudaGetLastError();
+    e = cudaSuccess;
+  }
+  if (e != cudaSuccess) return cuda_fail(e, "setGraph device allocation");
+
+  st = device_build_adjacency(c->stream, nV, nE, dD, dS, check.dstSorted, c->inOff, c->inSrc, c->cscPerm, sx);
+  if (st == GAS_OK)
+    st = device_build_adjacency(c->stream, nV, nE, dS, dD, check.srcSorted, c->outOff, c->outDst,
+                                c->csrPerm, sx);
+  if (st == GAS_OK && edgeMap)
+    st = device_csr_to_csc(c->stream, nE, c->cscPerm, c->csrPerm, c->csr2csc);
+  if (st == GAS_OK && edgeBytes > 0 && nE > 0)
+    st = device_gather_bytes(c->stream, dEd, c->cscPerm, nE, edgeBytes, c->ed);
+  // in-degree bins of the dense pass, heaviest first: the order in which it
+  // hands out work units
+  A(cudaMemsetAsync(dCounts, 0, sizeof(DegreeBins), c->stream));
+  const HubChunks hubs = {c->chunkVertex, c->chunkBegin, c->chunkFirst, c->chunkCount, c->chunkSlot};
+  if (st == GAS_OK && e == cudaSuccess)
+    st = device_degree_bins(c->stream, nV, c->inOff, c->outOff, maxHubs, c->bins, hubs, dCounts, sx);
+  if (st) return st;
+  auto clear_state = [&] {
+    carve_state(c, c->stateMem.p, maxHubs, maxChunks);
+    A(cudaMemsetAsync(c->mark, 0, sizeof(int32_t) * std::max(nV, 1), c->stream));
+    A(cudaMemsetAsync(c->retBits, 0, sizeof(uint32_t) * 3 * std::max(c->bitWords, 1), c->stream));
+    A(cudaMemsetAsync(c->chunkArrive, 0, sizeof(unsigned) * std::max(maxHubs, 1), c->stream));
+    A(cudaMemsetAsync(c->carryFlag, 0, sizeof(unsigned) * c->maxGatherTiles, c->stream));
+    A(cudaMemsetAsync(c->ctl, 0, sizeof(Ctl), c->stream));
+    A(cudaMemsetAsync(c->vd, 0, (size_t)vertexBytes * std::max(nV, 1), c->stream));
+  };
+  if (!tight) clear_state();
+  c->hInOff.resize((size_t)nV + 1);
+  c->hOutOff.resize((size_t)nV + 1);
+  DegreeBins bins;
+  A(cudaMemcpyAsync(c->hInOff.data(), c->inOff, sizeof(int32_t) * ((size_t)nV + 1),
+                    cudaMemcpyDeviceToHost, c->stream));
+  A(cudaMemcpyAsync(c->hOutOff.data(), c->outOff, sizeof(int32_t) * ((size_t)nV + 1),
+                    cudaMemcpyDeviceToHost, c->stream));
+  A(cudaMemcpyAsync(&bins, dCounts, sizeof(bins), cudaMemcpyDeviceToHost, c->stream));
+  A(cudaStreamSynchronize(c->stream));
+  if (e != cudaSuccess) return cuda_fail(e, "setGraph build");
+  if (edgeMap && !c->keepCsrPerm) {  // only the composed map is needed
+    cudaFree(c->csrPerm);
+    c->csrPerm = nullptr;
+  }
+  if (tight) {
+    work.release();
+    e = reserve(c->stateMem, stateBytes);
+    if (e != cudaSuccess) return cuda_fail(e, "setGraph device allocation");
+    clear_state();
+  }
+  c->maxInDeg = bins.maxIn;
+  c->maxOutDeg = bins.maxOut;
+  c->nMid = bins.nMid;
+  c->nSmall = bins.nSmall;
+  c->nTiny = bins.nTiny + bins.nZero;
+  c->binMid = c->bins + bins.nHub;
+  c->binSmall = c->binMid + bins.nMid;
+  c->binTiny = c->binSmall + bins.nSmall;
+  c->nChunks = bins.nChunks;
+  c->nChunkVertices = bins.nHub;
+  if (c->maxInDeg <= GAS_TPV_MAX_DEGREE && c->maxOutDeg <= GAS_TPV_MAX_DEGREE) {  // fused rounds
+    // fixed-width adjacency rows: a vertex's neighbours in one or two 16-byte
+    // loads addressed by its id, no offset lookup
+    c->ellWidth = std::max(c->maxInDeg, c->maxOutDeg) <= 4 ? 4 : 8;
+    const size_t fusedBytes = carve_fused(c, nullptr);
+    e = reserve(c->fusedMem, fusedBytes);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      work.release();
+      e = reserve(c->fusedMem, fusedBytes);
+    }
+    if (e != cudaSuccess) return cuda_fail(e, "setGraph device allocation");
+    carve_fused(c, c->fusedMem.p);
+    if (nV > 0) {
+      const int blocks = (int)std::min<int64_t>(((int64_t)nV + 255) / 256, 65535LL * 32);
+      ell_rows_kernel<<<blocks, 256, 0, c->stream>>>(nV, c->inOff, c->inSrc, c->ed, edgeBytes,
+                                                     c->ellWidth, c->ellIn, c->ellEd);
+      ell_rows_kernel<<<blocks, 256, 0, c->stream>>>(nV, c->outOff, c->outDst, nullptr, 0,
+                                                     c->ellWidth, c->ellOut, nullptr);
+      A(cudaGetLastError());
+    }
+    A(cudaMemsetAsync(c->frontBits, 0, sizeof(uint32_t) * 3 * std::max(c->bitWords, 1), c->stream));
+  } else {
+    give_back(c->fusedMem);
+  }
+  if (c->pullEntry > 0 && nV > 0 && work.p) {
+    st = build_layout(c, bins, hubs, dCounts, maxChunks, sx);
+    if (st == GAS_ERR_OOM) st = GAS_OK;
+  }
+  if (!c->pullIds) drop_layout(c);
+  A(cudaStreamSynchronize(c->stream));
+  if (st) return st;
+  if (e != cudaSuccess) return cuda_fail(e, "setGraph build");
+  c->haveGraph = true;
+  c->dirty = 0;
+  c->densePending = false;
+  c->epoch = 0;
+  c->stamp = 0;
+  c->iteration = 0;
+  c->round = 0;
+  c->rangeMode = true;
+  c->rstart = 0;
+  c->rcount = 0;
+  c->cur = c->sidx = 0;
+  c->pendingCommit = false;
+  c->haveScatList = false;
+  return GAS_OK;
+}
+
+}  // namespace
+
 extern "C" {
 
 gas_status gas_core_create(int32_t device, void *stream, gas_core **out) {
@@ -638,218 +926,14 @@ gas_status gas_core_set_graph(gas_core *c, int32_t nV, int32_t nE, const int32_t
   if (st) return st;
   if (c->stream) cudaStreamSynchronize(c->stream);
   free_graph(c, false);
-  auto give_up = [c](gas_status s) {  // no graph, and no memory kept for one
-    free_graph(c);
-    return s;
-  };
-
-  // working memory of the build, given back at its end: the edge list, the
-  // edge data in edge-list order, the sorts, the bins' counts
-  const size_t listBytes = ((size_t)std::max(nE, 1) * 4 + 255) & ~(size_t)255;
-  const size_t edBytes = ((size_t)edgeBytes * std::max(nE, 1) + 255) & ~(size_t)255;
-  const size_t sortBytes = sort_scratch_bytes(nV, nE, nullptr, nullptr);
-  unsigned char *work = nullptr;
-  cudaError_t e = cudaMalloc((void **)&work, 256 + 2 * listBytes + edBytes + sortBytes);
-  if (e == cudaErrorMemoryAllocation && c->arena) {  // the previous graph's memory makes room
-    cudaGetLastError();
-    free_graph(c);
-    e = cudaMalloc((void **)&work, 256 + 2 * listBytes + edBytes + sortBytes);
+  const bool kept = c->graphMem.p || c->stateMem.p || c->fusedMem.p || c->layoutMem.p || c->sliceMem.p;
+  st = build_graph(c, nV, nE, srcs, dsts, edgeData, edgeBytes, vertexBytes, gatherBytes);
+  if (st) free_graph(c);  // no graph, and no memory kept for one
+  if (st == GAS_ERR_OOM && kept) {  // what earlier graphs left is free now
+    st = build_graph(c, nV, nE, srcs, dsts, edgeData, edgeBytes, vertexBytes, gatherBytes);
+    if (st) free_graph(c);
   }
-  if (e != cudaSuccess) return give_up(cuda_fail(e, "setGraph edge list upload"));
-  struct Release {
-    unsigned char *p;
-    ~Release() { cudaFree(p); }
-  } release{work};
-  DegreeBins *dCounts = reinterpret_cast<DegreeBins *>(work);
-  int32_t *dS = reinterpret_cast<int32_t *>(work + 256);
-  int32_t *dD = reinterpret_cast<int32_t *>(work + 256 + listBytes);
-  unsigned char *dEd = work + 256 + 2 * listBytes;
-  SortScratch sx;
-  sort_scratch_bytes(nV, nE, &sx, dEd + edBytes);
-  auto A = [&](cudaError_t r) {
-    if (e == cudaSuccess) e = r;
-  };
-
-  // the edge list on the device: id check, then CSC (gather) and CSR
-  // (scatter) by stable radix sorts (gas_graph_build.cu)
-  if (nE > 0) {
-    A(cudaMemcpyAsync(dS, srcs, sizeof(int32_t) * nE, cudaMemcpyHostToDevice, c->stream));
-    A(cudaMemcpyAsync(dD, dsts, sizeof(int32_t) * nE, cudaMemcpyHostToDevice, c->stream));
-    if (edgeBytes > 0)
-      A(cudaMemcpyAsync(dEd, edgeData, (size_t)edgeBytes * nE, cudaMemcpyHostToDevice, c->stream));
-    if (e != cudaSuccess) return give_up(cuda_fail(e, "setGraph edge list upload"));
-  }
-  EdgeCheck check;
-  st = device_check_edges(c->stream, nV, nE, dS, dD, work, &check);
-  if (st == GAS_OK && check.firstBad >= 0)
-    st = fail(GAS_ERR_INVALID, "edge %lld (%d -> %d) has a vertex id outside [0, %d)", check.firstBad,
-              srcs[check.firstBad], dsts[check.firstBad], nV);
-  if (st) return give_up(st);
-
-  c->nV = nV;
-  c->nE = nE;
-  c->edgeBytes = edgeBytes;
-  c->vertexBytes = vertexBytes;
-  c->gatherBytes = gatherBytes;
-  c->maxGatherTiles = (int32_t)(((long long)nV + nE) / GAS_GATHER_TILE + 2);
-  c->maxScatTiles = (int32_t)(((long long)nV + nE) / GAS_SCATTER_TILE + 2);
-  c->bitWords = (nV + 31) / 32;
-  const bool edgeMap = c->edgeScatterOn && edgeBytes > 0;
-  // bounds on the vertices of more than kChunkEdges in-edges and their chunks
-  const int32_t maxHubs = nE / (gas::detail::kChunkEdges + 1);
-  const int32_t maxChunks = nE / gas::detail::kChunkEdges + maxHubs;
-
-  c->pullKept = c->pullEntry > 0;
-  size_t need = carve_arena(c, nullptr, edgeMap, maxHubs, maxChunks);
-  if (c->arenaBytes < need || c->arenaBytes / 4 > need) {  // too small, or mostly idle
-    if (c->arena) cudaFree(c->arena);
-    c->arena = nullptr;
-    c->arenaBytes = 0;
-    e = cudaMalloc((void **)&c->arena, need);
-    if (e == cudaErrorMemoryAllocation && c->pullKept) {  // a graph that fits without the layout
-      cudaGetLastError();
-      c->pullKept = false;
-      need = carve_arena(c, nullptr, edgeMap, maxHubs, maxChunks);
-      e = cudaMalloc((void **)&c->arena, need);
-    }
-    if (e != cudaSuccess) return give_up(cuda_fail(e, "setGraph device allocation"));
-    c->arenaBytes = need;
-  }
-  carve_arena(c, c->arena, edgeMap, maxHubs, maxChunks);
-  if (c->keepCsrPerm || edgeMap) A(dalloc(&c->csrPerm, (size_t)nE));
-  if (e != cudaSuccess) return give_up(cuda_fail(e, "setGraph device allocation"));
-
-  st = device_build_adjacency(c->stream, nV, nE, dD, dS, check.dstSorted, c->inOff, c->inSrc, c->cscPerm, sx);
-  if (st == GAS_OK)
-    st = device_build_adjacency(c->stream, nV, nE, dS, dD, check.srcSorted, c->outOff, c->outDst,
-                                c->csrPerm, sx);
-  if (st == GAS_OK && edgeMap)
-    st = device_csr_to_csc(c->stream, nE, c->cscPerm, c->csrPerm, c->csr2csc);
-  if (st == GAS_OK && edgeBytes > 0 && nE > 0)
-    st = device_gather_bytes(c->stream, dEd, c->cscPerm, nE, edgeBytes, c->ed);
-  // in-degree bins of the dense pass, heaviest first: the order in which it
-  // hands out work units
-  A(cudaMemsetAsync(dCounts, 0, sizeof(DegreeBins), c->stream));
-  const HubChunks hubs = {c->chunkVertex, c->chunkBegin, c->chunkFirst, c->chunkCount, c->chunkSlot};
-  if (st == GAS_OK && e == cudaSuccess)
-    st = device_degree_bins(c->stream, nV, c->inOff, c->outOff, maxHubs, c->bins, hubs, dCounts, sx);
-  HotInfo *dHot = reinterpret_cast<HotInfo *>(dCounts + 1);
-  A(cudaMemsetAsync(dHot, 0, sizeof(HotInfo), c->stream));
-  PullLayout pl = {c->slotOf, c->hotVertex, c->pullRec, c->chunkRec, c->pullAnyOrder, false};
-  if (st == GAS_OK && e == cudaSuccess && c->pullKept)
-    st = device_pull_records(c->stream, nV, c->inOff, c->outOff, c->bins, hubs, dCounts, maxChunks,
-                             gas::detail::pull_hot_capacity(c->pullEntry), pl, dHot, sx);
-  if (st) return give_up(st);
-  A(cudaMemsetAsync(c->mark, 0, sizeof(int32_t) * std::max(nV, 1), c->stream));
-  A(cudaMemsetAsync(c->retBits, 0, sizeof(uint32_t) * 3 * std::max(c->bitWords, 1), c->stream));
-  A(cudaMemsetAsync(c->chunkArrive, 0, sizeof(unsigned) * std::max(maxHubs, 1), c->stream));
-  A(cudaMemsetAsync(c->carryFlag, 0, sizeof(unsigned) * c->maxGatherTiles, c->stream));
-  A(cudaMemsetAsync(c->ctl, 0, sizeof(Ctl), c->stream));
-  A(cudaMemsetAsync(c->vd, 0, (size_t)vertexBytes * std::max(nV, 1), c->stream));
-  c->hInOff.resize((size_t)nV + 1);
-  c->hOutOff.resize((size_t)nV + 1);
-  DegreeBins bins;
-  HotInfo hot;
-  A(cudaMemcpyAsync(&hot, dHot, sizeof(hot), cudaMemcpyDeviceToHost, c->stream));
-  A(cudaMemcpyAsync(c->hInOff.data(), c->inOff, sizeof(int32_t) * ((size_t)nV + 1),
-                    cudaMemcpyDeviceToHost, c->stream));
-  A(cudaMemcpyAsync(c->hOutOff.data(), c->outOff, sizeof(int32_t) * ((size_t)nV + 1),
-                    cudaMemcpyDeviceToHost, c->stream));
-  A(cudaMemcpyAsync(&bins, dCounts, sizeof(bins), cudaMemcpyDeviceToHost, c->stream));
-  A(cudaStreamSynchronize(c->stream));
-  if (e != cudaSuccess) return give_up(cuda_fail(e, "setGraph build"));
-  if (edgeMap && !c->keepCsrPerm) {  // only the composed map is needed
-    cudaFree(c->csrPerm);
-    c->csrPerm = nullptr;
-  }
-  c->maxInDeg = bins.maxIn;
-  c->maxOutDeg = bins.maxOut;
-  c->nMid = bins.nMid;
-  c->nSmall = bins.nSmall;
-  c->nTiny = bins.nTiny + bins.nZero;
-  c->nZero = bins.nZero;
-  c->nHot = hot.nHot;
-  c->hotMinOut = hot.nHot > 1 ? hot.minOut : 0x7fffffff;
-  c->binMid = c->bins + bins.nHub;
-  c->binSmall = c->binMid + bins.nMid;
-  c->binTiny = c->binSmall + bins.nSmall;
-  c->nChunks = bins.nChunks;
-  c->nChunkVertices = bins.nHub;
-  if (c->pullKept) {
-    // the slices of the leading dense rounds' kernel; their extents are
-    // wanted before the rest of the memory can be sized
-    c->pullWide = pl.wide = bins.nChunks + bins.nMid / (32 / gas::detail::pull_mid_lanes(false)) + bins.nSmall / 32 <
-                            gas::detail::pull_narrow_units(c->pullAnyOrder);
-    const size_t listed = ((size_t)pull_slice_count(bins, pl.wide) + 1) * sizeof(int2);
-    const size_t sliceBytes = (listed + 255) & ~(size_t)255;
-    int2 *dSlices = reinterpret_cast<int2 *>(sx.keys[0]);
-    long long quads = 0;
-    st = device_pull_slices(c->stream, bins, pl, dSlices, &quads, sx);
-    if (st) return give_up(st);
-    const bool eds = c->pullQuadEd && edgeBytes == 4;
-    const size_t idBytes = ((size_t)quads * 16 + 256) & ~(size_t)255;
-    const size_t want = sliceBytes + idBytes * (eds ? 2 : 1);
-    if (c->pullBytes < want || c->pullBytes / 4 > want) {
-      if (c->pullMem) cudaFree(c->pullMem);
-      c->pullMem = nullptr;
-      c->pullBytes = 0;
-      if (cudaMalloc((void **)&c->pullMem, want) != cudaSuccess) {
-        cudaGetLastError();
-        c->pullMem = nullptr;
-        c->pullKept = false;  // the main kernel runs every round
-      } else {
-        c->pullBytes = want;
-      }
-    }
-    if (c->pullKept) {
-      c->pullSlices = reinterpret_cast<int2 *>(c->pullMem);
-      c->pullIds = reinterpret_cast<int4 *>(c->pullMem + sliceBytes);
-      c->pullEds = eds ? reinterpret_cast<int4 *>(c->pullMem + sliceBytes + idBytes) : nullptr;
-      if (nV > 0) A(cudaMemcpyAsync(c->pullSlices, dSlices, listed, cudaMemcpyDeviceToDevice, c->stream));
-      st = device_pull_fill(c->stream, bins, pl, c->pullSlices, c->inSrc, static_cast<const int32_t *>(c->ed),
-                            c->pullIds, c->pullEds);
-      if (st) return give_up(st);
-    }
-    A(cudaStreamSynchronize(c->stream));
-    if (e != cudaSuccess) return give_up(cuda_fail(e, "setGraph build"));
-  }
-  if (c->maxInDeg <= GAS_TPV_MAX_DEGREE && c->maxOutDeg <= GAS_TPV_MAX_DEGREE) {  // fused rounds
-    A(cudaMalloc(&c->fcell, (size_t)GAS_FUSED_CELL_BYTES(vertexBytes) * std::max(nV, 1)));
-    // fixed-width adjacency rows: a vertex's neighbours in one or two 16-byte
-    // loads addressed by its id, no offset lookup
-    c->ellWidth = std::max(c->maxInDeg, c->maxOutDeg) <= 4 ? 4 : 8;
-    const size_t cells = (size_t)std::max(nV, 1) * c->ellWidth;
-    A(dalloc(&c->ellIn, cells));
-    A(dalloc(&c->ellOut, cells));
-    if (edgeBytes > 0) A(cudaMalloc(&c->ellEd, cells * edgeBytes));
-    A(dalloc(&c->frontBits, 3 * (size_t)c->bitWords));
-    if (e == cudaSuccess && nV > 0) {
-      const int blocks = (int)std::min<int64_t>(((int64_t)nV + 255) / 256, 65535LL * 32);
-      ell_rows_kernel<<<blocks, 256, 0, c->stream>>>(nV, c->inOff, c->inSrc, c->ed, edgeBytes,
-                                                     c->ellWidth, c->ellIn, c->ellEd);
-      ell_rows_kernel<<<blocks, 256, 0, c->stream>>>(nV, c->outOff, c->outDst, nullptr, 0,
-                                                     c->ellWidth, c->ellOut, nullptr);
-      A(cudaGetLastError());
-    }
-    if (e == cudaSuccess)
-      A(cudaMemsetAsync(c->frontBits, 0, sizeof(uint32_t) * 3 * std::max(c->bitWords, 1), c->stream));
-    A(cudaStreamSynchronize(c->stream));
-    if (e != cudaSuccess) return give_up(cuda_fail(e, "setGraph device allocation"));
-  }
-  c->haveGraph = true;
-  c->dirty = 0;
-  c->densePending = false;
-  c->epoch = 0;
-  c->stamp = 0;
-  c->iteration = 0;
-  c->round = 0;
-  c->rangeMode = true;
-  c->rstart = 0;
-  c->rcount = 0;
-  c->cur = c->sidx = 0;
-  c->pendingCommit = false;
-  c->haveScatList = false;
-  return GAS_OK;
+  return st;
 }
 
 gas_status gas_core_set_pull_entry(gas_core *c, int32_t bytes, int32_t flags) {
