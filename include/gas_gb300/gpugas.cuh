@@ -190,9 +190,14 @@ class EngineGPU {
       std::is_empty<EdgeData>::value ? 0 : (int32_t)sizeof(EdgeData);
   static constexpr bool kScatterEdges =
       detail::ProgramScatterEdges<Program>::value && kEdgeBytes > 0;
-  // Programs with a scatter run list rounds only
+  // No layout of the leading dense rounds for Programs with a scatter, which
+  // run list rounds only, and without a gather: a BFS starts from a source,
+  // never with every vertex active, and would build and hold it for nothing
+  // (1 M vertices, 16.8 M edges: 115 MB).
   static constexpr int32_t kPullEntry =
-      kScatterEdges ? 0 : (int32_t)sizeof(typename detail::PullSource<Program>::type);
+      kScatterEdges || !ProgramHaveGather<Program>::value
+          ? 0
+          : (int32_t)sizeof(typename detail::PullSource<Program>::type);
   static constexpr int32_t kPullFlags =
       (detail::PullQuadEd<Program>::value ? GAS_PULL_QUAD_EDGES : 0) |
       (detail::ProgramReduceAnyOrder<Program>::value ? GAS_PULL_ANY_ORDER : 0);

@@ -11,7 +11,7 @@ import pytest
 
 from vertexapi2_gb300 import GASEngine
 from vertexapi2_gb300 import programs as P
-from vertexapi2_gb300._lib import PROGRAM_CC, load
+from vertexapi2_gb300._lib import PROGRAM_BFS, PROGRAM_CC, load
 
 pytestmark = pytest.mark.gpu
 
@@ -136,3 +136,22 @@ def test_state_may_take_the_build_memory(memory):
     assert st == 0
     memory.leave(held + SLACK)
     assert bare_set_graph(nv, s, d, 256)[0] == 0
+
+
+def held_by(program, *graphs):
+    """Bytes an engine holds after setting the graphs in turn."""
+    import torch
+    with GASEngine(program) as e:
+        free = torch.cuda.mem_get_info(0)[0]
+        for nv, s, d in graphs:
+            e.set_graph(nv, None, s, d)
+        return free - torch.cuda.mem_get_info(0)[0]
+
+
+def test_no_layout_without_a_gather(gpu):
+    pytest.importorskip("torch")
+    nv = 1 << 20
+    s, d = random_graph(nv, 1 << 24, 4)
+    bare = bare_set_graph(nv, s, d)[1]
+    assert held_by(PROGRAM_BFS, (nv, s, d)) <= bare + 8 * MB
+    assert held_by(PROGRAM_CC, (nv, s, d)) > bare + 64 * MB
