@@ -155,3 +155,15 @@ def test_no_layout_without_a_gather(gpu):
     bare = bare_set_graph(nv, s, d)[1]
     assert held_by(PROGRAM_BFS, (nv, s, d)) <= bare + 8 * MB
     assert held_by(PROGRAM_CC, (nv, s, d)) > bare + 64 * MB
+
+
+@pytest.mark.parametrize("kind", ["random", "ring"])
+def test_smaller_graph_gives_memory_back(gpu, kind):
+    pytest.importorskip("torch")
+    if kind == "random":
+        big, small = [(nv, *random_graph(nv, 16 * nv, nv)) for nv in (1 << 20, 1 << 19)]
+    else:
+        big, small = [(nv, *ring(nv)) for nv in (4 << 20, 2 << 20)]
+    own = held_by(PROGRAM_CC, small)
+    assert held_by(PROGRAM_CC, big, small) <= own * 4 // 3 + 12 * MB
+    assert held_by(PROGRAM_CC, small, big) <= held_by(PROGRAM_CC, big) + 12 * MB

@@ -282,9 +282,9 @@ void give_back(Block &b) {
 }
 
 // At least `need` bytes, the ones there already unless they are too few or
-// mostly idle.
+// more than a quarter of them would lie idle.
 cudaError_t reserve(Block &b, size_t need) {
-  if (b.bytes >= need && b.bytes / 4 <= need) return cudaSuccess;
+  if (b.bytes >= need && b.bytes - need <= b.bytes / 4) return cudaSuccess;
   give_back(b);
   const cudaError_t e = cudaMalloc((void **)&b.p, need);
   if (e == cudaSuccess)
