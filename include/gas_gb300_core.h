@@ -258,8 +258,12 @@ GAS_API gas_status gas_core_set_graph(gas_core *c, int32_t nVertices, int32_t nE
 /* Bytes of a source value in the leading dense rounds (the message of a
  * Program that declares gatherFromSource, else its VertexData), before
  * gas_core_set_graph: the graph then keeps the layout of that kernel
- * (gas_run_args::pullIds, about 5 bytes an edge, 10 with 4-byte edge
- * data, and 20 a vertex).  0 (the default): none. */
+ * (gas_run_args::pullIds).  It takes 20 bytes a vertex and, in steps of four
+ * in-edges a lane, 4 bytes an edge slot (8 with 4-byte edge data): about 5
+ * (10) an edge where vertices have many, at least 16 (32) for a vertex with
+ * any.  It is kept only where memory is to spare -- no more than an eighth of
+ * what is free beside the graph, and room left for another such graph and its
+ * build --, and its absence changes no result.  0 (the default): none. */
 #define GAS_PULL_QUAD_EDGES 1 /* flags: gatherMap reads 4-byte edge data */
 #define GAS_PULL_ANY_ORDER 2  /* flags: reductions in any order (reduceAnyOrder) */
 GAS_API gas_status gas_core_set_pull_entry(gas_core *c, int32_t bytes, int32_t flags);

@@ -138,6 +138,23 @@ def test_state_may_take_the_build_memory(memory):
     assert bare_set_graph(nv, s, d, 256)[0] == 0
 
 
+@pytest.mark.parametrize("kind", ["random", "ring"])
+def test_a_second_engine_still_fits(memory, kind):
+    nv, (s, d) = (1 << 20, random_graph(1 << 20, 1 << 24, 5)) if kind == "random" else (3 << 20, ring(3 << 20))
+    own = bare_set_graph(nv, s, d)[1]
+    least = least_free(memory, nv, s, d)
+    with GASEngine(PROGRAM_CC) as a, GASEngine(PROGRAM_CC) as b:
+        ref = labels(a, nv, s, d)
+        before = memory.free()
+        a.set_graph(0, None, s[:0], d[:0])
+        held = memory.free() - before
+        assert held > own + 16 * MB  # with its layout, where there is room
+        memory.leave(own + least + SLACK)  # two graphs, the second one's build
+        assert np.array_equal(labels(a, nv, s, d), ref)
+        assert np.array_equal(labels(b, nv, s, d), ref)
+        assert np.array_equal(labels(a, nv, s, d), ref)
+
+
 def held_by(program, *graphs):
     """Bytes an engine holds after setting the graphs in turn."""
     import torch

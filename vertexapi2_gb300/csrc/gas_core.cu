@@ -190,9 +190,10 @@ struct gas_core_s {
   bool fusedRounds = true;      // one-phase rounds when every degree is <= 8
   bool edgeScatterOn = false;   // keep csr2csc and run scatter-capable rounds
   bool edgeScatterReady = false;  // a scatter list awaits the Program's scatter
-  // adjacency, edge data, degree bins; vertex-sized state and lists; the
-  // fused rounds' arrays; the leading dense rounds' layout (records and
-  // tables, then slices), which a graph can do without
+  // adjacency, edge data, degree bins and (unless memory is tight) the
+  // vertex-sized state and lists; that state alone; the fused rounds' arrays;
+  // the leading dense rounds' layout (records and tables, then slices), which
+  // a graph can do without
   Block graphMem, stateMem, fusedMem, layoutMem, sliceMem;
   int32_t *inOff = nullptr, *inSrc = nullptr, *outOff = nullptr, *outDst = nullptr;
   void *ed = nullptr;
@@ -625,11 +626,25 @@ bool core_graph(gas_core_s *c, CoreGraph *out) {
 namespace {
 
 // The layout of the leading dense rounds (pull.cuh), from the CSC and the
-// bins, with the build's working memory; without it (c->pullIds null) the main
-// kernel runs every round.
+// bins, with the build's working memory (workBytes); without it (c->pullIds
+// null) the main kernel runs every round.
+//
+// It adds up to 10 bytes an edge and 20 a vertex to a graph that does not need
+// them, so it takes spare memory only: at most an eighth of what is free
+// beside the graph, and no more than leaves room for another such graph and
+// its build.
 gas_status build_layout(gas_core *c, const DegreeBins &bins, const HubChunks &hubs, DegreeBins *dCounts,
-                        int32_t maxChunks, const SortScratch &sx) {
-  cudaError_t e = reserve(c->layoutMem, carve_layout(c, nullptr, maxChunks));
+                        int32_t maxChunks, const SortScratch &sx, size_t workBytes) {
+  const bool eds = c->pullQuadEd && c->edgeBytes == 4;
+  size_t spare = 0, total = 0;
+  cudaError_t e = cudaMemGetInfo(&spare, &total);
+  if (e != cudaSuccess) return cuda_fail(e, "layout of the dense rounds");
+  spare += workBytes + c->layoutMem.bytes + c->sliceMem.bytes;  // what the build and an older layout hold
+  const size_t another = workBytes + c->graphMem.bytes + c->stateMem.bytes + c->fusedMem.bytes;
+  auto fits = [&](size_t bytes) { return bytes <= spare / 8 && spare - bytes >= another; };
+  const size_t tableBytes = carve_layout(c, nullptr, maxChunks);
+  if (!fits(tableBytes + (size_t)c->nE * (eds ? 8 : 4))) return GAS_OK;
+  e = reserve(c->layoutMem, tableBytes);
   if (e != cudaSuccess) return cuda_fail(e, "layout of the dense rounds");
   carve_layout(c, c->layoutMem.p, maxChunks);
   PullLayout pl = {c->slotOf, c->hotVertex, c->pullRec, c->chunkRec, c->pullAnyOrder, false};
@@ -650,9 +665,10 @@ gas_status build_layout(gas_core *c, const DegreeBins &bins, const HubChunks &hu
   long long quads = 0;
   st = device_pull_slices(c->stream, bins, pl, dSlices, &quads, sx);  // waits
   if (st) return st;
-  const bool eds = c->pullQuadEd && c->edgeBytes == 4;
   const size_t idBytes = ((size_t)quads * 16 + 256) & ~(size_t)255;
-  e = reserve(c->sliceMem, sliceBytes + idBytes * (eds ? 2 : 1));
+  const size_t idsBytes = sliceBytes + idBytes * (eds ? 2 : 1);
+  if (!fits(tableBytes + idsBytes)) return GAS_OK;
+  e = reserve(c->sliceMem, idsBytes);
   if (e != cudaSuccess) return cuda_fail(e, "layout of the dense rounds");
   c->pullSlices = reinterpret_cast<int2 *>(c->sliceMem.p);
   c->pullEds = eds ? reinterpret_cast<int4 *>(c->sliceMem.p + sliceBytes + idBytes) : nullptr;
@@ -687,7 +703,8 @@ gas_status build_graph(gas_core *c, int32_t nV, int32_t nE, const int32_t *srcs,
     }
     ~Work() { release(); }
   } work;
-  cudaError_t e = cudaMalloc((void **)&work.p, 256 + 2 * listBytes + edBytes + sortBytes);
+  const size_t workBytes = 256 + 2 * listBytes + edBytes + sortBytes;
+  cudaError_t e = cudaMalloc((void **)&work.p, workBytes);
   if (e != cudaSuccess) {
     work.p = nullptr;
     return cuda_fail(e, "setGraph edge list upload");
@@ -731,18 +748,18 @@ gas_status build_graph(gas_core *c, int32_t nV, int32_t nE, const int32_t *srcs,
   const int32_t maxHubs = nE / (gas::detail::kChunkEdges + 1);
   const int32_t maxChunks = nE / gas::detail::kChunkEdges + maxHubs;
 
-  e = reserve(c->graphMem, carve_graph(c, nullptr, edgeMap, maxChunks));
+  const size_t graphBytes = carve_graph(c, nullptr, edgeMap, maxChunks);
+  const size_t stateBytes = carve_state(c, nullptr, maxHubs, maxChunks);
+  give_back(c->stateMem);
+  e = reserve(c->graphMem, graphBytes + stateBytes);
+  const bool tight = e == cudaErrorMemoryAllocation;  // the state has to wait for the working memory
+  if (tight) {
+    cudaGetLastError();
+    e = reserve(c->graphMem, graphBytes);
+  }
   if (e != cudaSuccess) return cuda_fail(e, "setGraph device allocation");
   carve_graph(c, c->graphMem.p, edgeMap, maxChunks);
   if (c->keepCsrPerm || edgeMap) A(dalloc(&c->csrPerm, (size_t)nE));
-  if (e != cudaSuccess) return cuda_fail(e, "setGraph device allocation");
-  const size_t stateBytes = carve_state(c, nullptr, maxHubs, maxChunks);
-  e = reserve(c->stateMem, stateBytes);
-  const bool tight = e == cudaErrorMemoryAllocation;  // it has to wait for the working memory
-  if (tight) {
-    cudaGetLastError();
-    e = cudaSuccess;
-  }
   if (e != cudaSuccess) return cuda_fail(e, "setGraph device allocation");
 
   st = device_build_adjacency(c->stream, nV, nE, dD, dS, check.dstSorted, c->inOff, c->inSrc, c->cscPerm, sx);
@@ -761,7 +778,7 @@ gas_status build_graph(gas_core *c, int32_t nV, int32_t nE, const int32_t *srcs,
     st = device_degree_bins(c->stream, nV, c->inOff, c->outOff, maxHubs, c->bins, hubs, dCounts, sx);
   if (st) return st;
   auto clear_state = [&] {
-    carve_state(c, c->stateMem.p, maxHubs, maxChunks);
+    carve_state(c, tight ? c->stateMem.p : c->graphMem.p + graphBytes, maxHubs, maxChunks);
     A(cudaMemsetAsync(c->mark, 0, sizeof(int32_t) * std::max(nV, 1), c->stream));
     A(cudaMemsetAsync(c->retBits, 0, sizeof(uint32_t) * 3 * std::max(c->bitWords, 1), c->stream));
     A(cudaMemsetAsync(c->chunkArrive, 0, sizeof(unsigned) * std::max(maxHubs, 1), c->stream));
@@ -826,7 +843,7 @@ gas_status build_graph(gas_core *c, int32_t nV, int32_t nE, const int32_t *srcs,
     give_back(c->fusedMem);
   }
   if (c->pullEntry > 0 && nV > 0 && work.p) {
-    st = build_layout(c, bins, hubs, dCounts, maxChunks, sx);
+    st = build_layout(c, bins, hubs, dCounts, maxChunks, sx, workBytes);
     if (st == GAS_ERR_OOM) st = GAS_OK;
   }
   if (!c->pullIds) drop_layout(c);
