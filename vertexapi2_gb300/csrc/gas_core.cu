@@ -259,6 +259,7 @@ struct gas_core_s {
   // run bookkeeping
   unsigned long long *pinned = nullptr;
   CtlHead *head = nullptr;          // page-locked: control words read back
+  bool unchecked = false;           // rounds were queued since the error bits were last read
   cudaEvent_t ev[kRing] = {};
   cudaEvent_t t0 = nullptr, t1 = nullptr;
   float lastMs = 0.f;
@@ -500,6 +501,7 @@ gas_vertex_list scat_list(gas_core *c, int k) {
 gas_status materialize(gas_core *c) {
   if (!c->densePending) return GAS_OK;
   c->densePending = false;
+  c->unchecked = true;
   gas_status st = clean(c, sbit(c->sidx) | fbit(c->cur) | kT0 | kT1);
   if (st) return st;
   gas::detail::compact_ret_kernel<<<c->scatterGrid, 256, 0, c->stream>>>(
@@ -552,6 +554,7 @@ cudaError_t fetch_head(gas_core *c) {
 
 // The device error bits of a fetched head.
 gas_status head_error(gas_core *c) {
+  c->unchecked = false;
   const unsigned err = c->head->err;
   if (!err) return GAS_OK;
   cudaMemsetAsync(&c->ctl->err, 0, sizeof(unsigned), c->stream);
@@ -851,6 +854,7 @@ gas_status build_graph(gas_core *c, int32_t nV, int32_t nE, const int32_t *srcs,
   if (st) return st;
   if (e != cudaSuccess) return cuda_fail(e, "setGraph build");
   c->haveGraph = true;
+  c->unchecked = false;
   c->dirty = 0;
   c->densePending = false;
   c->epoch = 0;
@@ -976,13 +980,17 @@ gas_status gas_core_upload_vertex_data(gas_core *c, const void *host) {
 gas_status gas_core_download_vertex_data(gas_core *c, void *host) {
   if (!c || !host) return fail(GAS_ERR_INVALID, "download_vertex_data: null argument");
   if (!c->haveGraph) return fail(GAS_ERR_STATE, "no graph set");
-  // the error bits of the work before the copy come back with it; the data
-  // is the caller's only if there are none
-  cudaError_t e = fetch_head(c);
-  if (e == cudaSuccess && c->nV > 0)
-    e = cudaMemcpyAsync(host, c->vd, (size_t)c->vertexBytes * c->nV, cudaMemcpyDeviceToHost, c->stream);
+  // the caller's array is left alone when the rounds before failed; run() and
+  // count_active have mostly looked already, and one copy is all there is
+  if (c->unchecked) {
+    gas_status st = check_device_error(c);
+    if (st) return st;
+  }
+  if (c->nV == 0) return GAS_OK;
+  cudaError_t e =
+      cudaMemcpyAsync(host, c->vd, (size_t)c->vertexBytes * c->nV, cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  return e == cudaSuccess ? head_error(c) : cuda_fail(e, "vertex data download");
+  return e == cudaSuccess ? GAS_OK : cuda_fail(e, "vertex data download");
 }
 
 gas_status gas_core_download_edge_data(gas_core *c, void *host) {
@@ -1117,6 +1125,7 @@ gas_status gas_core_gather_apply(gas_core *c, int32_t haveGather, gas_gather_lau
   a.statSlot = c->round < kMaxRounds ? c->stats + 2 * (size_t)c->round : nullptr;
   a.iteration = c->iteration;
   a.haveGather = haveGather ? 1 : 0;
+  c->unchecked = true;
   st = launch(user, &a, (void *)c->stream);
   if (st) return st;
   cudaError_t e = cudaGetLastError();
@@ -1166,6 +1175,7 @@ gas_status gas_core_scatter_activate(gas_core *c) {
   a.resetScatMaxDeg = &c->ctl->s[c->sidx ^ 1].maxd;
   a.errWord = &c->ctl->err;
   a.statSlot = c->round < kMaxRounds ? c->stats + 2 * (size_t)c->round : nullptr;
+  c->unchecked = true;
   gas::detail::scatter_activate_kernel<<<c->scatterGrid, gas::detail::kSNT, 0, c->stream>>>(a);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "scatter launch");
@@ -1424,6 +1434,7 @@ gas_status gas_core_run_persistent(gas_core *c, int32_t maxIters, int32_t haveGa
   ra.denseEndOut = &c->ctl->denseEnd;
 
   cudaEventRecord(c->t0, c->stream);
+  c->unchecked = true;
   st = runLaunch(user, &ra, (void *)c->stream);
   if (st == GAS_ERR_UNSUPPORTED && ra.edgeScatter)  // the caller steps the rounds itself
     return fail(GAS_ERR_UNSUPPORTED, "persistent run unavailable");
@@ -1569,6 +1580,7 @@ gas_status gas_core_edge_scatter(gas_core *c, gas_edge_scatter_fn launch, void *
   a.csr2csc = c->csr2csc;
   a.vertexData = c->vd;
   a.edgeData = c->ed;
+  c->unchecked = true;
   st = launch(user, &a, (void *)c->stream);
   if (st) return st;
   cudaError_t e = cudaGetLastError();
