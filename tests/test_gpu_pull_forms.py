@@ -1,7 +1,10 @@
 """The leading dense rounds' kernel for Programs that declare nothing: their
 results equal, bit for bit, those of the same rounds run by the main kernel's
 pull pass.  256-byte vertex data with more sources of 65,535 and more
-out-edges than its table of hot sources holds."""
+out-edges than its table of hot sources holds; vertex data and edge data of 8
+bytes, and PageRank's messages, on graphs of enough work units for the narrow
+form (two for each warp of the chip), where a lane walks eight or four lanes'
+shares of a vertex one after the other."""
 from __future__ import annotations
 
 import os
@@ -9,6 +12,10 @@ import subprocess
 
 import numpy as np
 import pytest
+
+from vertexapi2_gb300 import GASEngine
+from vertexapi2_gb300 import programs as P
+from vertexapi2_gb300._lib import PROGRAM_PAGERANK
 
 pytestmark = pytest.mark.gpu
 
@@ -53,3 +60,53 @@ def test_large_vertex_data_hot_sources(driver, tmp_path, hubs, low, high):
     d = rng.integers(0, nv, s.size, dtype=np.int32)
     a, b = both(driver, tmp_path, nv, s, d, 0, 64)
     assert a[0] > 2 and np.array_equal(a, b)
+
+
+DEGREES = (0, 1, 3, 4, 7, 8, 9, 10, 31, 32, 33, 63, 64, 65, 66, 127, 129, 511, 1023, 1024, 1025, 2047, 2049)
+
+
+def narrow_graph(hot_share, seed):
+    """Every degree class and its edges, mostly vertices of 65 and 66
+    in-edges; `hot_share` of the edges leave 50 vertices."""
+    nv = 70000
+    rng = np.random.default_rng(seed)
+    deg = rng.choice([65, 66, 67, 70], nv)
+    some = rng.choice(nv, 20000, False)
+    deg[some] = rng.choice(DEGREES[:17], some.size)
+    deg[some[:400]] = rng.choice(DEGREES, 400)
+    assert (deg > 64).sum() // 4 + ((deg > 8) & (deg <= 64)).sum() // 32 > 2 * 152 * 28 + 2000
+    d = np.repeat(np.arange(nv, dtype=np.int32), deg)
+    s = rng.integers(0, nv, d.size, dtype=np.int32)
+    hot = rng.random(d.size) < hot_share
+    s[hot] = rng.integers(0, 50, int(hot.sum()), dtype=np.int32)
+    p = rng.permutation(d.size)
+    return nv, s[p], d[p]
+
+
+@pytest.mark.parametrize("hot", [0.0, 0.5])
+@pytest.mark.parametrize("which", [1, 2])
+def test_narrow_form_of_undeclared_programs(driver, tmp_path, which, hot):
+    nv, s, d = narrow_graph(hot, which)
+    a, b = both(driver, tmp_path, nv, s, d, which, 2)
+    assert a[0] > 2 and np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("hot", [0.0, 0.5])
+def test_narrow_form_of_messages(gpu, hot):
+    nv, s, d = narrow_graph(hot, 3)
+    out = []
+    for blocks in (0, 4):  # 4: a launch shape of its own, every round in the main kernel
+        vd = P.pagerank_init(nv, s)
+        with GASEngine(PROGRAM_PAGERANK) as e:
+            e.set_graph(nv, vd, s, d)
+            if blocks:
+                e.set_launch_config(True, blocks)
+            e.set_dense_policy(1 << 20)
+            e.set_active(0, nv)
+            rounds = e.run(12)
+            st = e.round_stats()
+            e.get_results()
+        out.append((rounds, vd["rank"].view(np.int32).copy(), st))
+    assert out[0][0] == out[1][0] and np.array_equal(out[0][1], out[1][1])
+    for k in out[0][2]:
+        assert np.array_equal(out[0][2][k], out[1][2][k])
