@@ -67,6 +67,23 @@ __host__ __device__ constexpr int pull_small_lanes(bool wide) { return wide ? kS
 __host__ __device__ constexpr long long pull_narrow_units(bool anyOrder) {
   return (anyOrder ? 1ll : 2ll) * 152 * 28;
 }
+// Whether a graph of `slices` slices is worth the layout, for source values of
+// `entry` bytes and edge data of edgeBytes.  Programs that declare nothing pull
+// whole vertices and keep dense.cuh's order: there only rounds short of units
+// gain, on which a warp has few chains to run one after the other, and values
+// that a lane can hold; edge data that the slices do not carry costs an access
+// of its own an edge.  run() of ten rounds (PageRank thirty), CSC -> wide form,
+// us, 8-byte values unless stated: PageRank R-MAT-14 570 -> 380, R-MAT-17
+// symmetric (20,688 slices) 1080 -> 1035, R-MAT-20 (108,595) 3011 -> 3973
+// (narrow form 4133), lattice 500 x 500 (7,808) 304 -> 292, 700 x 700 (15,305)
+// 420 -> 443; 256-byte values, R-MAT-17 symmetric 1280 -> 1688; 8-byte edge
+// data, R-MAT-14 (1,755) 234 -> 132, lattice 200 x 200 (1,250) 95 -> 72, 350 x
+// 350 (3,827) 120 -> 124 to 131, 500 x 500 154 -> 165.
+inline bool pull_pays(bool declared, int entry, int edgeBytes, bool quadEdges, bool wide, long long slices) {
+  if (declared) return true;
+  const bool carried = edgeBytes == 0 || quadEdges;
+  return wide && entry <= 32 && slices <= (carried ? 4ll : 1ll) * 152 * 24;
+}
 constexpr int kHotBytes = GAS_PULL_HOT_BYTES; // shared memory for hot values
 constexpr int kNoEdge = (int)0x80000000;      // stands for no edge: table slot 0, which no vertex has
 

@@ -200,7 +200,8 @@ class EngineGPU {
           : (int32_t)sizeof(typename detail::PullSource<Program>::type);
   static constexpr int32_t kPullFlags =
       (detail::PullQuadEd<Program>::value ? GAS_PULL_QUAD_EDGES : 0) |
-      (detail::ProgramReduceAnyOrder<Program>::value ? GAS_PULL_ANY_ORDER : 0);
+      (detail::ProgramReduceAnyOrder<Program>::value ? GAS_PULL_ANY_ORDER : 0) |
+      (detail::PullSource<Program>::kMessage ? GAS_PULL_MESSAGES : 0);
 
   bool note(gas_status s) {
     status_ = s;
@@ -237,43 +238,65 @@ class EngineGPU {
   // Fused rounds of an apply-only run (BFS: no gather) also use 1 CTA per SM.
   static constexpr int kFusedApplyBlocksPerSM = 1;
   // A run that starts with every vertex active runs its leading dense rounds
-  // in run_dense_kernel (one CTA per SM, up to 132 KB of shared memory), then resumes here.
+  // in a kernel of their own, then resumes here: run_dense_kernel where the
+  // graph keeps its layout (one CTA per SM, up to 132 KB of shared memory),
+  // else run_dense_csc_kernel.
+  static constexpr int kDenseCscBlocksPerSM = 6;
+
+  // The first of them that can be launched; false: none, the main kernel runs
+  // every round.
+  bool launchDense(const gas_run_args *ra, void *stream) {
+    constexpr bool kNarrow = (kPullFlags & (GAS_PULL_ANY_ORDER | GAS_PULL_MESSAGES)) != 0;  // pull_pays
+    const void *wide = nullptr, *narrow = nullptr;
+    if constexpr (kPullEntry > 0) wide = (const void *)detail::run_dense_kernel<Program, true>;
+    if constexpr (kPullEntry > 0 && kNarrow) narrow = (const void *)detail::run_dense_kernel<Program, false>;
+    const size_t most = detail::pull_smem_bytes<Program>(
+        detail::pull_hot_capacity((int)sizeof(typename detail::PullSource<Program>::type)));
+    const void *pull = ra->pullWide ? wide : narrow;
+    if (ra->pullIds && pull &&
+        launchDenseForm(denseGrid_[ra->pullWide ? 1 : 0], pull,
+                        ra->pullWide ? detail::PullThreads<Program, true>::value
+                                     : detail::PullThreads<Program, false>::value,
+                        most, detail::pull_smem_bytes<Program>(ra->nHot), 1, ra, stream))
+      return true;
+    return launchDenseForm(denseGrid_[2], (const void *)detail::run_dense_csc_kernel<Program, kDenseCscBlocksPerSM>,
+                           detail::kGNT, 0, 0, kDenseCscBlocksPerSM, ra, stream);
+  }
+
+  // One form: at most `perSM` CTAs per SM of `threads` threads and `smem` bytes
+  // (`most` on any graph).  grid: 0 not yet known, -1 not co-resident.
+  static bool launchDenseForm(int &grid, const void *kernel, int threads, size_t most, size_t smem, int perSM,
+                              const gas_run_args *ra, void *stream) {
+    if (grid == 0) {
+      int dev = 0, sms = 0, per = 0, coop = 0;
+      cudaGetDevice(&dev);
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+      if (most > 0) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, most);
+      cudaGetLastError();
+      if (per > perSM) per = perSM;
+      grid = (coop && per > 0 && sms > 0) ? per * sms : -1;
+    }
+    if (grid < 0) return false;
+    void *args[] = {const_cast<gas_run_args *>(ra)};
+    if (cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(threads), args, smem, (cudaStream_t)stream) ==
+        cudaSuccess)
+      return true;
+    cudaGetLastError();
+    grid = -1;
+    return false;
+  }
 
   static gas_status launchRun(void *user, const gas_run_args *ra, void *stream) {
     EngineGPU *self = static_cast<EngineGPU *>(user);
-    if (ra->allActive && ra->resume && ra->pullIds && !ra->denseFirst && self->runBlocksPerSM_ == 0) {
-      const void *dk = ra->pullWide ? (const void *)detail::run_dense_kernel<Program, true>
-                                    : (const void *)detail::run_dense_kernel<Program, false>;
-      const int threads =
-          ra->pullWide ? detail::PullThreads<Program, true>::value : detail::PullThreads<Program, false>::value;
-      const size_t most = detail::pull_smem_bytes<Program>(
-          detail::pull_hot_capacity((int)sizeof(typename detail::PullSource<Program>::type)));
-      if (self->denseGrid_ == 0 || self->denseWide_ != ra->pullWide) {
-        self->denseWide_ = ra->pullWide;
-        int dev = 0, sms = 0, per = 0, coop = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-        cudaFuncSetAttribute(dk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, dk, threads, most);
-        cudaGetLastError();
-        self->denseGrid_ = (coop && per > 0 && sms > 0) ? sms : -1;
-      }
-      if (self->denseGrid_ > 0) {
-        void *dargs[] = {const_cast<gas_run_args *>(ra)};
-        cudaError_t e = cudaLaunchCooperativeKernel(dk, dim3(self->denseGrid_), dim3(threads), dargs,
-                                                    detail::pull_smem_bytes<Program>(ra->nHot),
-                                                    (cudaStream_t)stream);
-        if (e == cudaSuccess) {
-          gas_run_args rest = *ra;
-          rest.denseFirst = 1;
-          const gas_status st = launchRun(user, &rest, stream);
-          // rounds already ran: a per-phase fallback would repeat them
-          return st == GAS_ERR_UNSUPPORTED ? GAS_ERR_CUDA : st;
-        }
-        cudaGetLastError();
-        self->denseGrid_ = -1;  // not co-resident: the main kernel runs every round
-      }
+    if (ra->allActive && ra->resume && !ra->denseFirst && self->runBlocksPerSM_ == 0 &&
+        self->launchDense(ra, stream)) {
+      gas_run_args rest = *ra;
+      rest.denseFirst = 1;
+      const gas_status st = launchRun(user, &rest, stream);
+      // rounds already ran: a per-phase fallback would repeat them
+      return st == GAS_ERR_UNSUPPORTED ? GAS_ERR_CUDA : st;
     }
     const bool applyOnly = ra->fused && !ra->g.haveGather;
     int &grid = !ra->fused ? self->runGrid_ : (applyOnly ? self->runGridFusedApply_ : self->runGridFused_);
@@ -323,8 +346,7 @@ class EngineGPU {
   int runGrid_ = 0;
   int runGridFused_ = 0;
   int runGridFusedApply_ = 0;
-  int denseGrid_ = 0;
-  int denseWide_ = 0;  // the form denseGrid_ was found for
+  int denseGrid_[3] = {0, 0, 0};  // run_dense_kernel narrow, wide; run_dense_csc_kernel
   int runBlocksPerSM_ = 0;
   VertexData *vdHost_ = nullptr;
   EdgeData *edHost_ = nullptr;

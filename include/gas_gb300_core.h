@@ -263,9 +263,11 @@ GAS_API gas_status gas_core_set_graph(gas_core *c, int32_t nVertices, int32_t nE
  * (10) an edge where vertices have many, at least 16 (32) for a vertex with
  * any.  It is kept only where memory is to spare -- no more than an eighth of
  * what is free beside the graph, and room left for another such graph and its
- * build --, and its absence changes no result.  0 (the default): none. */
+ * build --, and where its kernel is the faster one (pull_pays in pull.cuh);
+ * its absence changes no result.  0 (the default): none. */
 #define GAS_PULL_QUAD_EDGES 1 /* flags: gatherMap reads 4-byte edge data */
 #define GAS_PULL_ANY_ORDER 2  /* flags: reductions in any order (reduceAnyOrder) */
+#define GAS_PULL_MESSAGES 4   /* flags: the values are messages (gatherFromSource) */
 GAS_API gas_status gas_core_set_pull_entry(gas_core *c, int32_t bytes, int32_t flags);
 
 GAS_API gas_status gas_core_upload_vertex_data(gas_core *c, const void *host);

@@ -1,5 +1,5 @@
-// Programs that declare nothing (no gatherFromSource, no reduceAnyOrder),
-// from every vertex active: run() with the leading dense rounds in their own
+// Programs that declare nothing (no gatherFromSource, no reduceAnyOrder) and
+// one of minima in any order, from every vertex active: run() with the leading dense rounds in their own
 // kernel, and with every round in the main kernel.  Vertex data of 8 bytes,
 // of 256 bytes, and edge data of 8 bytes; sums in an order that shows.
 #include <cstdio>
@@ -42,6 +42,27 @@ struct Smooth {
   __host__ __device__ static void scatter(const VertexData *, const VertexData *, EdgeData *) {}
 };
 
+// 256 bytes a vertex, minima in any order.
+struct Least {
+  struct VertexData {
+    int x[64];
+  };
+  struct EdgeData {};
+  typedef int GatherResult;
+  static constexpr int gatherZero = 0x7fffffff;
+  static constexpr bool reduceAnyOrder = true;
+  __host__ __device__ static int gatherMap(const VertexData *, const VertexData *src, const EdgeData *) {
+    return src->x[0] ^ src->x[63];
+  }
+  __host__ __device__ static int gatherReduce(const int &l, const int &r) { return l < r ? l : r; }
+  __host__ __device__ static bool apply(VertexData *v, const int &g) {
+    v->x[63] = v->x[0];
+    v->x[0] = (int)((unsigned)(g + v->x[5]) * 2654435761u >> 3);  // keeps moving
+    return true;
+  }
+  __host__ __device__ static void scatter(const VertexData *, const VertexData *, EdgeData *) {}
+};
+
 template <class P>
 int run(int nV, int nE, const std::vector<int32_t> &s, const std::vector<int32_t> &d, FILE *out) {
   typedef typename P::VertexData VD;
@@ -54,7 +75,8 @@ int run(int nV, int nE, const std::vector<int32_t> &s, const std::vector<int32_t
   for (int main_only = 0; main_only < 2; ++main_only) {
     std::vector<VD> vd(nV);
     for (int v = 0; v < nV; ++v)
-      for (int k = 0; k < (int)(sizeof(VD) / 4); ++k) vd[v].x[k] = 0.001f * (float)((v * 7 + k) % 1013);
+      for (int k = 0; k < (int)(sizeof(VD) / 4); ++k)
+        vd[v].x[k] = std::is_same<P, Least>::value ? (v * 31 + k) % 100003 : 0.001f * (float)((v * 7 + k) % 1013);
     GASEngineGPU<P> engine;
     if (main_only) engine.setRunBlocksPerSM(4);  // a launch shape of its own
     engine.setGraph(nV, vd.data(), nE, ed.empty() ? nullptr : ed.data(), s.data(), d.data());
@@ -85,6 +107,7 @@ int main(int argc, char **argv) {
   if (!out) return 2;
   const int rc = h[2] == 0   ? run<Smooth<64, false>>(h[0], h[1], s, d, out)
                  : h[2] == 1 ? run<Smooth<2, false>>(h[0], h[1], s, d, out)
+                 : h[2] == 3 ? run<Least>(h[0], h[1], s, d, out)
                              : run<Smooth<2, true>>(h[0], h[1], s, d, out);
   fclose(out);
   return rc;

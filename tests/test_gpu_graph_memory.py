@@ -61,12 +61,13 @@ def i32(a):
     return a.ctypes.data_as(C.POINTER(C.c_int32))
 
 
-def bare_set_graph(nv, s, d, vertex_bytes=4):
-    """Status of set_graph on an engine that keeps no layout, and the bytes it
-    holds then."""
+def bare_set_graph(nv, s, d, vertex_bytes=4, entry=0, flags=0):
+    """Status of set_graph on an engine of source values of `entry` bytes (0:
+    it keeps no layout), and the bytes it holds then."""
     import torch
     lib, core = load(), C.c_void_p()
     assert lib.gas_core_create(0, None, C.byref(core)) == 0
+    assert lib.gas_core_set_pull_entry(core, entry, flags) == 0
     free = torch.cuda.mem_get_info(0)[0]
     st = lib.gas_core_set_graph(core, nv, s.size, i32(s), i32(d), None, 0, vertex_bytes, 4)
     held = free - torch.cuda.mem_get_info(0)[0]
@@ -184,3 +185,20 @@ def test_smaller_graph_gives_memory_back(gpu, kind):
     own = held_by(PROGRAM_CC, small)
     assert held_by(PROGRAM_CC, big, small) <= own * 4 // 3 + 12 * MB
     assert held_by(PROGRAM_CC, small, big) <= held_by(PROGRAM_CC, big) + 12 * MB
+
+
+def test_layout_only_where_it_pays(gpu):
+    """Programs that declare nothing keep no layout on large graphs, where the
+    kernel that reads the CSC is the faster one."""
+    pytest.importorskip("torch")
+    nv = 1 << 20
+    s, d = random_graph(nv, 1 << 24, 6)
+    bare = bare_set_graph(nv, s, d, 8)[1]
+    assert bare_set_graph(nv, s, d, 8, 8, 0)[1] <= bare + 8 * MB
+    for declared in (2, 4):  # any order, messages
+        assert bare_set_graph(nv, s, d, 8, 8, declared)[1] > bare + 64 * MB
+    nv = 100000  # 3,125 slices
+    s, d = ring(nv)
+    bare = bare_set_graph(nv, s, d)[1]
+    assert bare_set_graph(nv, s, d, 4, 4, 0)[1] > bare
+    assert bare_set_graph(nv, s, d, 4, 64, 0)[1] <= bare  # too large a value for a lane

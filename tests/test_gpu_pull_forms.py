@@ -1,10 +1,11 @@
-"""The leading dense rounds' kernel for Programs that declare nothing: their
-results equal, bit for bit, those of the same rounds run by the main kernel's
-pull pass.  256-byte vertex data with more sources of 65,535 and more
-out-edges than its table of hot sources holds; vertex data and edge data of 8
-bytes, and PageRank's messages, on graphs of enough work units for the narrow
-form (two for each warp of the chip), where a lane walks eight or four lanes'
-shares of a vertex one after the other."""
+"""The leading dense rounds' kernels: results equal, bit for bit, those of the
+same rounds run by the main kernel's pull pass.  256-byte vertex data with more
+sources of 65,535 and more out-edges than the table of hot sources holds;
+Programs that declare nothing, with vertex data and edge data of 8 bytes, on
+small graphs (the sliced layout, wide) and on large ones (the CSC kernel);
+PageRank's messages on a graph of enough work units for the narrow form (two
+for each warp of the chip), where a lane walks eight or four lanes' shares of
+a vertex one after the other."""
 from __future__ import annotations
 
 import os
@@ -51,14 +52,15 @@ def both(exe, tmp_path, nv, s, d, which, words):
     return data[0, 1:], data[1, 1:]
 
 
+@pytest.mark.parametrize("which", [0, 3])  # undeclared, minima in any order
 @pytest.mark.parametrize("hubs,low,high", [(600, 66000, 80000), (200, 60000, 70000), (600, 300, 900)])
-def test_large_vertex_data_hot_sources(driver, tmp_path, hubs, low, high):
+def test_large_vertex_data_hot_sources(driver, tmp_path, hubs, low, high, which):
     nv = 40000
     rng = np.random.default_rng(hubs + low)
     s = np.repeat(rng.choice(nv, hubs, False), rng.integers(low, high, hubs)).astype(np.int32)
     s = np.concatenate([s, rng.integers(0, nv, 200000, dtype=np.int32)])
     d = rng.integers(0, nv, s.size, dtype=np.int32)
-    a, b = both(driver, tmp_path, nv, s, d, 0, 64)
+    a, b = both(driver, tmp_path, nv, s, d, which, 64)
     assert a[0] > 2 and np.array_equal(a, b)
 
 
@@ -85,10 +87,23 @@ def narrow_graph(hot_share, seed):
 
 @pytest.mark.parametrize("hot", [0.0, 0.5])
 @pytest.mark.parametrize("which", [1, 2])
-def test_narrow_form_of_undeclared_programs(driver, tmp_path, which, hot):
+def test_undeclared_programs_on_a_large_graph(driver, tmp_path, which, hot):
     nv, s, d = narrow_graph(hot, which)
     a, b = both(driver, tmp_path, nv, s, d, which, 2)
     assert a[0] > 2 and np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("which", [1, 2])
+@pytest.mark.parametrize("nv", [1, 33, 700, 3000])
+def test_undeclared_programs_on_a_small_graph(driver, tmp_path, nv, which):
+    rng = np.random.default_rng(nv + which)
+    deg = rng.choice(DEGREES, nv) if nv > 1 else np.array([5])
+    d = np.repeat(np.arange(nv, dtype=np.int32), deg)
+    s = rng.integers(0, nv, d.size, dtype=np.int32)
+    s[rng.random(d.size) < 0.3] = nv // 2
+    p = rng.permutation(d.size)
+    a, b = both(driver, tmp_path, nv, s[p], d[p], which, 2)
+    assert np.array_equal(a, b)
 
 
 @pytest.mark.parametrize("hot", [0.0, 0.5])

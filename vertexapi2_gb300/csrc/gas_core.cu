@@ -215,6 +215,7 @@ struct gas_core_s {
   int32_t pullEntry = 0;
   bool pullQuadEd = false;      // its gathers read 4-byte edge data
   bool pullAnyOrder = false;    // its reductions may take any order
+  bool pullMessages = false;    // its source values are messages
   bool pullWide = false;        // this graph's layout has more lanes a vertex
   int2 *pullSlices = nullptr;
   int4 *pullIds = nullptr, *pullEds = nullptr;
@@ -296,7 +297,7 @@ cudaError_t reserve(Block &b, size_t need) {
   return e;
 }
 
-// No layout of the leading dense rounds: the main kernel runs every round.
+// No layout of the leading dense rounds: they run from the CSC.
 void forget_layout(gas_core *c) {
   c->pullSlices = nullptr;
   c->pullIds = c->pullEds = c->pullRec = c->chunkRec = nullptr;
@@ -630,7 +631,7 @@ namespace {
 
 // The layout of the leading dense rounds (pull.cuh), from the CSC and the
 // bins, with the build's working memory (workBytes); without it (c->pullIds
-// null) the main kernel runs every round.
+// null) those rounds run from the CSC.
 //
 // It adds up to 10 bytes an edge and 20 a vertex to a graph that does not need
 // them, so it takes spare memory only: at most an eighth of what is free
@@ -639,6 +640,13 @@ namespace {
 gas_status build_layout(gas_core *c, const DegreeBins &bins, const HubChunks &hubs, DegreeBins *dCounts,
                         int32_t maxChunks, const SortScratch &sx, size_t workBytes) {
   const bool eds = c->pullQuadEd && c->edgeBytes == 4;
+  PullLayout pl;
+  pl.anyOrder = c->pullAnyOrder;
+  c->pullWide = pl.wide = bins.nChunks + bins.nMid / (32 / gas::detail::pull_mid_lanes(false)) + bins.nSmall / 32 <
+                          gas::detail::pull_narrow_units(c->pullAnyOrder);
+  const int32_t slices = pull_slice_count(bins, pl.wide);
+  if (!gas::detail::pull_pays(c->pullAnyOrder || c->pullMessages, c->pullEntry, c->edgeBytes, eds, pl.wide, slices))
+    return GAS_OK;
   size_t spare = 0, total = 0;
   cudaError_t e = cudaMemGetInfo(&spare, &total);
   if (e != cudaSuccess) return cuda_fail(e, "layout of the dense rounds");
@@ -650,7 +658,10 @@ gas_status build_layout(gas_core *c, const DegreeBins &bins, const HubChunks &hu
   e = reserve(c->layoutMem, tableBytes);
   if (e != cudaSuccess) return cuda_fail(e, "layout of the dense rounds");
   carve_layout(c, c->layoutMem.p, maxChunks);
-  PullLayout pl = {c->slotOf, c->hotVertex, c->pullRec, c->chunkRec, c->pullAnyOrder, false};
+  pl.slotOf = c->slotOf;
+  pl.hotVertex = c->hotVertex;
+  pl.rec = c->pullRec;
+  pl.chunkRec = c->chunkRec;
   HotInfo *dHot = reinterpret_cast<HotInfo *>(dCounts + 1), hot = {0, 0};
   e = cudaMemsetAsync(dHot, 0, sizeof(HotInfo), c->stream);
   if (e != cudaSuccess) return cuda_fail(e, "layout of the dense rounds");
@@ -660,9 +671,7 @@ gas_status build_layout(gas_core *c, const DegreeBins &bins, const HubChunks &hu
   e = cudaMemcpyAsync(&hot, dHot, sizeof(hot), cudaMemcpyDeviceToHost, c->stream);
   if (e != cudaSuccess) return cuda_fail(e, "layout of the dense rounds");
   // the slices' extents are wanted before the rest of the memory can be sized
-  c->pullWide = pl.wide = bins.nChunks + bins.nMid / (32 / gas::detail::pull_mid_lanes(false)) + bins.nSmall / 32 <
-                          gas::detail::pull_narrow_units(c->pullAnyOrder);
-  const size_t listed = ((size_t)pull_slice_count(bins, pl.wide) + 1) * sizeof(int2);
+  const size_t listed = ((size_t)slices + 1) * sizeof(int2);
   const size_t sliceBytes = (listed + 255) & ~(size_t)255;
   int2 *dSlices = reinterpret_cast<int2 *>(sx.keys[0]);
   long long quads = 0;
@@ -964,6 +973,7 @@ gas_status gas_core_set_pull_entry(gas_core *c, int32_t bytes, int32_t flags) {
   c->pullEntry = bytes > 0 && gas::detail::pull_hot_capacity(bytes) > 0 ? std::max(bytes, 4) : 0;
   c->pullQuadEd = (flags & GAS_PULL_QUAD_EDGES) != 0;
   c->pullAnyOrder = (flags & GAS_PULL_ANY_ORDER) != 0;
+  c->pullMessages = (flags & GAS_PULL_MESSAGES) != 0;
   return GAS_OK;
 }
 
