@@ -46,6 +46,21 @@
 #include "gather.cuh"
 
 namespace gas {
+
+// A Program may declare `static constexpr bool haveGather = false`.
+template <class P>
+struct ProgramHaveGather {
+  template <class Q>
+  static constexpr bool get(decltype(Q::haveGather) *) {
+    return Q::haveGather;
+  }
+  template <class Q>
+  static constexpr bool get(...) {
+    return true;
+  }
+  static constexpr bool value = get<P>(nullptr);
+};
+
 namespace detail {
 
 struct DenseCtx {
@@ -209,9 +224,12 @@ __device__ __forceinline__ void group_edges(const DenseCtx &a, int v, int beg, i
     edge_acc<P>(a, v, __ldg(a.inSources + e), edge_ptr<P>(a.edgeData, e), known, x);
   }
   // without a gather the vertex needs no further edge once it is known active
+  // (compiled for Programs without one only: the tests took 4 to 10 % of the
+  // short dense rounds of others on lattices)
+  constexpr bool kGather = ProgramHaveGather<P>::value;
   if constexpr (W == 32) {
     known = known || __any_sync(kFullMask, x.act != 0u);
-    for (int q0 = qb; q0 < qe && (a.haveGather || !known); q0 += 32) {
+    for (int q0 = qb; q0 < qe && (kGather || a.haveGather || !known); q0 += 32) {
       if (q0 + sl < qe) quad_acc<P>(a, v, q0 + sl, known, x);
       known = known || __any_sync(kFullMask, x.act != 0u);
     }
@@ -219,7 +237,7 @@ __device__ __forceinline__ void group_edges(const DenseCtx &a, int v, int beg, i
     static_assert(W * 8 >= 64, "a group walks at most 64 edges in two steps");
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-      if (!a.haveGather) {  // uniform
+      if (!kGather && !a.haveGather) {  // uniform
         const unsigned act = __ballot_sync(kFullMask, x.act != 0u);
         known = known || ((act >> ((threadIdx.x & 31) / W * W)) & ((1u << W) - 1u)) != 0u;
         if (known) {
@@ -230,7 +248,7 @@ __device__ __forceinline__ void group_edges(const DenseCtx &a, int v, int beg, i
       if (qb + sl + W * k < qe) quad_acc<P>(a, v, qb + sl + W * k, known, x);
     }
   }
-  if (known) x.act = 1u;
+  if (!kGather && known) x.act = 1u;
 }
 
 struct DenseCounts {
@@ -382,7 +400,7 @@ __device__ void dense_warp_unit(const DenseCtx &a, long long u, DenseCounts &c) 
     unsigned act = 0u;
 #pragma unroll
     for (int k = 0; k < GAS_TPV_MAX_DEGREE; ++k)
-      if (beg + k < end && (a.haveGather || !act)) {
+      if (beg + k < end && (ProgramHaveGather<P>::value || a.haveGather || !act)) {
         act |= (a.skipBits || bit_test(a.prevBits, src[k])) ? 1u : 0u;
         if (a.haveGather)
           g = P::gatherReduce(g, P::gatherMap(vd + v, vd + src[k], edge_ptr<P>(a.edgeData, beg + k)));

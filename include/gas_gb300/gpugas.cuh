@@ -47,19 +47,6 @@
 
 namespace gas {
 
-template <class P>
-struct ProgramHaveGather {
-  template <class Q>
-  static constexpr bool get(decltype(Q::haveGather) *) {
-    return Q::haveGather;
-  }
-  template <class Q>
-  static constexpr bool get(...) {
-    return true;
-  }
-  static constexpr bool value = get<P>(nullptr);
-};
-
 template <typename Program, typename Int = int32_t, bool sortEdgesForGather = true>
 class EngineGPU {
   static_assert(std::is_same<Int, int32_t>::value, "vertex and edge ids are int32");
