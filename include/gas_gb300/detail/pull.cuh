@@ -59,30 +59,55 @@ constexpr int kPullBatch = 2;                 // work units a warp takes at a ti
 // 207 with dense.cuh's pass).
 __host__ __device__ constexpr int pull_mid_lanes(bool wide) { return wide ? 32 : 8; }
 __host__ __device__ constexpr int pull_small_lanes(bool wide) { return wide ? kSmallLanes : 1; }
-// Narrow units a graph needs for the narrow form: two for each warp of the
-// chip, one for Programs that reduce in any order, whose narrow units are the
-// shorter chains.  Measured at one and at two (run(), us): SSSP, 300,000
-// vertices 414, 472, 200,000 332, 369, 100,000 281, 279; CC 300,000 144, 162;
-// PageRank 400,000 1744, 1598, 200,000 and 1,000,000 the same.
-__host__ __device__ constexpr long long pull_narrow_units(bool anyOrder) {
-  return (anyOrder ? 1ll : 2ll) * 152 * 28;
+// What the choice of a kernel goes by.
+struct PullShape {
+  bool anyOrder, messages;  // the Program's declarations
+  int entry;                // bytes of a source value
+  bool carried;             // the slices carry the edge data (or there is none)
+  long long nVertices, nEdges, maxOut;
+  long long narrowUnits;    // chunks, mid / 4, small / 32
+};
+// Out-degrees of one size (random graphs, lattices): no few sources hold most
+// of the edges.
+inline bool pull_even(const PullShape &p) { return p.maxOut * p.nVertices < 16 * p.nEdges; }
+
+// The wide form: fewer narrow units than two for each warp of the chip (152
+// SMs of 28, the middle of 24 to 32), than one for Programs that reduce in any
+// order, whose narrow units are the shorter chains.  Measured at one and at
+// two (run(), us): SSSP, R-MAT of 300,000 vertices 414, 472, 200,000 332, 369,
+// 100,000 281, 279; CC 300,000 144, 162; PageRank 400,000 1744, 1598, 200,000
+// and 1,000,000 the same.  On even graphs the table answers little, the wide
+// form's bit tests are gathers too, and a third of a unit is enough (random
+// graphs, CSC, narrow, wide: CC, 70,000 vertices, 840,000 edges 126, 97, 140,
+// 40,000, 640,000 74, 60, 66, 1,600,000 74, 74, 70, 20,000, 320,000 60, 56,
+// 48; PageRank, 100,000, 1.6 M 484, 316, 500, 40,000, 1.6 M 406, 351, 287).
+inline bool pull_wide(const PullShape &p) {
+  return p.narrowUnits < (pull_even(p) ? 152ll * 10 : (p.anyOrder ? 1ll : 2ll) * 152 * 28);
 }
-// Whether a graph of `slices` slices is worth the layout, for source values of
-// `entry` bytes and edge data of edgeBytes.  Programs that declare nothing pull
-// whole vertices and keep dense.cuh's order: there only rounds short of units
-// gain, on which a warp has few chains to run one after the other, and values
-// that a lane can hold; edge data that the slices do not carry costs an access
-// of its own an edge.  run() of ten rounds (PageRank thirty), CSC -> wide form,
-// us, 8-byte values unless stated: PageRank R-MAT-14 570 -> 380, R-MAT-17
-// symmetric (20,688 slices) 1080 -> 1035, R-MAT-20 (108,595) 3011 -> 3973
-// (narrow form 4133), lattice 500 x 500 (7,808) 304 -> 292, 700 x 700 (15,305)
-// 420 -> 443; 256-byte values, R-MAT-17 symmetric 1280 -> 1688; 8-byte edge
-// data, R-MAT-14 (1,755) 234 -> 132, lattice 200 x 200 (1,250) 95 -> 72, 350 x
-// 350 (3,827) 120 -> 124 to 131, 500 x 500 154 -> 165.
-inline bool pull_pays(bool declared, int entry, int edgeBytes, bool quadEdges, bool wide, long long slices) {
-  if (declared) return true;
-  const bool carried = edgeBytes == 0 || quadEdges;
-  return wide && entry <= 32 && slices <= (carried ? 4ll : 1ll) * 152 * 24;
+// Whether the layout pays, `slices` slices of the form pull_wide chose.
+//
+// Programs that declare nothing pull whole vertices and keep dense.cuh's
+// order: there only rounds short of units gain, on which a warp has few chains
+// to run one after the other, and values that a lane can hold; edge data that
+// the slices do not carry costs an access of its own an edge.  run() of ten
+// rounds (PageRank thirty), CSC -> wide form, us, 8-byte values unless stated:
+// PageRank R-MAT-14 570 -> 380, R-MAT-17 symmetric (20,688 slices) 1080 ->
+// 1035, R-MAT-20 (108,595) 3011 -> 3973 (narrow form 4133), lattice 500 x 500
+// (7,808) 304 -> 292, 700 x 700 (15,305) 420 -> 443; 256-byte values, R-MAT-17
+// symmetric 1280 -> 1688; 8-byte edge data, R-MAT-14 (1,755) 234 -> 132,
+// lattice 200 x 200 (1,250) 95 -> 72, 350 x 350 (3,827) 120 -> 124 to 131, 500
+// x 500 154 -> 165.
+//
+// Minima on even graphs of 2 to 3.5 edges a vertex: the layout moves 48 bytes
+// a vertex and round where the CSC moves 34, which shows once they leave L2
+// (CC, 200 rounds, CSC -> layout, ms: lattice 1400 x 1400 9.9 -> 9.8, 1500 x
+// 1500 10.5 -> 11.8, 2000 x 2000 19.9 -> 23.0; random, 2 edges a vertex, 2 M
+// vertices 1.60 -> 1.72, 5 M 3.40 -> 3.84; 4 edges, 5 M 2.91 -> 2.71).  Sums
+// have a division an edge to spare (PageRank 2000 x 2000 2.34 -> 2.32).
+inline bool pull_pays(const PullShape &p, bool wide, long long slices) {
+  if (p.anyOrder && pull_even(p) && p.nVertices >= 2000000 && 2 * p.nEdges < 7 * p.nVertices) return false;
+  if (p.anyOrder || p.messages) return true;
+  return wide && p.entry <= 32 && slices <= (p.carried ? 4ll : 1ll) * 152 * 24;
 }
 constexpr int kHotBytes = GAS_PULL_HOT_BYTES; // shared memory for hot values
 constexpr int kNoEdge = (int)0x80000000;      // stands for no edge: table slot 0, which no vertex has

@@ -113,8 +113,8 @@ def labels(e, nv, s, d):
 @pytest.mark.parametrize("kind", ["random", "ring"])
 @pytest.mark.parametrize("before", ["new engine", "other graph before"])
 def test_a_graph_that_fits_is_taken(memory, kind, before):
-    nv, (s, d) = (1 << 20, random_graph(1 << 20, 1 << 24, 1)) if kind == "random" else (3 << 20, ring(3 << 20))
-    other = random_graph(1 << 19, 3 << 23, 2)
+    nv, (s, d) = (1 << 20, random_graph(1 << 20, 1 << 24, 1)) if kind == "random" else (3 << 19, ring(3 << 19))
+    other = random_graph(1 << 19, 3 << 21, 2)
     with GASEngine(PROGRAM_CC) as e:
         ref = labels(e, nv, s, d)
     least = least_free(memory, nv, s, d)
@@ -141,7 +141,7 @@ def test_state_may_take_the_build_memory(memory):
 
 @pytest.mark.parametrize("kind", ["random", "ring"])
 def test_a_second_engine_still_fits(memory, kind):
-    nv, (s, d) = (1 << 20, random_graph(1 << 20, 1 << 24, 5)) if kind == "random" else (3 << 20, ring(3 << 20))
+    nv, (s, d) = (1 << 20, random_graph(1 << 20, 1 << 24, 5)) if kind == "random" else (3 << 19, ring(3 << 19))
     own = bare_set_graph(nv, s, d)[1]
     least = least_free(memory, nv, s, d)
     with GASEngine(PROGRAM_CC) as a, GASEngine(PROGRAM_CC) as b:

@@ -642,11 +642,18 @@ gas_status build_layout(gas_core *c, const DegreeBins &bins, const HubChunks &hu
   const bool eds = c->pullQuadEd && c->edgeBytes == 4;
   PullLayout pl;
   pl.anyOrder = c->pullAnyOrder;
-  c->pullWide = pl.wide = bins.nChunks + bins.nMid / (32 / gas::detail::pull_mid_lanes(false)) + bins.nSmall / 32 <
-                          gas::detail::pull_narrow_units(c->pullAnyOrder);
+  gas::detail::PullShape shape;
+  shape.anyOrder = c->pullAnyOrder;
+  shape.messages = c->pullMessages;
+  shape.entry = c->pullEntry;
+  shape.carried = eds || c->edgeBytes == 0;
+  shape.nVertices = c->nV;
+  shape.nEdges = c->nE;
+  shape.maxOut = bins.maxOut;
+  shape.narrowUnits = bins.nChunks + bins.nMid / (32 / gas::detail::pull_mid_lanes(false)) + bins.nSmall / 32;
+  c->pullWide = pl.wide = gas::detail::pull_wide(shape);
   const int32_t slices = pull_slice_count(bins, pl.wide);
-  if (!gas::detail::pull_pays(c->pullAnyOrder || c->pullMessages, c->pullEntry, c->edgeBytes, eds, pl.wide, slices))
-    return GAS_OK;
+  if (!gas::detail::pull_pays(shape, pl.wide, slices)) return GAS_OK;
   size_t spare = 0, total = 0;
   cudaError_t e = cudaMemGetInfo(&spare, &total);
   if (e != cudaSuccess) return cuda_fail(e, "layout of the dense rounds");
