@@ -104,8 +104,16 @@ inline bool pull_wide(const PullShape &p) {
 // 1500 10.5 -> 11.8, 2000 x 2000 19.9 -> 23.0; random, 2 edges a vertex, 2 M
 // vertices 1.60 -> 1.72, 5 M 3.40 -> 3.84; 4 edges, 5 M 2.91 -> 2.71).  Sums
 // have a division an edge to spare (PageRank 2000 x 2000 2.34 -> 2.32).
+// Programs that gather vertex data are not even paid for smaller ones: a
+// shortest-path run has one dense round there, after which L2 holds the layout
+// in place of the CSC that the list rounds read (SSSP, random, 2 edges a vertex,
+// 700,000 vertices 1172 -> 1230 us, 1 M 1285 -> 1395; 4 edges, 1 M 1473 ->
+// 1524; 6 edges the same, lattice 1000 x 1000, 200 rounds, 922 -> 926).
 inline bool pull_pays(const PullShape &p, bool wide, long long slices) {
-  if (p.anyOrder && pull_even(p) && p.nVertices >= 2000000 && 2 * p.nEdges < 7 * p.nVertices) return false;
+  if (p.anyOrder && pull_even(p) &&
+      (p.messages ? p.nVertices >= 2000000 && 2 * p.nEdges < 7 * p.nVertices
+                  : p.nVertices >= 500000 && p.nEdges < 6 * p.nVertices))
+    return false;
   if (p.anyOrder || p.messages) return true;
   return wide && p.entry <= 32 && slices <= (p.carried ? 4ll : 1ll) * 152 * 24;
 }

@@ -60,11 +60,12 @@ def rmat(scale, symmetric):
     ((rmat, 16, False), {CC: "wide", PAGERANK: "wide", PLAIN: "wide", EDGES8: "csc"}),
     ((rmat, 19, True), {CC: "narrow", SSSP: "narrow", PAGERANK: "narrow", PLAIN: "csc", LARGE: "csc", EDGES8: "csc"}),
     ((lattice, 200), {CC: "wide", PAGERANK: "wide", PLAIN: "wide", EDGES8: "wide"}),
-    ((lattice, 1000), {CC: "wide", SSSP: "wide", PAGERANK: "wide", PLAIN: "csc", EDGES8: "csc"}),
+    ((lattice, 1000), {CC: "wide", SSSP: "csc", PAGERANK: "wide", PLAIN: "csc", EDGES8: "csc"}),
     ((lattice, 1700), {CC: "csc", PAGERANK: "wide", PLAIN: "csc"}),
     ((even, 20000, 16), {CC: "wide", PAGERANK: "wide"}),
     ((even, 100000, 16), {CC: "narrow", SSSP: "narrow", PAGERANK: "narrow", PLAIN: "csc"}),
-    ((even, 2000000, 8), {CC: "narrow", PAGERANK: "narrow"}),
+    ((even, 1000000, 3), {CC: "wide", SSSP: "csc", PAGERANK: "wide"}),
+    ((even, 2000000, 8), {CC: "narrow", SSSP: "narrow", PAGERANK: "narrow"}),
 ], ids=str)
 def test_choice(choose, graph, expected):
     make, *size = graph
