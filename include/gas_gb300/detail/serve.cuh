@@ -406,11 +406,22 @@ __device__ __forceinline__ void ppr_long_units(const PprArgs &a, const PprRound 
   }
 }
 
+// Rows of QP floats whose long units go through the ring.  Rows of less than
+// 16 bytes cannot, and of 32 floats the 32 rows that a warp's registers hold
+// in flight are more than the ring's five stages of 8 (20 rounds, 32 queries,
+// us, with the ring and without: R-MAT-12 860, 401, R-MAT-16 3020, 1732,
+// R-MAT-18 6068, 5025).
+__host__ __device__ constexpr bool ppr_ring_rows(int QP) { return QP >= 4 && QP < 32; }
+
 // Round r of rows of QP <= 32 floats: long units through the ring, then
 // groups of QP lanes take units (the groups of a warp neighbouring ones, so
 // similar lengths).  Work is dealt block-first, so that the longest units
-// spread over the SMs.  Rows of less than 16 bytes have no ring.
-template <int QP>
+// spread over the SMs.  kL1: rows are read through L1, which pays where a line
+// holds many and few sources have most of the edges (rows of 1 and 2; 20
+// rounds, us, past L1 and through it: 2 queries, R-MAT-18 2788, 2245, lattice
+// 500 x 500 243, 274; 4 queries 1808, 1841, 370, 452; 16 queries, 200,000
+// vertices of 8 random edges 857, 1100).
+template <int QP, bool kL1>
 __device__ __forceinline__ void ppr_round_narrow(const PprArgs &a, int r, PprRing &ring) {
   constexpr int L = QP, G = 32 / L, M = 32 / L;
   const PprRound b = ppr_buffers(a, r);
@@ -420,11 +431,11 @@ __device__ __forceinline__ void ppr_round_narrow(const PprArgs &a, int r, PprRin
   const long long gw = (long long)(threadIdx.x / 32) * gridDim.x + blockIdx.x;
   const unsigned mask = L == 32 ? kFullMask : (((1u << (L & 31)) - 1u) << (grp * L));
   long long first = 0;
-  if constexpr (QP >= 4) {
+  if constexpr (ppr_ring_rows(QP)) {
     ppr_long_units(a, b, ring);
     first = a.nLong;
   }
-  const long long busy = QP >= 4 ? ppr_long_warps(a, warps) : 0;
+  const long long busy = ppr_ring_rows(QP) ? ppr_long_warps(a, warps) : 0;
   for (long long base = first + (gw - busy) * G; gw >= busy && base < a.nUnits; base += (warps - busy) * G) {
     const long long u = base + grp;
     const int4 un = u < a.nUnits ? __ldg(a.unit + u) : make_int4(-1, 0, 0, -1);
@@ -443,7 +454,10 @@ __device__ __forceinline__ void ppr_round_narrow(const PprArgs &a, int r, PprRin
 #pragma unroll
       for (int t = 0; t < 32; ++t) {
         const int s = __shfl_sync(kFullMask, ids[t / L], t % L, L);
-        c[t] = t < len - o ? b.ct[(size_t)s * QP + j] : 0.0f;
+        if constexpr (kL1)
+          c[t] = t < len - o ? b.ct[(size_t)s * QP + j] : 0.0f;
+        else
+          c[t] = t < len - o ? __ldcg(b.ct + (size_t)s * QP + j) : 0.0f;
       }
 #pragma unroll
       for (int m = 0; m < M; ++m) ids[m] = o + 32 + m * L + j < len ? __ldg(src + o + 32 + m * L + j) : 0;
@@ -549,8 +563,15 @@ template <int QP>
 __device__ __forceinline__ void ppr_round(const PprArgs &a, int r) {
   __shared__ PprRing rings[8];  // a warp's each (256 threads)
   PprRing &ring = rings[threadIdx.x / 32];
-  if constexpr (QP <= 32)
-    ppr_round_narrow<QP>(a, r, ring);
+  if constexpr (QP == 1)
+    ppr_round_narrow<1, true>(a, r, ring);
+  else if constexpr (QP == 2) {
+    if (a.nLong > 0)
+      ppr_round_narrow<2, true>(a, r, ring);
+    else
+      ppr_round_narrow<2, false>(a, r, ring);
+  } else if constexpr (QP <= 32)
+    ppr_round_narrow<QP, false>(a, r, ring);
   else
     ppr_round_wide<QP>(a, r, ring);
 }
