@@ -274,7 +274,7 @@ GAS_API gas_status gas_batch_last_ms(gas_batch *b, float *ms);
  * vertices, with rows of Q queries (the next power of two >= n, at least 32
  * for BFS and SSSP; for PPR above 32 the next multiple of 8) and E edges,
  * needs working state of (BFS) V*Q*4 + V*(Q/8)*4 + 28*V + 24*E/512 bytes, and
- * V*Q*12 more on graphs of out-degrees <= 64 with V*Q/32 > 2^20, (SSSP)
+ * V*Q*12 more on graphs of out-degrees <= 64 with V*Q/32 > 3*2^18, (SSSP)
  * V*Q*4 + V*(Q/32)*12 + 28*V + 24*E/512, (PPR) V*Q*16 plus Q*4 bytes per
  * 4096 in-edges of vertices above 4096, plus V*n*4 for its results.  It starts only
  * when cudaMemGetInfo's free bytes plus the server pool's cached bytes,

@@ -494,9 +494,12 @@ __device__ __forceinline__ void batch_push_unit(const BatchArgs &a, int u, int c
 // 48 -> 35 (256 queries 193 -> 154); 64 BFS queries, 256 x 256 3.25 -> 2.06.
 //
 // From a list, for BFS over large masks: its rounds are short against the
-// passes over the mask (64 queries, 1000 x 1000: 21.7 ms from the mask, 19.1
-// from the list).
-constexpr long long kPairMaskWords = 1ll << 20;  // BFS: lists above
+// passes over the mask, the more so the fewer of a word's queries are live
+// (lattices, from a list and from the mask, ms: 1000 x 1000, 1 M words, 4
+// queries 12.4, 13.4, 16 12.6, 14.9, 32 13.0, 12.3; 700 x 700, 980,000 words,
+// 33 queries 9.3, 9.8, 64 9.7, 9.5, but 490,000 words, 4 queries 8.1, 6.6; 500
+// x 500, 500,000 words, 33 queries 6.3, 5.2).
+constexpr long long kPairMaskWords = 3ll << 18;  // BFS: lists above
 enum PairMode { kPairsOff = 0, kPairsMask = 1, kPairsList = 2 };
 inline int pair_mode_of(bool bfs, long long nVertices, int W) {
   return bfs && nVertices * W > kPairMaskWords ? kPairsList : kPairsMask;
