@@ -1,5 +1,7 @@
 // The leading dense (pull) rounds of a run that starts with every vertex
-// active, in a kernel of their own (see dense.cuh for what a dense round is).
+// active, in a kernel of their own (see dense.cuh for what a dense round is),
+// on graphs that keep its layout: where pull_pays, and memory is to spare.  The
+// others take run_dense_csc_kernel (persistent.cuh).
 //
 // dense.cuh's pass spends its time on instructions and L1 wavefronts, not on
 // bytes: finding a vertex's share of unaligned quads, testing a frontier bit
@@ -39,10 +41,11 @@
 //
 // Measured (run(), GB300): PageRank R-MAT-22 (4.0 M vertices, 62 M edges, 50
 // rounds) 19.6 -> 12.7 ms, R-MAT-20 5.1 -> 4.3; CC R-MAT-22 (128 M edges)
-// 1.93 -> 1.49; SSSP R-MAT-18 0.50 -> 0.46, R-MAT-21 2.71 -> 2.00.  L2 is
-// then about 64 % busy.  Table size (PageRank R-MAT-22, any order): 64 KB
-// 11.0 ms, 96 KB 10.2, 128 KB 10.0, 160 KB 10.7, 192 KB 15.8: what the table
-// takes, L1 lacks for loads in flight.
+// 1.93 -> 1.49; SSSP R-MAT-18 0.50 -> 0.46, R-MAT-21 2.71 -> 2.00.  No unit
+// is at its limit then (PageRank: L2 53 % busy on R-MAT-22, 30 % on R-MAT-20,
+// DRAM 27 and 19 %): a lane has four values in flight.  Table size (PageRank
+// R-MAT-22, any order): 64 KB 11.0 ms, 96 KB 10.2, 128 KB 10.0, 160 KB 10.7,
+// 192 KB 15.8: what the table takes, L1 lacks for loads in flight.
 #pragma once
 
 #include "dense.cuh"
@@ -155,10 +158,10 @@ struct PullSource {
   typedef typename std::conditional<kMessage, GR, VD>::type type;
 };
 
-// Threads of the CTA, by the registers a thread needs: with the table in
-// place of L1 a spill is an L2 round trip (SSSP R-MAT-18 0.54 ms at 1,024
-// threads with 88 bytes of spills, 0.45 at 896 without).  The wide form keeps
-// more: of 640, 768 and 896 threads (none spills at 768), 768 is 1 to 2 %
+// Threads of the CTA, by the registers a thread needs (SSSP R-MAT-18 0.54 ms
+// at 1,024 threads and 88 bytes of spills, 0.45 at 896 without; PageRank's 100
+// bytes at 896 and CC's 40 at 1,024 cost less than the warps are worth:
+// narrower blocks were up to 17 % slower).  The wide form keeps more: of 640, 768 and 896 threads (none spills at 768), 768 is 1 to 2 %
 // ahead over R-MAT graphs of 4,096..150,000 vertices (PageRank 60,000: 644,
 // 564, 619 us; 9,001: 386, 390, 416).
 constexpr int kWideThreads = 768;

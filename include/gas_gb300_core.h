@@ -313,7 +313,10 @@ GAS_API gas_status gas_core_restore_vertex_data(gas_core *c);
 GAS_API gas_status gas_core_set_profiling(gas_core *c, int32_t enabled);
 /* run(): a round runs dense (pull over every vertex) when the previous
  * round's apply-returned-true vertices have more than nEdges/alpha
- * out-edges; 0 disables dense rounds.  Results do not depend on it. */
+ * out-edges; 0 disables dense rounds.  The rounds that lead a run with every
+ * vertex active also stay dense, whatever alpha > 0, while those out-edges are
+ * more than nVertices/4 (Programs with a gather).  Results do not depend on
+ * it. */
 GAS_API gas_status gas_core_set_dense_policy(gas_core *c, int32_t alpha);
 /* run(): on graphs whose in- and out-degrees are all <= 8, list rounds run
  * as one phase (gather, apply and activation together, one grid barrier)
