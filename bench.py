@@ -71,13 +71,13 @@ PROGRAM_NAMES = {1: "bfs", 2: "sssp", 3: "cc", 4: "pagerank", 5: "ppr"}
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per run (the
 # run's kernels) from ncu captures of the same command (profiles/): the
-# lattice run's two kernels directly (main kernel 71.8 + 7.4 MB, one-round
-# dense kernel 54.8 + 0.1 MB, L2 flushed before the step); PageRank's dense
+# lattice run's two kernels directly (main kernel 71.7 + 6.0 MB, one-round
+# dense kernel 41.1 + 0.2 MB, L2 flushed before the step); PageRank's dense
 # kernel directly and its main kernel from R-MAT-20 scaled by edges, its traffic
 # being per-edge gathers and the CSC stream; CC's two scaled so; BFS on R-MAT-16
 # directly.  None where no capture exists.
 TRAFFIC_PER_LAUNCH = {
-    "sssp-grid1024": 71.796992e6 + 7.400192e6 + 54.819328e6 + 0.101632e6,
+    "sssp-grid1024": 71.741952e6 + 5.998080e6 + 41.142784e6 + 0.205824e6,
     "pagerank-rmat22": 26.077443e9 + 2.507805e9 + (0.064646e9 + 0.004093e9) * (65244320 / 16086703),
     # CC's two kernels on R-MAT-20 symmetric (31,406,204 edges), scaled by edges
     "cc-rmat22": (494.119680e6 + 27.425536e6 + 38.007040e6 + 0.051712e6) * (128308912 / 31406204),
